@@ -26,6 +26,7 @@
 #include "gram_dmma.cuh"
 #include "gram_tc.cuh"
 #include "sublattice.cuh"
+#include "zmix_wht.cuh"
 
 using clk::cx;
 using clk::FftPlan;
@@ -252,6 +253,10 @@ struct Sublattice {
     Axis ax[3];                           // plans and twiddles of the transform lengths
     DevBuf<cx<double>> H64, phxy64, phz64;
     DevBuf<cx<float>> H32, phxy32, phz32;
+    // FP32, zinc-blende or two classes: the tables of the z pass that mixes in registers (zmix_wht.cuh)
+    bool zw = false;
+    DevBuf<float4> zw_tab;
+    DevBuf<cx<float>> zw_col, zw_zph;
     long long tables_version = -1;        // kernel version the tables were built from
 };
 
@@ -890,7 +895,8 @@ void ensure_sl_tables(cl_ctx* c) {
     }
     const double denom = (double)((unsigned long long)c->M * 8ull);
     const int blocks = grid_for(nq);
-    if (sl.zb) {
+    sl.zw = fp32 && (sl.zb ? clp::zw_zb_supported(pz) : sl.S == 2 && clp::zw_pair_supported(pz));
+    if (sl.zb || sl.zw) {
         // raw class kernels in FP64, then their Walsh-Hadamard form (sublattice.cuh) rounded once
         DevBuf<cx<double>> raw;
         raw.alloc((size_t)res.nh * nq);
@@ -898,11 +904,34 @@ void ensure_sl_tables(cl_ctx* c) {
                                                                  res, denom, raw.p);
         CL_LAUNCHED();
         clk::SlWht w{};
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < sl.S; ++k) {
             w.src[k] = sl.table.h[k * clk::kSlMaxClasses];  // (class k, class 0): alpha_k, then beta_k
             w.cj[k] = sl.table.cj[k * clk::kSlMaxClasses];
         }
-        if (fp32) {
+        if (sl.zw) {
+            const int half = sl.S / 2;  // class 0 of the second half
+            clk::ZwBuild zb{};
+            std::memcpy(zb.src, w.src, sizeof zb.src);
+            std::memcpy(zb.cj, w.cj, sizeof zb.cj);
+            for (int d = 0; d < 3; ++d) {
+                zb.delta[d] = sl.off[half][d] - sl.off[0][d];
+                zb.n[d] = c->n[d];
+                zb.p[d] = sl.pad[d];
+                // the half's offsets along the axis are its class 0's and that +- 2 (zinc-blende, mod 4)
+                for (int h = 0; h < 2; ++h) zb.sgn[h][d] = sl.off[h * half][d] < 2 ? 1 : -1;
+            }
+            if (sl.zb) {
+                sl.zw_tab.alloc((size_t)3 * nq);
+                sl.zw_col.alloc((size_t)7 * nxy);
+                sl.zw_zph.alloc((size_t)2 * pz);
+                clk::k_zw_table<clk::kZwZb><<<blocks, 256, 0, c->stream>>>(raw.p, zb, sl.zw_tab.p);
+                CL_LAUNCHED();
+                clk::k_zw_columns<<<grid_for(nxy), 256, 0, c->stream>>>(zb, sl.zw_col.p, sl.zw_zph.p);
+            } else {
+                sl.zw_tab.alloc((size_t)nq);
+                clk::k_zw_table<clk::kZwPair><<<blocks, 256, 0, c->stream>>>(raw.p, zb, sl.zw_tab.p);
+            }
+        } else if (fp32) {
             sl.H32.alloc((size_t)8 * nq);
             clk::k_sl_zb_wht<float><<<blocks, 256, 0, c->stream>>>(raw.p, nq, w, sl.H32.p);
         } else {
@@ -921,6 +950,10 @@ void ensure_sl_tables(cl_ctx* c) {
                                                                  res, denom, sl.H64.p);
     }
     CL_LAUNCHED();
+    if (sl.zw) {
+        sl.tables_version = c->kernel_version;
+        return;
+    }
     // phases: phxy[s][ky][kx] = exp(-i pi (kx bx/nx + ky by/ny)), phz[b][kz] = exp(-i pi kz b/nz) (b < m;
     // rows up to 4), in extended precision and rounded once
     const long double pi = 3.141592653589793238462643383279502884L;
@@ -1052,7 +1085,8 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
     const double atoms = (double)n_at;
     const double live = skip_empty ? (double)c->live_rows / nrows : 1.0;
     const double row_side = (double)c->live_rows / nrows;
-    const double h_bytes = (double)sl.table.nh * sl.pad[2] * nxy * sizeof(cx<T>);
+    const double h_bytes = sl.zw ? (sl.zb ? 48.0 : 16.0) * sl.pad[2] * nxy
+                                 : (double)sl.table.nh * sl.pad[2] * nxy * sizeof(cx<T>);
     for (int p0 = 0; p0 < np; p0 += chunk) {
         const int cnt = std::min(chunk, np - p0);
         const cx<T>* rho_c = rho + (long long)p0 * rho_stride;
@@ -1082,7 +1116,16 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
             prof_end(c, e, CL_KCLASS_YPASS, cnt * (1.0 + live) * gbytes);
         }
         e = prof_begin(c);
-        if (!clp::zmix<T>(c->stream, buf, vM, twz, H, phxy, phz, mix, sl.zb, nxy, sl.pad[2], cnt))
+        bool mixed;
+        if (sl.zw) {
+            cx<float>* b32 = reinterpret_cast<cx<float>*>(buf);
+            const cx<float>* t32 = reinterpret_cast<const cx<float>*>(twz);
+            mixed = sl.zb ? clp::zw_zb(c->stream, b32, vM, t32, sl.zw_tab.p, sl.zw_col.p, sl.zw_zph.p, nxy, sl.pad[2], cnt)
+                          : clp::zw_pair(c->stream, b32, vM, t32, sl.zw_tab.p, nxy, sl.pad[2], cnt);
+        } else {
+            mixed = clp::zmix<T>(c->stream, buf, vM, twz, H, phxy, phz, mix, sl.zb, nxy, sl.pad[2], cnt);
+        }
+        if (!mixed)
             cl::fail(CL_ERR_UNSUPPORTED, "no sub-lattice z pass for %d points", sl.pad[2]);
         CL_LAUNCHED();
         prof_end(c, e, CL_KCLASS_ZPASS, cnt * 2.0 * gbytes + h_bytes);

@@ -94,4 +94,14 @@ template <typename T>
 bool zmix(cudaStream_t s, cx<T>* buf, long long stride, const cx<T>* tw, const cx<T>* H, const cx<T>* phxy,
           const cx<T>* phz, const clk::SlMix& mix, bool zb, long long nxy, int nz, int cnt);
 
+// The same for FP32 and the class sets that one thread mixes in registers (zmix_wht.cuh): the zinc-blende
+// classes and two-class sets, with their packed coefficient table (k_zw_table) and, for zinc-blende, the
+// column and z phases (k_zw_columns).  false: no compiled split of nz (nothing launched).
+bool zw_zb_supported(int nz);
+bool zw_pair_supported(int nz);
+bool zw_zb(cudaStream_t s, cx<float>* buf, long long stride, const cx<float>* tw, const float4* tab,
+           const cx<float>* col, const cx<float>* zph, long long nxy, int nz, int cnt);
+bool zw_pair(cudaStream_t s, cx<float>* buf, long long stride, const cx<float>* tw, const float4* tab, long long nxy,
+             int nz, int cnt);
+
 }  // namespace clp
