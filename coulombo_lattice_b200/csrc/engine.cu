@@ -1240,20 +1240,8 @@ TcShape tc_shape(const cl_ctx* c, int nl, int nr, long long n_atoms) {
     return s;
 }
 
-// FP32 potentials and FP32 densities in one tile of each operand (at most 64 left and 64 right
-// densities): the Gram splits its operands itself (k_gram_tc_fused) and needs no operand
-// buffer.  With more tiles a block would convert its operands once per tile of the other
-// side, and the split pass + k_gram_tc is used.  CL_TC_SPLIT=1 keeps the split pass
-// everywhere; CL_TC_FUSED=1 takes the fused Gram at any tile count.
-bool fused_gram(bool v_f32, bool rho_f32, int nl, int nr) {
-    if (!v_f32 || !rho_f32 || std::getenv("CL_TC_SPLIT")) return false;
-    if (std::getenv("CL_TC_FUSED")) return true;
-    return 2 * nl <= clk::tc::BM && 2 * nr <= clk::tc::BN;
-}
-
 // Reductions of the FP32 forms over fewer than 65,536 atoms (CL_TC_MIN_ATOMS) are summed in
-// FP64: the FP64 tensor-core Gram (k_gram_dmma) on FP32 potentials and densities, k_gram on FP64
-// potentials.  The TF32x3 Gram's error is ~2^-23 of each product, random in sign, so relative to
+// FP64 (k_gram_dmma).  The TF32x3 Gram's error is ~2^-23 of each product, random in sign, so relative to
 // the sum of the terms' magnitudes it falls as 1/sqrt(atoms): at 2M atoms it is far below the
 // FP32 gate even where the terms cancel 1000:1, while on a box of a hundred atoms it can reach
 // the 1e-9 eV floor on integrals that small.  Below the threshold the FP64 Gram costs little.
@@ -1265,13 +1253,56 @@ bool small_gram(const cl_ctx* c, long long n_atoms) {
     return !fp64_form(c) && n_atoms < tc_min_atoms() && !std::getenv("CL_TC_FUSED") && !std::getenv("CL_TC_SPLIT");
 }
 
-// Operand buffer for (nl, nr, n_atoms): whole atom range when it fits in a quarter of the free
+// Pairs of densities a request reduces: the result is [nl][nr], its needed part a few blocks
+// (gram_blocks.hpp), which can also be taken as one block.
+struct GramPlan {
+    int nl = 0, nr = 0;
+    std::vector<clk::GramBlock> blocks;  // at most clk::kGramBlocks
+    clk::GramBlock whole{};
+};
+GramPlan whole_gram(int nl, int nr, bool sym) {
+    GramPlan g;
+    g.nl = nl;
+    g.nr = nr;
+    g.whole = clk::GramBlock{0, nl, 0, nr, sym ? 1 : 0};
+    g.blocks = {g.whole};
+    return g;
+}
+// The plan's tiles of at most max_l x max_r densities: as separate blocks, or as one block where that
+// gives fewer (a tensor-core tile costs nearly the same whatever it holds).
+clk::GramTiles tc_tiles(const GramPlan& g, int max_l, int max_r) {
+    const clk::GramTiles parts = clk::gram_tiles(g.blocks.data(), (int)g.blocks.size(), g.nr, max_l, max_r, 1);
+    const clk::GramTiles one = clk::gram_tiles(&g.whole, 1, g.nr, max_l, max_r, 1);
+    return clk::gram_tile_count(one) <= clk::gram_tile_count(parts) ? one : parts;
+}
+
+// How a request's reductions are computed.
+enum class GramKind {
+    kFp64,   // FP64 tensor cores (k_gram_dmma)
+    kFused,  // TF32x3, operands split inside the kernel (k_gram_tc_ws)
+    kSplit,  // TF32x3 after the split pass (k_tf32_split, k_gram_tc)
+};
+// FP32 potentials and densities can take either TF32x3 Gram: the fused one splits the operands of its
+// tile (at most 64 x 40 densities) itself, once per tile, the other reads split operands that a pass of
+// their own writes.  Per k-tile of 32 atoms an SM takes 1.06 us for a fused tile and 1.17 us for a
+// 64 x 64 tile after the split, whose pass costs 0.019 us a density (36 densities a side over 2.1M
+// atoms: 0.47 ms in one fused tile; 820: 11.0 ms in 169 tiles, and 1.64 ms the split).  CL_TC_SPLIT=1
+// keeps the split pass everywhere; CL_TC_FUSED=1 takes the fused Gram at any tile count.
+GramKind gram_kind(const cl_ctx* c, const GramPlan& g, bool v_f32, bool rho_f32, long long n_atoms) {
+    if (!use_tc_gram(c) || small_gram(c, n_atoms)) return GramKind::kFp64;
+    if (!v_f32 || !rho_f32 || std::getenv("CL_TC_SPLIT")) return GramKind::kSplit;
+    if (std::getenv("CL_TC_FUSED")) return GramKind::kFused;
+    const double fused = 1.06 * clk::gram_tile_count(tc_tiles(g, clk::tc::BM / 2, clk::tc::WS_MAX_NB / 2));
+    const double split = 1.17 * clk::gram_tile_count(tc_tiles(g, clk::tc::BM / 2, clk::tc::BN / 2)) +
+                         0.019 * (g.nl + g.nr);
+    return fused <= split ? GramKind::kFused : GramKind::kSplit;
+}
+
+// Operand buffer of the split pass: whole atom range when it fits in a quarter of the free
 // device memory (at most 8 GiB), else chunks of the atom range.  Called outside any capture.
-void tc_reserve(cl_ctx* c, int nl, int nr, long long n_atoms, bool v_f32, bool rho_f32) {
-    if (!use_tc_gram(c) || nl <= 0 || nr <= 0 || n_atoms <= 0 || fused_gram(v_f32, rho_f32, nl, nr) ||
-        small_gram(c, n_atoms))
-        return;
-    const int rowsA = 2 * nl, rowsB = 2 * nr;
+void tc_reserve(cl_ctx* c, const GramPlan& g, long long n_atoms, bool v_f32, bool rho_f32) {
+    if (g.nl <= 0 || g.nr <= 0 || n_atoms <= 0 || gram_kind(c, g, v_f32, rho_f32, n_atoms) != GramKind::kSplit) return;
+    const int rowsA = 2 * g.nl, rowsB = 2 * g.nr;
     const long long per_atom = tc_bytes_per_atom(rowsA, rowsB);
     const long long full = (n_atoms + clk::tc::BK - 1) / clk::tc::BK * clk::tc::BK;
     const long long have = (long long)(c->tc_buf.n * sizeof(float)) / per_atom;
@@ -1304,45 +1335,107 @@ int gram_splits(int tiles, int kt_total) {
     return best_s;
 }
 
-// The FP64 tensor-core Gram on FP32 operands over the whole atom range (see k_gram_dmma).
-void gram_dmma(cl_ctx* c, const cx<float>* V, long long v_stride, int nl, const cx<float>* rho, long long r_stride,
-               const int* ridx_dev, int nr, long long n_atoms, double* out4_dev) {
+// Register tile (A x B MMA tiles a warp) and warp grid of an FP64 Gram over C tiles of ta x tb MMA tiles:
+// the least work of a warp per k-step -- 16 cycles of its FP64 pipe an MMA, about 5 a fragment -- times
+// the warps that share it.
+struct DmmaShape {
+    int reg = 0, wr = 1, wc = 1;
+    double cost = 1e300;
+};
+constexpr int kDmmaReg[8][2] = {{1, 1}, {2, 2}, {3, 3}, {4, 4}, {5, 5}, {6, 6}, {7, 4}, {8, 4}};
+DmmaShape dmma_shape(int ta, int tb) {
+    DmmaShape best;
+    for (int wr = 1; wr <= clk::dm::WARPS; wr *= 2)
+        for (int wc = 1; wr * wc <= clk::dm::WARPS; wc *= 2)
+            for (int r = 0; r < 8; ++r) {
+                const int A = kDmmaReg[r][0], B = kDmmaReg[r][1];
+                if (wr * A < ta || wc * B < tb) continue;
+                const double t = (16.0 * A * B + 5.0 * (A + B)) * wr * wc;
+                if (t < best.cost) best = DmmaShape{r, wr, wc, t};
+            }
+    return best;
+}
+
+// The FP64 tensor-core Gram over the whole atom range (see k_gram_dmma).  Tile sides of at most 24, 48
+// or 64 densities, whichever takes the fewest MMAs over all tiles (smaller ones follow a symmetric
+// block's diagonal closer), in whole 8-row tiles of the MMA.
+template <typename SV, typename SR>
+void gram_dmma(cl_ctx* c, const cx<SV>* V, long long v_stride, const cx<SR>* rho, long long r_stride,
+               const int* ridx_dev, const GramPlan& plan, long long n_atoms, double* out4_dev) {
     using namespace clk::dm;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        CL_CUDA(cudaFuncSetAttribute(k_gram_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    });
-    const int tilesA = (2 * nl + TILE - 1) / TILE, tilesB = (2 * nr + TILE - 1) / TILE;
-    const int nA4 = (std::min(TILE / 2, nl) + 3) & ~3, nB4 = (std::min(TILE / 2, nr) + 3) & ~3;
-    GramArgs g{};
-    g.V = reinterpret_cast<const float2*>(V);
+    GramArgs<SV> g{};
+    g.V = V;
     g.v_stride = v_stride;
-    g.rho = reinterpret_cast<const float2*>(rho);
-    g.r_stride = r_stride;
     g.ridx = ridx_dev;
-    g.nl = nl;
-    g.nr = nr;
+    g.r_stride = r_stride;
     g.na = n_atoms;
-    g.nd_max = nA4 + nB4;
     g.out4 = out4_dev;
-    const int chunks = (int)std::min<long long>((n_atoms + KC - 1) / KC, 1LL << 30);
-    // small boxes: enough atom splits to occupy every SM (at least 2 chunks a block)
-    const int splits0 = std::max(gram_splits(tilesA * tilesB, chunks),
-                                 std::min(chunks / 2, (148 + tilesA * tilesB - 1) / (tilesA * tilesB)));
+    DmmaShape shape;
+    for (int width : {WIDTH, 48, 24}) {
+        const clk::GramTiles t = clk::gram_tiles(plan.blocks.data(), (int)plan.blocks.size(), plan.nr, width, width, 4);
+        int a = 0, b = 0;
+        for (int k = 0; k < t.n; ++k) {
+            a = std::max(a, t.wl[k]);
+            b = std::max(b, t.wr[k]);
+        }
+        DmmaShape sh = dmma_shape(a / 4, b / 4);
+        sh.cost *= clk::gram_tile_count(t);
+        if (sh.cost < 0.9 * shape.cost) {
+            shape = sh;
+            g.tiles = t;
+            g.nd_a = a;
+            g.nd_b = b;
+        }
+    }
+    g.wr = shape.wr;
+    g.wc = shape.wc;
+    g.align_v = reinterpret_cast<uintptr_t>(V) % 16 == 0 && v_stride * sizeof(cx<SV>) % 16 == 0;
+    g.align_r = reinterpret_cast<uintptr_t>(rho) % 16 == 0 && r_stride * sizeof(cx<SR>) % 16 == 0;
+    const int tiles = clk::gram_tile_count(g.tiles);
+    const int kc = g.wr * g.wc == 1 && n_atoms / 64 * tiles >= 148 * 4 ? 64 : 32;
+    const int chunks = (int)std::min<long long>((n_atoms + kc - 1) / kc, 1LL << 30);
+    // small boxes: enough atom splits to occupy the SMs in one wave (at least 2 chunks a block)
+    const int splits0 = std::max(1, std::max(gram_splits(tiles, chunks), std::min(chunks / 2, 148 / tiles)));
     const long long per_chunks = (chunks + splits0 - 1) / splits0;
-    g.atoms_per_split = per_chunks * KC;
+    g.atoms_per_split = per_chunks * kc;
     const int splits = (int)((n_atoms + g.atoms_per_split - 1) / g.atoms_per_split);
-    const size_t smem = smem_bytes(g.nd_max);
-    if (smem > 227 * 1024) cl::fail(CL_ERR_UNSUPPORTED, "FP64 Gram needs %zu bytes of shared memory", smem);
+    const size_t stage = stage_bytes<SV, SR>(kc, g.nd_a, g.nd_b);
+    g.stages = 4 * stage <= 220 * 1024 ? 4 : 3 * stage <= 224 * 1024 ? 3 : 2;
+    const size_t smem = std::max(g.stages * stage, reduce_bytes(kDmmaReg[shape.reg][0], kDmmaReg[shape.reg][1],
+                                                                 WARPS / (g.wr * g.wc)));
     cudaEvent_t e = prof_begin(c);
-    k_gram_dmma<<<dim3(tilesA, tilesB, splits), THREADS, smem, c->stream>>>(g);
+    const dim3 grid(tiles, splits);
+    const auto launch = [&](auto kern) {
+        ensure_smem(kern, 226 * 1024);  // beside 256 bytes of static shared memory
+        kern<<<grid, THREADS, smem, c->stream>>>(rho, g);
+    };
+    const auto square = [&](auto k) {
+        constexpr int KC = decltype(k)::value;
+        switch (shape.reg) {
+            case 0: launch(k_gram_dmma<SV, SR, KC, 1, 1>); break;
+            case 1: launch(k_gram_dmma<SV, SR, KC, 2, 2>); break;
+            case 2: launch(k_gram_dmma<SV, SR, KC, 3, 3>); break;
+            case 3: launch(k_gram_dmma<SV, SR, KC, 4, 4>); break;
+            case 4: launch(k_gram_dmma<SV, SR, KC, 5, 5>); break;
+            default: launch(k_gram_dmma<SV, SR, KC, 6, 6>); break;
+        }
+    };
+    if (shape.reg == 6)
+        launch(k_gram_dmma<SV, SR, 32, 7, 4>);
+    else if (shape.reg == 7)
+        launch(k_gram_dmma<SV, SR, 32, 8, 4>);
+    else if (kc == 64)
+        square(std::integral_constant<int, 64>{});
+    else
+        square(std::integral_constant<int, 32>{});
     CL_LAUNCHED();
-    prof_end(c, e, CL_KCLASS_GRAM, (double)n_atoms * (nl + nr) * (double)sizeof(cx<float>));
+    prof_end(c, e, CL_KCLASS_GRAM,
+             (double)n_atoms * (plan.nl * (double)sizeof(cx<SV>) + plan.nr * (double)sizeof(cx<SR>)));
 }
 
 // The fused Gram on FP32 operands over the whole atom range (see k_gram_tc_fused).
-void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, int nl, const cx<float>* rho,
-                   long long r_stride, const int* ridx_dev, int nr, long long n_atoms, double* out4_dev) {
+void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, const cx<float>* rho, long long r_stride,
+                   const int* ridx_dev, const GramPlan& plan, long long n_atoms, double* out4_dev) {
     using namespace clk::tc;
     static std::once_flag once;
     std::call_once(once, [] {
@@ -1353,19 +1446,25 @@ void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, int nl, co
         CL_CUDA(cudaFuncSetAttribute(k_gram_tc_ws<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         CL_CUDA(cudaFuncSetAttribute(k_gram_tc_ws<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     });
-    const int tilesA = (2 * nl + BM - 1) / BM, tilesB = (2 * nr + BN - 1) / BN;
-    const int nA = std::min(BM / 2, nl), nB = std::min(BN / 2, nr);
-    const int nb = std::max(16, (2 * nB + 15) / 16 * 16);
+    // the warp-specialised kernel takes up to 40 right densities a tile; CL_TC_NO_WS=1 keeps the kernel
+    // whose warps take every role in turn, up to 64
+    const bool ws = !std::getenv("CL_TC_NO_WS");
     FusedGram g{};
+    g.tiles = tc_tiles(plan, BM / 2, ws ? WS_MAX_NB / 2 : BN / 2);
+    int nA = 1, nB = 1;
+    for (int b = 0; b < g.tiles.n; ++b) {
+        nA = std::max(nA, std::min(g.tiles.wl[b], g.tiles.b[b].nl));
+        nB = std::max(nB, std::min(g.tiles.wr[b], g.tiles.b[b].nr));
+    }
+    const int nb = std::max(16, (2 * nB + 15) / 16 * 16);
     g.V = reinterpret_cast<const float2*>(V);
     g.v_stride = v_stride;
     g.rho = reinterpret_cast<const float2*>(rho);
     g.r_stride = r_stride;
     g.ridx = ridx_dev;
-    g.nl = nl;
-    g.nr = nr;
     g.na = n_atoms;
     g.out4 = out4_dev;
+    g.err = out4_dev + (size_t)4 * plan.nl * plan.nr;
     g.kt_total = (int)((n_atoms + BK - 1) / BK);
     g.stage_bytes = (uint32_t)(2 * BM * 128 + 2 * nb * 128);
     g.raw_slot_bytes = (uint32_t)((nA + nB) * BK * 8);
@@ -1374,29 +1473,23 @@ void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, int nl, co
                    v_stride % 2 == 0 && r_stride % 2 == 0 && !std::getenv("CL_TC_COPY8"))
                       ? 1
                       : 0;
-    const int splits0 = gram_splits(tilesA * tilesB, g.kt_total);
+    const int tiles = clk::gram_tile_count(g.tiles);
+    const int splits0 = gram_splits(tiles, g.kt_total);
     g.kt_per = (g.kt_total + splits0 - 1) / splits0;
     const int splits = (g.kt_total + g.kt_per - 1) / g.kt_per;
     // the deepest copy ring that fits: 5 k-tiles ahead (6 slots) at the 2.1M-atom box's 72 densities
-    const size_t smem5 = fused_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 5);
-    const size_t smem3 = fused_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 3);
-    const size_t smem2 = fused_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 2);
+    const size_t smem5 = ws ? ws_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 5) : fused_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 5);
+    const size_t smem3 = ws ? ws_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 3) : fused_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 3);
+    const size_t smem2 = ws ? ws_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 2) : fused_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 2);
     if (smem2 > 227 * 1024) cl::fail(CL_ERR_UNSUPPORTED, "fused Gram needs %zu bytes of shared memory", smem2);
     cudaEvent_t e = prof_begin(c);
-    const dim3 grid(tilesA, tilesB, splits);
-    // up to 40 right densities a block (N <= 80): the warp-specialised kernel; CL_TC_NO_WS=1
-    // keeps the kernel whose warps take every role in turn
-    const bool ws = nb <= WS_MAX_NB && !std::getenv("CL_TC_NO_WS");
-    const size_t ws5 = ws_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 5);
-    const size_t ws3 = ws_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 3);
-    const size_t ws2 = ws_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 2);
-    if (ws && ws2 > 227 * 1024) cl::fail(CL_ERR_UNSUPPORTED, "fused Gram needs %zu bytes of shared memory", ws2);
-    if (ws && ws5 <= 227 * 1024)
-        k_gram_tc_ws<5><<<grid, WS_THREADS, ws5, c->stream>>>(g);
-    else if (ws && ws3 <= 227 * 1024)
-        k_gram_tc_ws<3><<<grid, WS_THREADS, ws3, c->stream>>>(g);
+    const dim3 grid(tiles, splits);
+    if (ws && smem5 <= 227 * 1024)
+        k_gram_tc_ws<5><<<grid, WS_THREADS, smem5, c->stream>>>(g);
+    else if (ws && smem3 <= 227 * 1024)
+        k_gram_tc_ws<3><<<grid, WS_THREADS, smem3, c->stream>>>(g);
     else if (ws)
-        k_gram_tc_ws<2><<<grid, WS_THREADS, ws2, c->stream>>>(g);
+        k_gram_tc_ws<2><<<grid, WS_THREADS, smem2, c->stream>>>(g);
     else if (smem5 <= 227 * 1024)
         k_gram_tc_fused<5><<<grid, FUSED_THREADS, smem5, c->stream>>>(g);
     else if (smem3 <= 227 * 1024)
@@ -1404,31 +1497,23 @@ void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, int nl, co
     else
         k_gram_tc_fused<2><<<grid, FUSED_THREADS, smem2, c->stream>>>(g);
     CL_LAUNCHED();
-    prof_end(c, e, CL_KCLASS_GRAM, (double)n_atoms * (nl + nr) * (double)sizeof(cx<float>));
+    prof_end(c, e, CL_KCLASS_GRAM, (double)n_atoms * (plan.nl + plan.nr) * (double)sizeof(cx<float>));
 }
 
-// out4[l][r] += {sum ac, bd, ad, bc} (out4 zeroed by the caller, error slot included).
-void gram_tc(cl_ctx* c, const void* V, bool v_f32, long long v_stride, int nl, const void* rho, bool rho_f32,
-             long long r_stride, const int* ridx_dev, int nr, long long n_atoms, double* out4_dev) {
+// The split pass and the TF32x3 Gram on its operands, in chunks of the atom range.
+void gram_tc_split(cl_ctx* c, const void* V, bool v_f32, long long v_stride, const void* rho, bool rho_f32,
+                   long long r_stride, const int* ridx_dev, const GramPlan& plan, long long n_atoms, double* out4_dev) {
     using namespace clk::tc;
-    if (fused_gram(v_f32, rho_f32, nl, nr)) {
-        gram_tc_fused(c, static_cast<const cx<float>*>(V), v_stride, nl, static_cast<const cx<float>*>(rho), r_stride,
-                      ridx_dev, nr, n_atoms, out4_dev);
-        return;
-    }
+    const int nl = plan.nl, nr = plan.nr;
     const TcShape sh = tc_shape(c, nl, nr, n_atoms);
     if (sh.k_pad < BK) cl::fail(CL_ERR_STATE, "tensor-core Gram operands not reserved");
-    static bool smem_set = false;
-    if (!smem_set) {
-        ensure_smem(clk::tc::k_gram_tc, SMEM_BYTES);
-        smem_set = true;
-    }
+    ensure_smem(clk::tc::k_gram_tc, SMEM_BYTES);
     float* A = c->tc_buf.p;
     float* B = A + 2LL * sh.rowsA * sh.k_pad;
     const CUtensorMap mapA = tc_tensor_map(A, sh.k_pad, sh.rowsA, BM);
     const CUtensorMap mapB = tc_tensor_map(B, sh.k_pad, sh.rowsB, BN);
-    const int tilesA = (sh.rowsA + BM - 1) / BM, tilesB = (sh.rowsB + BN - 1) / BN;
-    const int tiles = tilesA * tilesB;
+    const clk::GramTiles gt = tc_tiles(plan, BM / 2, BN / 2);
+    const int tiles = clk::gram_tile_count(gt);
     for (long long a0 = 0; a0 < n_atoms; a0 += sh.chunk) {
         const long long na = std::min(sh.chunk, n_atoms - a0);
         const long long kp = (na + BK - 1) / BK * BK;  // k-tiles that hold atoms of this chunk
@@ -1456,8 +1541,8 @@ void gram_tc(cl_ctx* c, const void* V, bool v_f32, long long v_stride, int nl, c
         const int kt_per = (kt_total + best_s - 1) / best_s;
         const int splits = (kt_total + kt_per - 1) / kt_per;
         cudaEvent_t e1 = prof_begin(c);
-        clk::tc::k_gram_tc<<<dim3(tilesA, tilesB, splits), THREADS, SMEM_BYTES, c->stream>>>(
-            mapA, mapB, kt_total, kt_per, nl, nr, out4_dev);
+        clk::tc::k_gram_tc<<<dim3(tiles, splits), THREADS, SMEM_BYTES, c->stream>>>(
+            mapA, mapB, kt_total, kt_per, gt, out4_dev, out4_dev + (size_t)4 * nl * nr);
         CL_LAUNCHED();
         prof_end(c, e1, CL_KCLASS_GRAM, (double)tc_bytes_per_atom(sh.rowsA, sh.rowsB) * kp);
     }
@@ -1468,63 +1553,36 @@ void check_gram_slot(double slot) {
     if (slot != 0.0) cl::fail(CL_ERR_TIMEOUT, "tensor-core Gram: a device-side wait timed out");
 }
 
-// out4[l][r] = {sum ac, bd, ad, bc} over atoms (see k_gram); out4 holds 4 * nl * nr + 1
-// doubles, the last one an error slot.  The FP32 form runs the tensor-core Gram; the plain
-// form runs k_gram in FP64, whose register block IB (tile 16*IB) is the one that pads
-// max(nl, nr) least, preferring larger blocks.
-// rho: the right densities, complex64 when rho_f32 (the FP32 form's pair densities), else
-// complex128 (the plain form's, and the grid API's caller-given density).
-void gram(cl_ctx* c, const void* V_any, bool v_f32, long long v_stride, int nl, const void* rho_any, bool rho_f32,
-          long long r_stride, const int* ridx_dev, int nr, long long n_atoms, double* out4_dev) {
-    CL_CUDA(cudaMemsetAsync(out4_dev, 0, sizeof(double) * (4 * (size_t)nl * nr + 1), c->stream));
-    const bool small = small_gram(c, n_atoms);
-    if (small && v_f32 && rho_f32) {
-        gram_dmma(c, static_cast<const cx<float>*>(V_any), v_stride, nl, static_cast<const cx<float>*>(rho_any),
-                  r_stride, ridx_dev, nr, n_atoms, out4_dev);
-        return;
+// out4[l][r] = {sum ac, bd, ad, bc} over atoms for the pairs of the plan's blocks; out4 holds
+// 4 * nl * nr + 1 doubles, the last one an error slot.  rho: the right densities, complex64 when rho_f32
+// (the FP32 form's pair densities), else complex128 (the plain form's, and the grid API's caller-given
+// density).
+void gram(cl_ctx* c, const void* V_any, bool v_f32, long long v_stride, const void* rho_any, bool rho_f32,
+          long long r_stride, const int* ridx_dev, const GramPlan& plan, long long n_atoms, double* out4_dev) {
+    CL_CUDA(cudaMemsetAsync(out4_dev, 0, sizeof(double) * (4 * (size_t)plan.nl * plan.nr + 1), c->stream));
+    const auto* v32 = static_cast<const cx<float>*>(V_any);
+    const auto* v64 = static_cast<const cx<double>*>(V_any);
+    const auto* r32 = static_cast<const cx<float>*>(rho_any);
+    const auto* r64 = static_cast<const cx<double>*>(rho_any);
+    switch (gram_kind(c, plan, v_f32, rho_f32, n_atoms)) {
+        case GramKind::kFused:
+            if (!v_f32 || !rho_f32) cl::fail(CL_ERR_STATE, "the fused Gram needs FP32 operands");
+            gram_tc_fused(c, v32, v_stride, r32, r_stride, ridx_dev, plan, n_atoms, out4_dev);
+            break;
+        case GramKind::kSplit:
+            gram_tc_split(c, V_any, v_f32, v_stride, rho_any, rho_f32, r_stride, ridx_dev, plan, n_atoms, out4_dev);
+            break;
+        case GramKind::kFp64:
+            if (v_f32 && rho_f32)
+                gram_dmma(c, v32, v_stride, r32, r_stride, ridx_dev, plan, n_atoms, out4_dev);
+            else if (v_f32)
+                cl::fail(CL_ERR_STATE, "FP32 potentials go with FP32 densities");
+            else if (rho_f32)
+                gram_dmma(c, v64, v_stride, r32, r_stride, ridx_dev, plan, n_atoms, out4_dev);
+            else
+                gram_dmma(c, v64, v_stride, r64, r_stride, ridx_dev, plan, n_atoms, out4_dev);
+            break;
     }
-    if (use_tc_gram(c) && !small) {
-        gram_tc(c, V_any, v_f32, v_stride, nl, rho_any, rho_f32, r_stride, ridx_dev, nr, n_atoms, out4_dev);
-        return;
-    }
-    if (v_f32) cl::fail(CL_ERR_STATE, "the FP64 Gram needs FP64 potentials");
-    const cx<double>* V = static_cast<const cx<double>*>(V_any);
-    const int pmax = std::max(nl, nr);
-    int ib = 4;
-    long long best = -1;
-    for (int cand = 4; cand >= 1; --cand) {
-        const long long ts = 16 * cand, padded = (pmax + ts - 1) / ts * ts;
-        if (best < 0 || padded < best) { best = padded; ib = cand; }
-    }
-    const int ts = 16 * ib;
-    const int tl = (nl + ts - 1) / ts, tr = (nr + ts - 1) / ts;
-    long long want = std::max(1LL, (148LL * 4) / std::max(1, tl * tr));
-    long long per = std::max(256LL, (n_atoms + want - 1) / want);
-    per = (per + 15) / 16 * 16;
-    long long splits = std::max(1LL, (n_atoms + per - 1) / per);
-    if (splits > 65535) {
-        splits = 65535;
-        per = ((n_atoms + splits - 1) / splits + 15) / 16 * 16;
-    }
-    cudaEvent_t e = prof_begin(c);
-    const dim3 grid(tl, tr, (unsigned)splits);
-    // FP32 densities (the FP32 form with CL_NO_TC_GRAM) are widened as they are loaded
-    const auto launch = [&](auto tag) {
-        using RT = decltype(tag);
-        const cx<RT>* rho = static_cast<const cx<RT>*>(rho_any);
-        switch (ib) {
-            case 1: clk::k_gram<1, RT><<<grid, 256, 0, c->stream>>>(V, v_stride, nl, rho, r_stride, ridx_dev, nr, n_atoms, per, out4_dev); break;
-            case 2: clk::k_gram<2, RT><<<grid, 256, 0, c->stream>>>(V, v_stride, nl, rho, r_stride, ridx_dev, nr, n_atoms, per, out4_dev); break;
-            case 3: clk::k_gram<3, RT><<<grid, 256, 0, c->stream>>>(V, v_stride, nl, rho, r_stride, ridx_dev, nr, n_atoms, per, out4_dev); break;
-            default: clk::k_gram<4, RT><<<grid, 256, 0, c->stream>>>(V, v_stride, nl, rho, r_stride, ridx_dev, nr, n_atoms, per, out4_dev); break;
-        }
-    };
-    if (rho_f32)
-        launch(float{});
-    else
-        launch(double{});
-    CL_LAUNCHED();
-    prof_end(c, e, CL_KCLASS_GRAM, (double)n_atoms * (nl * 16.0 + nr * (rho_f32 ? 8.0 : 16.0)));
 }
 
 // Pair densities rho[p][atom] for products (fl[p], fr[p]) (0-based state indices): the
@@ -1914,8 +1972,9 @@ int cl_calculate_grid(cl_ctx* c, const double* rho2, double out[2]) {
         DevBuf<int> ridx;
         int zero = 0;
         ridx.upload(&zero, 1, c->stream);
-        tc_reserve(c, 1, 1, c->M, false, false);
-        gram(c, c->grid_V.p, false, c->M, 1, c->grid_rho2.p, false, c->M, ridx.p, 1, c->M, o4.p);
+        const GramPlan dot = whole_gram(1, 1, false);
+        tc_reserve(c, dot, c->M, false, false);
+        gram(c, c->grid_V.p, false, c->M, c->grid_rho2.p, false, c->M, ridx.p, dot, c->M, o4.p);
         double h[5];
         CL_CUDA(cudaMemcpyAsync(h, o4.p, sizeof h, cudaMemcpyDeviceToHost, c->stream));
         CL_CUDA(cudaStreamSynchronize(c->stream));
@@ -2142,19 +2201,150 @@ int cl_set_states(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, int n_o
 
 namespace {
 
+// The densities of a request: rows (left densities first), right columns, and the blocks of the Gram
+// that its steps read (gram_blocks.hpp).
+struct DensityLayout {
+    std::vector<int> prods, slot;   // product of each row; row of each product, -1: none
+    std::vector<int> rights, rcol;  // row of each right column; column of each product
+    std::vector<char> sym;          // per product: pairs with it are read with the larger product on the left
+    GramPlan gram;
+    // (state, state) of every row, 0-based, the higher first
+    std::vector<int2> states() const {
+        std::vector<int2> fl(prods.size());
+        for (size_t i = 0; i < prods.size(); ++i) {
+            int a, b;
+            cl::product_states(prods[i], &a, &b);
+            fl[i] = make_int2(a - 1, b - 1);
+        }
+        return fl;
+    }
+};
+
+// Symmetry needs the whole convolution (all 8 rounds).  The FP64 forms use it at any size (2); the FP32
+// forms, whose V_l rho_r and V_r rho_l differ by the transforms' rounding, only where it leaves out whole
+// 64 x 64 tiles (1), so that up to 64 densities a shard's integrals equal the full request's.
+int symmetric_blocks(const cl_ctx* c, int round_mask = 0xFF) {
+    return (round_mask & 0xFF) != 0xFF ? 0 : fp64_form(c) ? 2 : 1;
+}
+
+// Rows and columns go block by block, in ascending product order within a block; with `by_state` (the
+// overlapped upload) all left densities in one block, ordered by their higher state.  `symmetric`: which
+// blocks are treated as symmetric (symmetric_blocks).
+DensityLayout layout_densities(const std::vector<cl::PlanStep>& plan, int n_states, int symmetric, bool by_state) {
+    const int P = n_states * (n_states + 1) / 2;
+    std::vector<char> is_left(P, 0), is_right(P, 0);
+    for (const auto& st : plan) {
+        is_left[st.left.product] = 1;
+        is_right[st.right.product] = 1;
+    }
+    // connected components of the pairing (union-find; over as soon as one is left)
+    std::vector<int> root(P);
+    std::iota(root.begin(), root.end(), 0);
+    const auto find = [&](int p) {
+        while (root[p] != p) p = root[p] = root[root[p]];
+        return p;
+    };
+    int parts = 0;
+    for (int p = 0; p < P; ++p) parts += is_left[p] || is_right[p];
+    for (size_t i = 0; i < plan.size() && parts > 1; ++i) {
+        const int a = find(plan[i].left.product), b = find(plan[i].right.product);
+        if (a == b) continue;
+        root[std::max(a, b)] = std::min(a, b);
+        --parts;
+    }
+    struct Part {
+        std::vector<int> lefts, rights;
+    };
+    std::vector<Part> found;
+    std::vector<int> id(P, -1);
+    for (int p = 0; p < P; ++p) {
+        if (!is_left[p] && !is_right[p]) continue;
+        int& k = id[find(p)];
+        if (k < 0) {
+            k = (int)found.size();
+            found.emplace_back();
+        }
+        if (is_left[p]) found[k].lefts.push_back(p);
+        if (is_right[p]) found[k].rights.push_back(p);
+    }
+    // parts of fewer than 4 densities (half an MMA tile) share one block, and so do the smallest beyond
+    // the blocks a launch can hold
+    std::stable_sort(found.begin(), found.end(), [](const Part& a, const Part& b) {
+        return a.lefts.size() + a.rights.size() > b.lefts.size() + b.rights.size();
+    });
+    const auto small = [](const Part& q) { return q.lefts.size() < 4 && q.rights.size() < 4; };
+    while (found.size() > 1 && ((int)found.size() > clk::kGramBlocks || (small(found.back()) && small(found[found.size() - 2])))) {
+        Part last = std::move(found.back());
+        found.pop_back();
+        Part& into = found.back();
+        into.lefts.insert(into.lefts.end(), last.lefts.begin(), last.lefts.end());
+        into.rights.insert(into.rights.end(), last.rights.begin(), last.rights.end());
+    }
+    DensityLayout d;
+    d.slot.assign(P, -1);
+    d.rcol.assign(P, -1);
+    d.sym.assign(P, 0);
+    std::vector<char> part_sym;
+    for (Part& q : found) {
+        std::sort(q.lefts.begin(), q.lefts.end());
+        std::sort(q.rights.begin(), q.rights.end());
+        const bool sym = (symmetric == 2 || (symmetric == 1 && q.lefts.size() > 64)) && q.lefts == q.rights;
+        part_sym.push_back(sym);
+        if (sym)
+            for (int p : q.lefts) d.sym[p] = 1;
+    }
+    const bool all_sym = std::find(part_sym.begin(), part_sym.end(), 0) == part_sym.end();
+    if (by_state) {
+        Part all;
+        for (int p = 0; p < P; ++p) {
+            if (is_left[p]) all.lefts.push_back(p);  // ascending products: ascending higher states
+            if (is_right[p]) all.rights.push_back(p);
+        }
+        found.assign(1, std::move(all));
+        part_sym.assign(1, all_sym);
+    }
+    for (size_t k = 0; k < found.size(); ++k) {
+        const Part& q = found[k];
+        d.gram.blocks.push_back(clk::GramBlock{(int)d.prods.size(), (int)q.lefts.size(), (int)d.rights.size(),
+                                               (int)q.rights.size(), part_sym[k]});
+        for (int p : q.lefts) {
+            d.slot[p] = (int)d.prods.size();
+            d.prods.push_back(p);
+        }
+        for (int p : q.rights) {
+            d.rcol[p] = (int)d.rights.size();
+            d.rights.push_back(p);  // the product; its row below
+        }
+    }
+    d.gram.nl = (int)d.prods.size();
+    d.gram.nr = (int)d.rights.size();
+    d.gram.whole = clk::GramBlock{0, d.gram.nl, 0, d.gram.nr, all_sym};
+    for (int p : d.rights)
+        if (d.slot[p] < 0) {
+            d.slot[p] = (int)d.prods.size();
+            d.prods.push_back(p);
+        }
+    for (int& r : d.rights) r = d.slot[r];
+    return d;
+}
+
 // Step values (coulombo.cpp:199-207): step s takes the Gram entry of its (left, right) pair,
 // combined for the pair's conjugation flags and conjugated when the left product is.  Long
 // integral lists are mapped on several host threads.
-void map_step_values(const std::vector<cl::PlanStep>& plan, const std::vector<int>& slot,
-                     const std::vector<int>& rcol, int nr, const double* h, double* out) {
+void map_step_values(const std::vector<cl::PlanStep>& plan, const DensityLayout& d, const double* h, double* out) {
+    const int nr = d.gram.nr;
     const auto work = [&](size_t i0, size_t i1) {
         for (size_t i = i0; i < i1; ++i) {
             const auto& st = plan[i];
-            const int l = slot[st.left.product], r = rcol[st.right.product];
+            // a symmetric block holds the pairs with the larger product on the left
+            const bool turned = d.sym[st.left.product] && st.left.product < st.right.product;
+            const int l = d.slot[turned ? st.right.product : st.left.product];
+            const int r = d.rcol[turned ? st.left.product : st.right.product];
             const double* q = &h[((size_t)l * nr + r) * 4];
+            const double ad = turned ? q[3] : q[2], bc = turned ? q[2] : q[3];
             const bool rconj = st.left.conjugate != st.right.conjugate;
             const double re = rconj ? q[0] + q[1] : q[0] - q[1];
-            double im = rconj ? q[3] - q[2] : q[2] + q[3];
+            double im = rconj ? bc - ad : ad + bc;
             if (st.left.conjugate) im = -im;
             out[2 * st.id] = re;
             out[2 * st.id + 1] = im;
@@ -2206,29 +2396,10 @@ void compute_impl(cl_ctx* c, int64_t n_int, const int16_t* spec, double* out, in
         const auto plan = shard_steps(cl::orient_steps(c->n_states, specs), c->n_states, shard, n_shards);
         if (n_shards > 1) std::memset(out, 0, sizeof(double) * 2 * (size_t)n_int);
         if (plan.empty()) return;
-        // densities: prepared (left) products first, then right-only products
-        const int P = c->n_states * (c->n_states + 1) / 2;
-        std::vector<int> slot(P, -1), is_left(P, 0), is_right(P, 0);
-        for (const auto& s : plan) {
-            is_left[s.left.product] = 1;
-            is_right[s.right.product] = 1;
-        }
-        std::vector<int> prods;
-        for (int p = 0; p < P; ++p)
-            if (is_left[p]) { slot[p] = (int)prods.size(); prods.push_back(p); }
-        const int nl = (int)prods.size();
-        for (int p = 0; p < P; ++p)
-            if (is_right[p] && slot[p] < 0) { slot[p] = (int)prods.size(); prods.push_back(p); }
-        std::vector<int> rights, rcol(P, -1);
-        for (int p = 0; p < P; ++p)
-            if (is_right[p]) { rcol[p] = (int)rights.size(); rights.push_back(slot[p]); }
-        const int nu = (int)prods.size(), nr = (int)rights.size();
-        std::vector<int2> fl(nu);
-        for (int i = 0; i < nu; ++i) {
-            int a, b;
-            cl::product_states(prods[i], &a, &b);
-            fl[i] = make_int2(a - 1, b - 1);
-        }
+        const DensityLayout lay = layout_densities(plan, c->n_states, symmetric_blocks(c, round_mask), false);
+        const std::vector<int>& rights = lay.rights;
+        const std::vector<int2> fl = lay.states();
+        const int nu = (int)lay.prods.size(), nl = lay.gram.nl, nr = lay.gram.nr;
         const long long As = c->n_sorted;
         DevBuf<int>& dr = c->req_ridx;
         grow(dr, rights.size());
@@ -2239,14 +2410,14 @@ void compute_impl(cl_ctx* c, int64_t n_int, const int16_t* spec, double* out, in
         grow(V, (size_t)nl * As);
         DevBuf<double>& o4 = c->req_o4;
         grow(o4, (size_t)4 * nl * nr + 1);
-        tc_reserve(c, nl, nr, As, v_fp32(c), rho_bytes(c) == sizeof(cx<float>));
+        tc_reserve(c, lay.gram, As, v_fp32(c), rho_bytes(c) == sizeof(cx<float>));
         CL_CUDA(cudaEventRecord(c->ev[0], c->stream));
         pair_densities(c, fl, rho.p);
         CL_CUDA(cudaEventRecord(c->ev[1], c->stream));
         const bool v32 = v_fp32(c);
         run_transforms(c, rho.p, As, nl, V.p, As, v32, round_mask);
         CL_CUDA(cudaEventRecord(c->ev[2], c->stream));
-        gram(c, V.p, v32, As, nl, rho.p, rho_bytes(c) == sizeof(cx<float>), As, dr.p, nr, As, o4.p);
+        gram(c, V.p, v32, As, rho.p, rho_bytes(c) == sizeof(cx<float>), As, dr.p, lay.gram, As, o4.p);
         CL_CUDA(cudaEventRecord(c->ev[3], c->stream));
         std::vector<double> h((size_t)4 * nl * nr + 1);
         CL_CUDA(cudaMemcpyAsync(h.data(), o4.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -2262,7 +2433,7 @@ void compute_impl(cl_ctx* c, int64_t n_int, const int16_t* spec, double* out, in
         c->timings[2] = t23;
         c->timings[3] = t03;
         prof_collect(c);
-        map_step_values(plan, slot, rcol, nr, h.data(), out);
+        map_step_values(plan, lay, h.data(), out);
     }
 }
 
@@ -2330,32 +2501,11 @@ void compute_states_impl(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, 
             upload_through(n_states - 1);
         cudaGetLastError();  // pageable memory is not an error
     }
-    const int P = n_states * (n_states + 1) / 2;
-    std::vector<int> is_left(P, 0), is_right(P, 0);
-    for (const auto& st : plan) {
-        is_left[st.left.product] = 1;
-        is_right[st.right.product] = 1;
-    }
-    // product -> (higher, lower) 0-based state
-    auto states_of = [](int p) {
-        int a, b;
-        cl::product_states(p, &a, &b);
-        return std::make_pair(a - 1, b - 1);
-    };
-    // left densities ordered by their higher state (stable), then right-only densities
-    std::vector<int> lefts, prods, slot(P, -1);
-    for (int p = 0; p < P; ++p)
-        if (is_left[p]) lefts.push_back(p);
-    std::stable_sort(lefts.begin(), lefts.end(),
-                     [&](int x, int y) { return states_of(x).first < states_of(y).first; });
-    for (int p : lefts) { slot[p] = (int)prods.size(); prods.push_back(p); }
-    const int nl = (int)lefts.size();
-    for (int p = 0; p < P; ++p)
-        if (is_right[p] && slot[p] < 0) { slot[p] = (int)prods.size(); prods.push_back(p); }
-    std::vector<int> rights, rcol(P, -1);
-    for (int p = 0; p < P; ++p)
-        if (is_right[p]) { rcol[p] = (int)rights.size(); rights.push_back(slot[p]); }
-    const int nu = (int)prods.size(), nr = (int)rights.size();
+    // left densities ordered by their higher state, then right-only densities
+    const DensityLayout lay = layout_densities(plan, n_states, symmetric_blocks(c), true);
+    const std::vector<int>& rights = lay.rights;
+    const std::vector<int2> rows = lay.states();
+    const int nu = (int)lay.prods.size(), nl = lay.gram.nl, nr = lay.gram.nr;
     // groups of left densities: cut at a state boundary once a group holds nl/6 densities
     struct Group {
         int begin, end, last_state;
@@ -2365,9 +2515,9 @@ void compute_states_impl(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, 
     const int min_group = std::max(1, nl / 6);
     for (int i = 0; i < nl;) {
         int j = i;
-        int hi = states_of(prods[i]).first;
-        while (j < nl && (j - i < min_group || states_of(prods[j]).first == hi)) {
-            hi = std::max(hi, states_of(prods[j]).first);
+        int hi = rows[i].x;
+        while (j < nl && (j - i < min_group || rows[j].x == hi)) {
+            hi = std::max(hi, rows[j].x);
             ++j;
         }
         auto g = std::make_unique<Group>();
@@ -2377,14 +2527,7 @@ void compute_states_impl(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, 
         groups.push_back(std::move(g));
         i = j;
     }
-    auto pairs_of = [&](int b, int e) {
-        std::vector<int2> fl;
-        for (int i = b; i < e; ++i) {
-            const auto st = states_of(prods[i]);
-            fl.push_back(make_int2(st.first, st.second));
-        }
-        return fl;
-    };
+    auto pairs_of = [&](int b, int e) { return std::vector<int2>(rows.begin() + b, rows.begin() + e); };
     for (auto& g : groups) pair_setup(c, pairs_of(g->begin, g->end), g->ps);
     PairSetup ps_right;
     if (nu > nl) pair_setup(c, pairs_of(nl, nu), ps_right);
@@ -2399,7 +2542,7 @@ void compute_states_impl(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, 
     grow(V, (size_t)nl * As);
     DevBuf<double>& o4 = c->req_o4;
     grow(o4, (size_t)4 * nl * nr + 1);
-    tc_reserve(c, nl, nr, As, v_fp32(c), rho_bytes(c) == sizeof(cx<float>));
+    tc_reserve(c, lay.gram, As, v_fp32(c), rho_bytes(c) == sizeof(cx<float>));
     CL_CUDA(cudaStreamSynchronize(c->stream));
     for (auto& g : groups) {
         upload_through(g->last_state);
@@ -2412,7 +2555,7 @@ void compute_states_impl(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, 
     CL_CUDA(cudaStreamWaitEvent(c->stream, c->state_ev[n_states - 1], 0));
     if (nu > nl) pair_launch(c, ps_right, rho_at(c, rho.p, (long long)nl * As));
     CL_CUDA(cudaEventRecord(c->ev[2], c->stream));
-    gram(c, V.p, v32, As, nl, rho.p, rho_bytes(c) == sizeof(cx<float>), As, dr.p, nr, As, o4.p);
+    gram(c, V.p, v32, As, rho.p, rho_bytes(c) == sizeof(cx<float>), As, dr.p, lay.gram, As, o4.p);
     CL_CUDA(cudaEventRecord(c->ev[3], c->stream));
     std::vector<double> h((size_t)4 * nl * nr + 1);
     CL_CUDA(cudaMemcpyAsync(h.data(), o4.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -2428,7 +2571,7 @@ void compute_states_impl(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, 
     c->timings[2] = t23;
     c->timings[3] = t03;
     prof_collect(c);
-    map_step_values(plan, slot, rcol, nr, h.data(), out);
+    map_step_values(plan, lay, h.data(), out);
 }
 }  // namespace
 
@@ -2526,7 +2669,7 @@ struct cl_request {
     cl_ctx* ctx = nullptr;
     int64_t n_int = 0;
     std::vector<cl::PlanStep> plan;
-    std::vector<int> slot, rcol;
+    DensityLayout lay;
     int nl = 0, nr = 0;
     PairSetup ps;
     DevBuf<int> ridx;
@@ -2574,7 +2717,7 @@ void request_enqueue(cl_request* r) {
     pair_launch(c, r->ps, r->rho.p);
     const bool v32 = v_fp32(c);
     run_transforms(c, r->rho.p, As, r->nl, r->V.p, As, v32);
-    gram(c, r->V.p, v32, As, r->nl, r->rho.p, rho_bytes(c) == sizeof(cx<float>), As, r->ridx.p, r->nr, As, r->o4.p);
+    gram(c, r->V.p, v32, As, r->rho.p, rho_bytes(c) == sizeof(cx<float>), As, r->ridx.p, r->lay.gram, As, r->o4.p);
     CL_CUDA(cudaMemcpyAsync(r->o4_host, r->o4.p, sizeof(double) * (4 * (size_t)r->nl * r->nr + 1),
                             cudaMemcpyDeviceToHost, c->stream));
 }
@@ -2583,7 +2726,7 @@ void request_finish(cl_request* r, double* out) {
     if (r->n_shards > 1) std::memset(out, 0, sizeof(double) * 2 * (size_t)r->n_int);
     if (r->nl == 0) return;
     check_gram_slot(r->o4_host[4 * (size_t)r->nl * r->nr]);
-    map_step_values(r->plan, r->slot, r->rcol, r->nr, r->o4_host, out);
+    map_step_values(r->plan, r->lay, r->o4_host, out);
 }
 
 }  // namespace
@@ -2616,37 +2759,19 @@ int cl_request_create_shard(cl_ctx* c, int64_t n_int, const int16_t* spec, int s
             *out = r;
             return;
         }
-        const int P = c->n_states * (c->n_states + 1) / 2;
-        std::vector<int> is_left(P, 0), is_right(P, 0);
-        r->slot.assign(P, -1);
-        r->rcol.assign(P, -1);
-        for (const auto& s : r->plan) {
-            is_left[s.left.product] = 1;
-            is_right[s.right.product] = 1;
-        }
-        std::vector<int> prods, rights;
-        for (int p = 0; p < P; ++p)
-            if (is_left[p]) { r->slot[p] = (int)prods.size(); prods.push_back(p); }
-        r->nl = (int)prods.size();
-        for (int p = 0; p < P; ++p)
-            if (is_right[p] && r->slot[p] < 0) { r->slot[p] = (int)prods.size(); prods.push_back(p); }
-        for (int p = 0; p < P; ++p)
-            if (is_right[p]) { r->rcol[p] = (int)rights.size(); rights.push_back(r->slot[p]); }
-        r->nr = (int)rights.size();
-        std::vector<int2> fl(prods.size());
-        for (size_t i = 0; i < prods.size(); ++i) {
-            int a, b;
-            cl::product_states(prods[i], &a, &b);
-            fl[i] = make_int2(a - 1, b - 1);
-        }
+        r->lay = layout_densities(r->plan, c->n_states, symmetric_blocks(c), false);
+        r->nl = r->lay.gram.nl;
+        r->nr = r->lay.gram.nr;
+        const std::vector<int>& rights = r->lay.rights;
+        const std::vector<int2> fl = r->lay.states();
         const long long As = c->n_sorted;
         pair_setup(c, fl, r->ps);
         r->ridx.upload(rights.data(), rights.size(), c->stream);
-        r->rho.alloc((size_t)prods.size() * As);
+        r->rho.alloc(fl.size() * As);
         r->V.alloc((size_t)r->nl * As);
         r->o4.alloc((size_t)4 * r->nl * r->nr + 1);
         CL_CUDA(cudaMallocHost(&r->o4_host, sizeof(double) * (4 * (size_t)r->nl * r->nr + 1)));
-        tc_reserve(c, r->nl, r->nr, As, v_fp32(c), rho_bytes(c) == sizeof(cx<float>));
+        tc_reserve(c, r->lay.gram, As, v_fp32(c), rho_bytes(c) == sizeof(cx<float>));
         CL_CUDA(cudaStreamSynchronize(c->stream));
         *out = r;
     });

@@ -1,55 +1,73 @@
-// FP64 tensor-core Gram over atoms for FP32 operands (FP32 potentials and pair densities).
+// FP64 tensor-core Gram over atoms, for every reduction that is summed in FP64: the FP64 forms, the FP32
+// forms' small boxes and FP64 potentials.
 //
 // The reductions of CoulombCalculator::calculate (CoulombCalculator.cpp:165-172) restricted to
-// atom cells and batched over every (left, right) pair of a request, as in gram_tc.cuh:
+// atom cells and batched over the (left, right) pairs of a request, as in gram_tc.cuh:
 //   C = A . B^T,  A rows = {Re V_l, Im V_l},  B rows = {Re rho_r, Im rho_r},  K = atoms,
-// here with FP64 products and FP64 sums on the FP64 tensor cores (mma.sync m8n8k4 .f64): the
-// FP32 operands are widened exactly, so the only rounding left is that of FP64 accumulation.
+// with FP64 products and FP64 sums on the FP64 tensor cores (mma.sync m8n8k4 .f64): FP32 operands are
+// widened exactly, so the only rounding is that of FP64 accumulation.
 //
-// A block takes up to 64 left and 64 right densities (a 128 x 128 tile of C) and an atom range,
-// in chunks of 32 atoms:
-//   copy     8-byte cp.async of the chunk's raw complex values into one of two raw slots, a
-//            chunk ahead ([density][36] complex float; thread e takes element e + 256 j, atom
-//            e % 32 of density e / 32: 256 contiguous bytes a warp);
-//   widen    each thread widens the elements it copied itself into the FP64 stage of the next
-//            chunk ([density][36] complex double; the pitch of 36 puts the 16 lanes of a
-//            fragment load on distinct banks);
-//   multiply 8 warps in a 2 x 4 grid over the C tiles of 8 x 8: warp (wr, wc) holds the tiles
-//            (wr + 2a, wc + 4b); per k-step of 4 atoms it loads one A fragment per row tile and
-//            one B fragment per column tile and issues one mma per tile.
-// One barrier per chunk separates the widening of chunk c + 1 from the reads of chunk c - 1's
-// stage.  Left densities are staged at [0, nA4), right ones at [nA4, nA4 + nB4), each count
-// rounded up to 4 with zero rows, so every fragment of a partial 8-row tile reads staged zeros.
+// A block takes one tile of the Gram (gram_blocks.hpp) and an atom range, in chunks of KC atoms (32, or 64
+// where the warps split the atoms and the box has enough of them, so that a chunk's barrier and copies
+// are spread over more MMAs):
+//   copy      cp.async of the chunk's raw complex values, 1 to 3 chunks ahead ([density][KC + 4], 16
+//             bytes a copy, 8 for FP32 rows that do not start on a 16-byte boundary);
+//   multiply  8 warps as WR x WC x KS: warp (wr, wc, ks) holds the 8 x 8 tiles (wr + WR a, wc + WC b) of
+//             C, a < A, b < B, over every KS-th k-step of 4 atoms.  A fragment value is one shared load
+//             (re or im of an operand value; the pitch of KC + 4 puts a warp's 32 on distinct banks) and,
+//             for FP32 operands, one conversion.
+// At the end the KS partial sums are added through shared memory and the results go to out4 with FP64
+// atomics.  Every MMA of the A x B register tile is issued whether its rows exist or not (a predicated-off
+// one takes its 16 pipe cycles all the same), so the host picks A, B and the warp grid to fit: splitting
+// the warps over atoms keeps them at full register tiles (20 densities a side: 5 x 5 tiles, which a
+// 2 x 4 grid of 3 x 2 would fill to 52 %).
+//
+// Bound: the FP64 tensor pipe (64 FMA a clock and SM measured, 18.2 T FMA/s) at many densities, the
+// latency of the chunks of a small box at few.  Measured on a B200 against the kernels this one replaced
+// (register products for FP64 operands; every pair of densities, FP32 operands widened into a second
+// stage, a 2 x 4 warp grid for any tile): 96^3 box, 12 states in FP64 (42 and 36 densities, 6 symmetric
+// tiles) 0.898 -> 0.186 ms, the FP64 tensor pipe half busy; six boxes of 13,824 to 24,192 atoms, 8
+// states, FP32: 0.346 -> 0.144 ms; 64^3 grid product 0.085 -> 0.027 ms; 4,096 atoms, 4 states,
+// 18.9 -> 10.0 us.
 #pragma once
 
 #include <cstdint>
 
 #include "fft.cuh"
+#include "gram_blocks.hpp"
 
 namespace clk {
 namespace dm {
 
-constexpr int TILE = 128;          // C rows (left re/im rows) and columns per block
-constexpr int KC = 32;             // atoms per chunk
-constexpr int PITCH = KC + 4;      // complex elements per staged density
-constexpr int THREADS = 256;
-constexpr int MAX_DENS = TILE;     // staged densities per block (64 left + 64 right, rounded)
+__host__ __device__ constexpr int pitch(int kc) { return kc + 4; }  // complex elements per staged density
+constexpr int WARPS = 8;
+constexpr int THREADS = 32 * WARPS;
+constexpr int WIDTH = 64;      // densities a tile side, at most
 
+template <typename S>
 struct GramArgs {
-    const float2* V;      // left densities: V[l * v_stride + atom]
+    const cx<S>* V;       // left densities: V[l * v_stride + atom]
     long long v_stride;
-    const float2* rho;    // right densities: rho[(ridx ? ridx[r] : r) * r_stride + atom]
-    long long r_stride;
-    const int* ridx;
+    const int* ridx;      // right densities: rho[(ridx ? ridx[r] : r) * r_stride + atom]
     int nl, nr;
+    long long r_stride;
     long long na;               // atoms
-    long long atoms_per_split;  // a multiple of KC
-    int nd_max;                 // staged densities of the largest block (nA4 + nB4)
+    long long atoms_per_split;  // a multiple of the chunk
+    int stages;                 // chunks in shared memory
+    int nd_a, nd_b;             // staged densities of the largest tile, a side (multiples of 4)
+    int wr, wc;                 // warp grid over the C tile; 8 / (wr * wc) k slices
+    int align_v, align_r;       // every row of the operand starts on a 16-byte boundary
     double* out4;               // out4[l][r] += {ac, bd, ad, bc}
+    GramTiles tiles;
 };
 
-__host__ __device__ constexpr size_t smem_bytes(int nd_max) {
-    return (size_t)nd_max * PITCH * (2 * 16 + 2 * 8) + sizeof(void*) * MAX_DENS;
+template <typename SV, typename SR>
+__host__ __device__ constexpr size_t stage_bytes(int kc, int nd_a, int nd_b) {
+    return (size_t)pitch(kc) * (nd_a * sizeof(cx<SV>) + nd_b * sizeof(cx<SR>));
+}
+// Shared memory of the reduction over k slices: half the slices' sums at a time.
+__host__ __device__ constexpr size_t reduce_bytes(int a, int b, int slices) {
+    return slices > 1 ? (size_t)(WARPS / 2) * a * b * 2 * 32 * sizeof(double) : 0;
 }
 
 __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
@@ -57,136 +75,151 @@ __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
                  : "+d"(d[0]), "+d"(d[1])
                  : "d"(a), "d"(b));
 }
-__device__ __forceinline__ void cp_async8_zfill(void* dst, const void* src, bool in) {
+template <int BYTES>
+__device__ __forceinline__ void cp_async_part(void* dst, const void* src, unsigned bytes) {
     const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(in ? 8u : 0u) : "memory");
+    if constexpr (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
 }
 
-__global__ void __launch_bounds__(THREADS, 1) k_gram_dmma(const GramArgs g) {
+// Copies atoms [k0, k0 + KC) of n densities (rows beyond n, up to n4, and atoms beyond k_end as zeros).
+template <int KC, typename S, typename ROW>
+__device__ __forceinline__ void copy_chunk(cx<S>* dst, int n, int n4, long long k0, long long k_end, bool aligned,
+                                           const cx<S>* any, ROW&& row) {
+    constexpr int PITCH = pitch(KC), PER = 16 / sizeof(cx<S>);  // PER: atoms per 16-byte copy
+    if (aligned) {
+        for (int e = threadIdx.x; e < n4 * (KC / PER); e += THREADS) {
+            const int i = e / (KC / PER), k = (e % (KC / PER)) * PER;
+            const long long left = i < n ? k_end - (k0 + k) : 0;
+            const unsigned bytes = left >= PER ? 16u : left > 0 ? (unsigned)(left * sizeof(cx<S>)) : 0u;
+            cp_async_part<16>(dst + i * PITCH + k, bytes ? row(i) + k0 + k : any, bytes);
+        }
+    } else {
+        for (int e = threadIdx.x; e < n4 * KC; e += THREADS) {
+            const int i = e / KC, k = e % KC;
+            const bool in = i < n && k0 + k < k_end;
+            if constexpr (sizeof(cx<S>) == 16)
+                cp_async_part<16>(dst + i * PITCH + k, in ? row(i) + k0 + k : any, in ? 16u : 0u);
+            else
+                cp_async_part<8>(dst + i * PITCH + k, in ? row(i) + k0 + k : any, in ? 8u : 0u);
+        }
+    }
+}
+
+template <typename SV, typename SR, int KC, int A, int B>
+__global__ void __launch_bounds__(THREADS, 1) k_gram_dmma(const cx<SR>* __restrict__ rho, const GramArgs<SV> g) {
+    constexpr int PITCH = pitch(KC);
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double2* stage = reinterpret_cast<double2*>(smem_raw);                 // [2][nd_max][PITCH]
-    float2* raw = reinterpret_cast<float2*>(stage + 2 * g.nd_max * PITCH);  // [2][nd_max][PITCH]
-    const float2** src_tab = reinterpret_cast<const float2**>(raw + 2 * g.nd_max * PITCH);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * TILE, n0 = blockIdx.y * TILE;
-    const int la0 = m0 / 2, rb0 = n0 / 2;
-    const int nA = min(TILE / 2, g.nl - la0), nB = min(TILE / 2, g.nr - rb0);
-    const int nA4 = (nA + 3) & ~3, nB4 = (nB + 3) & ~3;
-    const int nd = nA4 + nB4;
-    const int ta = (2 * nA + 7) / 8, tb = (2 * nB + 7) / 8;  // 8-row tiles of C
-    const long long k_begin = (long long)blockIdx.z * g.atoms_per_split;
+    __shared__ int right_row[WIDTH];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    GramTile tile;
+    gram_tile(g.tiles, blockIdx.x, &tile);
+    const int nA4 = (tile.nl + 3) & ~3, nB4 = (tile.nr + 3) & ~3;
+    const int ta = nA4 / 4, tb = nB4 / 4;  // 8-row tiles of C
+    const long long k_begin = (long long)blockIdx.y * g.atoms_per_split;
     const long long k_end = min(g.na, k_begin + g.atoms_per_split);
     const int nc = (int)((k_end - k_begin + KC - 1) / KC);
-
-    for (int i = tid; i < nd; i += THREADS) {
-        const float2* p = nullptr;
-        if (i < nA) {
-            p = g.V + (long long)(la0 + i) * g.v_stride;
-        } else if (i >= nA4 && i < nA4 + nB) {
-            const int r = rb0 + (i - nA4);
-            p = g.rho + (long long)(g.ridx ? g.ridx[r] : r) * g.r_stride;
-        }
-        src_tab[i] = p;  // null: a zero row
-    }
+    const size_t stage = stage_bytes<SV, SR>(KC, g.nd_a, g.nd_b);
+    const size_t b_off = (size_t)PITCH * g.nd_a * sizeof(cx<SV>);
+    for (int r = threadIdx.x; r < tile.nr; r += THREADS)
+        right_row[r] = g.ridx ? g.ridx[tile.r0 + r] : tile.r0 + r;
     __syncthreads();
-
-    // this thread's elements of a chunk: e = tid + 256 j < nd * KC
     const auto issue = [&](int c) {
-        float2* slot = raw + (c & 1) * g.nd_max * PITCH;
+        unsigned char* st = smem_raw + (size_t)(c % g.stages) * stage;
         const long long k0 = k_begin + (long long)c * KC;
-        for (int e = tid; e < nd * KC; e += THREADS) {
-            const int i = e / KC, k = e % KC;
-            const float2* p = src_tab[i];
-            const bool in = p != nullptr && k0 + k < k_end;
-            cp_async8_zfill(slot + i * PITCH + k, in ? p + k0 + k : g.V, in);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        copy_chunk<KC, SV>(reinterpret_cast<cx<SV>*>(st), tile.nl, nA4, k0, k_end, g.align_v, g.V,
+                       [&](int i) { return g.V + (long long)(tile.l0 + i) * g.v_stride; });
+        copy_chunk<KC, SR>(reinterpret_cast<cx<SR>*>(st + b_off), tile.nr, nB4, k0, k_end, g.align_r, rho,
+                       [&](int i) { return rho + (long long)right_row[i] * g.r_stride; });
     };
-    const auto widen_chunk = [&](int c) {
-        const float2* slot = raw + (c & 1) * g.nd_max * PITCH;
-        double2* st = stage + (c & 1) * g.nd_max * PITCH;
-        for (int e = tid; e < nd * KC; e += THREADS) {
-            const int i = e / KC, k = e % KC;
-            const float2 v = slot[i * PITCH + k];
-            st[i * PITCH + k] = make_double2((double)v.x, (double)v.y);
-        }
-    };
-
-    // warp grid 2 x 4 over the C tiles
-    const int wr = warp & 1, wc = warp >> 1;
+    const int slices = WARPS / (g.wr * g.wc);
+    const int ks0 = warp % slices, wr = warp / slices % g.wr, wc = warp / slices / g.wr;
     const int grp = lane >> 2, tig = lane & 3;
-    double acc[8][4][2];
+    double acc[A][B][2];
 #pragma unroll
-    for (int a = 0; a < 8; ++a)
+    for (int a = 0; a < A; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-
-    if (nc > 0) {
-        issue(0);
-        if (nc > 1) issue(1);
-        if (nc > 1)
+        for (int b = 0; b < B; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    for (int c = 0; c < g.stages - 1; ++c) {
+        if (c < nc) issue(c);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+#pragma unroll 1
+    for (int c = 0; c < nc; ++c) {
+        // chunk c has landed: all but the newest stages - 2 groups of this thread are complete
+        if (g.stages == 4)
+            asm volatile("cp.async.wait_group 2;" ::: "memory");
+        else if (g.stages == 3)
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         else
             asm volatile("cp.async.wait_group 0;" ::: "memory");
-        widen_chunk(0);
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int c = 0; c < nc; ++c) {
-        if (c + 1 < nc) {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");  // chunk c + 1 (this thread's copies)
-            widen_chunk(c + 1);
-            if (c + 2 < nc) issue(c + 2);  // into the raw slot of chunk c, widened last iteration
-        }
-        const double2* st = stage + (c & 1) * g.nd_max * PITCH;
+        __syncthreads();  // everyone's copies of chunk c, and everyone is done with chunk c - 1
+        if (c + g.stages - 1 < nc) issue(c + g.stages - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const unsigned char* st = smem_raw + (size_t)(c % g.stages) * stage;
+        const SV* sa = reinterpret_cast<const SV*>(st) + (size_t)(grp >> 1) * (2 * PITCH) + (grp & 1);
+        const SR* sb = reinterpret_cast<const SR*>(st + b_off) + (size_t)(grp >> 1) * (2 * PITCH) + (grp & 1);
 #pragma unroll 2
-        for (int ks = 0; ks < KC / 4; ++ks) {
-            const int k = ks * 4 + tig;
-            double af[8], bf[4];
+        for (int ks = ks0; ks < KC / 4; ks += slices) {
+            const int k = 2 * (ks * 4 + tig);
+            double af[A], bf[B];
 #pragma unroll
-            for (int a = 0; a < 8; ++a) {
-                const int ti = wr + 2 * a;
-                const int row = ti * 8 + grp;  // re/im row of left density row / 2 (< nA4)
-                af[a] = 0.0;
-                if (ti < ta) {
-                    const double2 v = st[(row >> 1) * PITCH + k];
-                    af[a] = (row & 1) ? v.y : v.x;
-                }
+            for (int a = 0; a < A; ++a) {
+                const int ti = wr + g.wr * a;
+                af[a] = ti < ta ? (double)sa[ti * (8 * PITCH) + k] : 0.0;
             }
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const int tj = wc + 4 * b;
-                const int col = tj * 8 + grp;  // re/im row of right density col / 2 (< nB4)
-                bf[b] = 0.0;
-                if (tj < tb) {
-                    const double2 v = st[(nA4 + (col >> 1)) * PITCH + k];
-                    bf[b] = (col & 1) ? v.y : v.x;
-                }
+            for (int b = 0; b < B; ++b) {
+                const int tj = wc + g.wc * b;
+                bf[b] = tj < tb ? (double)sb[tj * (8 * PITCH) + k] : 0.0;
             }
 #pragma unroll
-            for (int a = 0; a < 8; ++a)
+            for (int a = 0; a < A; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b)
-                    if (wr + 2 * a < ta && wc + 4 * b < tb) mma_f64(acc[a][b], af[a], bf[b]);
+                for (int b = 0; b < B; ++b) mma_f64(acc[a][b], af[a], bf[b]);
         }
-        __syncthreads();  // stage c & 1 is rewritten by the widening of chunk c + 2
     }
-
+    // the k slices' sums: the upper half of the slices hands its sums to the lower half, until one is left
+    double* red = reinterpret_cast<double*>(smem_raw);
+#pragma unroll 1
+    for (int h = slices / 2; h >= 1; h /= 2) {
+        double* mine = red + (size_t)((warp / slices) * h + (ks0 & (h - 1))) * (A * B * 2 * 32) + lane;
+        __syncthreads();
+        if (ks0 >= h && ks0 < 2 * h) {
 #pragma unroll
-    for (int a = 0; a < 8; ++a)
+            for (int a = 0; a < A; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int ti = wr + 2 * a, tj = wc + 4 * b;
-            if (ti >= ta || tj >= tb) continue;
-            const int R = m0 + ti * 8 + grp;
-            const int l = R >> 1, pa = R & 1;
+                for (int b = 0; b < B; ++b) {
+                    mine[(a * B + b) * 64] = acc[a][b][0];
+                    mine[(a * B + b) * 64 + 32] = acc[a][b][1];
+                }
+        }
+        __syncthreads();
+        if (ks0 < h) {
+#pragma unroll
+            for (int a = 0; a < A; ++a)
+#pragma unroll
+                for (int b = 0; b < B; ++b) {
+                    acc[a][b][0] += mine[(a * B + b) * 64];
+                    acc[a][b][1] += mine[(a * B + b) * 64 + 32];
+                }
+        }
+    }
+    if (ks0 != 0) return;
+#pragma unroll
+    for (int a = 0; a < A; ++a)
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            const int ti = wr + g.wr * a, tj = wc + g.wc * b;
+            const int row = ti * 8 + grp, l = row >> 1, pa = row & 1;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int Cg = n0 + tj * 8 + 2 * tig + h;
-                const int r = Cg >> 1, pc = Cg & 1;
-                if (l < g.nl && r < g.nr) {
+                const int col = tj * 8 + 2 * tig + h, r = col >> 1, pc = col & 1;
+                if (l < tile.nl && r < tile.nr && l + tile.diag >= r) {
                     const int qi = (pa == pc) ? pa : 2 + pa;  // ac, bd, ad, bc
-                    atomicAdd(g.out4 + ((long long)l * g.nr + r) * 4 + qi, acc[a][b][h]);
+                    atomicAdd(g.out4 + ((long long)(tile.l0 + l) * g.tiles.ldr + tile.r0 + r) * 4 + qi, acc[a][b][h]);
                 }
             }
         }

@@ -29,6 +29,7 @@
 #include <cstdint>
 
 #include "fft.cuh"
+#include "gram_blocks.hpp"
 
 namespace clk {
 namespace tc {
@@ -184,13 +185,13 @@ __global__ void __launch_bounds__(256) k_tf32_split(const cx<S>* __restrict__ sr
 }
 
 // ---------------------------------------------------------------------------------------
-// The Gram.  grid = (ceil(2 nl / BM), ceil(2 nr / BN), splits); block z covers k-tiles
-// [z * kt_per, min(kt_total, (z + 1) * kt_per)), never empty.  out4[l][r] += {ac, bd, ad, bc};
-// out4[4 * nl * nr] (as int) is set to 1 if any wait expired.
+// The Gram.  grid = (tiles, splits), tiles of at most 64 x 64 densities (gram_blocks.hpp); split y covers
+// k-tiles [y * kt_per, min(kt_total, (y + 1) * kt_per)), never empty.  out4[l][r] += {ac, bd, ad, bc};
+// *err (as int) is set to 1 if any wait expired.
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(THREADS, 1)
     k_gram_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int kt_total,
-              int kt_per, int nl, int nr, double* __restrict__ out4) {
+              int kt_per, const GramTiles tiles, double* __restrict__ out4, double* __restrict__ err) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -203,8 +204,10 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int FULL = 0, EMPTY = STAGES, ACCF = 2 * STAGES, ACCE = 2 * STAGES + 2, DRAIN = 2 * STAGES + 4;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    const int kt0 = blockIdx.z * kt_per;
+    GramTile tile;
+    gram_tile(tiles, blockIdx.x, &tile);
+    const int m0 = 2 * tile.l0, n0 = 2 * tile.r0;
+    const int kt0 = blockIdx.y * kt_per;
     const int kt1 = min(kt_total, kt0 + kt_per);
     const int nchunks = (kt1 - kt0 + CH - 1) / CH;
 
@@ -352,16 +355,17 @@ __global__ void __launch_bounds__(THREADS, 1)
             for (int i = 0; i < 32; ++i) acc[32 + i] += (double)v[i];
         }
         if (ok) {
-            const int R = m0 + 32 * q + lane;
+            const int R = 32 * q + lane;
             const int l = R >> 1, pa = R & 1;
-            if (l < nl) {
+            if (l < tile.nl) {
+                double* row = out4 + ((long long)(tile.l0 + l) * tiles.ldr + tile.r0) * 4;
 #pragma unroll
                 for (int j = 0; j < 64; ++j) {
-                    const int Cg = n0 + h * 64 + j;
+                    const int Cg = h * 64 + j;
                     const int r = Cg >> 1, pc = Cg & 1;
-                    if (r < nr) {
+                    if (r < tile.nr) {
                         const int qi = (pa == pc) ? pa : 2 + pa;  // ac, bd, ad, bc
-                        atomicAdd(out4 + ((long long)l * nr + r) * 4 + qi, acc[j]);
+                        atomicAdd(row + 4 * r + qi, acc[j]);
                     }
                 }
             }
@@ -371,7 +375,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     fence_before();
     __syncthreads();
     if (threadIdx.x == 0 && *abort_flag)
-        *reinterpret_cast<volatile int*>(out4 + (long long)4 * nl * nr) = 1;
+        *reinterpret_cast<volatile int*>(err) = 1;
     if (warp == 1) {
         __syncwarp();
         fence_after();
@@ -407,13 +411,14 @@ struct FusedGram {
     const float2* rho;    // right densities: rho[(ridx ? ridx[r] : r) * r_stride + atom]
     long long r_stride;
     const int* ridx;
-    int nl, nr;
     long long na;         // atoms
     int kt_total, kt_per;
     uint32_t stage_bytes;     // 2 * BM * 128 + 2 * nb_max * 128
     uint32_t raw_slot_bytes;  // (left + right densities of a block, at most) * 32 * 8
     double* out4;
+    double* err;
     int aligned16;            // every density row starts on a 16-byte boundary (16-byte copies)
+    GramTiles tiles;
 };
 
 constexpr int FUSED_WARPS = 16;
@@ -458,8 +463,7 @@ __device__ __forceinline__ void cp_async_wait() {
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// grid = (ceil(2 nl / BM), ceil(2 nr / BN), splits); block z covers k-tiles
-// [z * kt_per, min(kt_total, (z + 1) * kt_per)), never empty.  out4 as for k_gram_tc.
+// grid = (tiles, splits), k-tiles, out4 and err as for k_gram_tc.
 template <int AHEAD>
 __global__ void __launch_bounds__(FUSED_THREADS, 1) k_gram_tc_fused(const FusedGram g) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -478,13 +482,13 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_gram_tc_fused(const FusedG
     const uint32_t b_part = (g.stage_bytes - 2u * A_PART) / 2u;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    const int la0 = m0 / 2, rb0 = n0 / 2;
-    const int nA = min(BM / 2, g.nl - la0), nB = min(BN / 2, g.nr - rb0);
+    GramTile tile;
+    gram_tile(g.tiles, blockIdx.x, &tile);
+    const int la0 = tile.l0, rb0 = tile.r0, nA = tile.nl, nB = tile.nr;
     const int nd = nA + nB;
     const int nb = max(16, (2 * nB + 15) / 16 * 16);  // MMA N: the block's right rows, rounded up
     const uint32_t idesc = fused_idesc(nb);
-    const int kt0 = blockIdx.z * g.kt_per;
+    const int kt0 = blockIdx.y * g.kt_per;
     const int nt = min(g.kt_total, kt0 + g.kt_per) - kt0;
 
     if (threadIdx.x == 0) {
@@ -661,16 +665,17 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_gram_tc_fused(const FusedG
         mbar_drain(bar(DRAIN), 0);
     }
     if (ok) {
-        const int R = m0 + 32 * q + lane;
+        const int R = 32 * q + lane;
         const int l = R >> 1, pa = R & 1;
-        if (l < g.nl) {
+        if (l < nA) {
+            double* row = g.out4 + ((long long)(la0 + l) * g.tiles.ldr + rb0) * 4;
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
-                const int Cg = n0 + c0 + j;
+                const int Cg = c0 + j;
                 const int r = Cg >> 1, pc = Cg & 1;
-                if (r < g.nr) {
+                if (r < nB) {
                     const int qi = (pa == pc) ? pa : 2 + pa;  // ac, bd, ad, bc
-                    atomicAdd(g.out4 + ((long long)l * g.nr + r) * 4 + qi, acc[j]);
+                    atomicAdd(row + 4 * r + qi, acc[j]);
                 }
             }
         }
@@ -679,7 +684,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_gram_tc_fused(const FusedG
     fence_before();
     __syncthreads();
     if (threadIdx.x == 0 && *abort_flag)
-        *reinterpret_cast<volatile int*>(g.out4 + (long long)4 * g.nl * g.nr) = 1;
+        *reinterpret_cast<volatile int*>(g.err) = 1;
     if (warp == 0) {
         __syncwarp();
         fence_after();
@@ -775,13 +780,13 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_gram_tc_ws(const FusedGram g)
     constexpr int CONV_THREADS = 32 * WS_CONV_WARPS;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    const int la0 = m0 / 2, rb0 = n0 / 2;
-    const int nA = min(BM / 2, g.nl - la0), nB = min(BN / 2, g.nr - rb0);
+    GramTile tile;
+    gram_tile(g.tiles, blockIdx.x, &tile);
+    const int la0 = tile.l0, rb0 = tile.r0, nA = tile.nl, nB = tile.nr;
     const int nd = nA + nB;
     const int nb = max(16, (2 * nB + 15) / 16 * 16);
     const uint32_t idesc = fused_idesc(nb);
-    const int kt0 = blockIdx.z * g.kt_per;
+    const int kt0 = blockIdx.y * g.kt_per;
     const int nt = min(g.kt_total, kt0 + g.kt_per) - kt0;
 
     if (threadIdx.x == 0) {
@@ -1019,16 +1024,17 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_gram_tc_ws(const FusedGram g)
             // the correction accumulator is complete with the last k-tile's commit
             fence_after();
             add_cols((uint32_t)(WS_NACC * BN));
-            const int R = m0 + 32 * q + lane;
+            const int R = 32 * q + lane;
             const int l = R >> 1, pa = R & 1;
-            if (l < g.nl) {
+            if (l < nA) {
+                double* row = g.out4 + ((long long)(la0 + l) * g.tiles.ldr + rb0) * 4;
 #pragma unroll
                 for (int j = 0; j < WS_MAX_DC; ++j) {
-                    const int Cg = n0 + col0 + j;
+                    const int Cg = col0 + j;
                     const int r = Cg >> 1, pc = Cg & 1;
-                    if (j < dc && r < g.nr) {
+                    if (j < dc && r < nB) {
                         const int qi = (pa == pc) ? pa : 2 + pa;  // ac, bd, ad, bc
-                        atomicAdd(g.out4 + ((long long)l * g.nr + r) * 4 + qi, acc[j]);
+                        atomicAdd(row + 4 * r + qi, acc[j]);
                     }
                 }
             }
@@ -1038,7 +1044,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_gram_tc_ws(const FusedGram g)
     fence_before();
     __syncthreads();
     if (threadIdx.x == 0 && *abort_flag)
-        *reinterpret_cast<volatile int*>(g.out4 + (long long)4 * g.nl * g.nr) = 1;
+        *reinterpret_cast<volatile int*>(g.err) = 1;
     if (warp == 0) {
         __syncwarp();
         fence_after();

@@ -711,81 +711,6 @@ __global__ void __launch_bounds__(256, 8) k_round_sum(const cx<T>* __restrict__ 
     }
 }
 
-// ---------------------------------------------------------------------------------------
-// Real-space reductions in FP64 (CoulombCalculator.cpp:165-172 restricted to the atom
-// cells, where the right density is non-zero): for left l and right r with V = a+ib and
-// rho = c+id, out[l][r] += {sum ac, sum bd, sum ad, sum bc}; then
-//   sum V rho       = (ac - bd) + i (ad + bc)
-//   sum V conj(rho) = (ac + bd) + i (bc - ad).
-// 64x64 (l, r) tiles, 4x4 per thread, atoms staged 16 at a time; split over atoms with one
-// FP64 atomicAdd per result per block.
-// ---------------------------------------------------------------------------------------
-template <int IB, typename RT>
-__global__ void __launch_bounds__(256) k_gram(const cx<double>* __restrict__ V, long long v_stride, int nl,
-                                             const cx<RT>* __restrict__ rho, long long r_stride,
-                                             const int* __restrict__ ridx, int nr, long long n_atoms,
-                                             long long atoms_per_split, double* __restrict__ out) {
-    // (16*IB) x (16*IB) tile of (left, right) pairs, IB x IB per thread; IB is chosen on the host
-    // so the tiles waste little of a small density count.
-    constexpr int TS = 16 * IB;
-    __shared__ cx<double> vs[16][TS];
-    __shared__ cx<double> rs[16][TS];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int l0 = blockIdx.x * TS, r0 = blockIdx.y * TS;
-    const long long k_begin = (long long)blockIdx.z * atoms_per_split;
-    const long long k_end = min(n_atoms, k_begin + atoms_per_split);
-    double acc[IB][IB][4];
-#pragma unroll
-    for (int i = 0; i < IB; ++i)
-#pragma unroll
-        for (int j = 0; j < IB; ++j)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0;
-    for (long long k0 = k_begin; k0 < k_end; k0 += 16) {
-        for (int e = threadIdx.x; e < 16 * TS; e += 256) {
-            const int row = e >> 4, k = e & 15;
-            const long long atom = k0 + k;
-            const bool ok = atom < k_end;
-            const int l = l0 + row, r = r0 + row;
-            vs[k][row] = (ok && l < nl) ? V[(long long)l * v_stride + atom] : mk(0.0, 0.0);
-            rs[k][row] = (ok && r < nr) ? widen(rho[(long long)ridx[r] * r_stride + atom]) : mk(0.0, 0.0);
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int k = 0; k < 16; ++k) {
-            cx<double> v[IB], r[IB];
-#pragma unroll
-            for (int i = 0; i < IB; ++i) v[i] = vs[k][ty + 16 * i];
-#pragma unroll
-            for (int j = 0; j < IB; ++j) r[j] = rs[k][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < IB; ++i)
-#pragma unroll
-                for (int j = 0; j < IB; ++j) {
-                    acc[i][j][0] += v[i].re * r[j].re;
-                    acc[i][j][1] += v[i].im * r[j].im;
-                    acc[i][j][2] += v[i].re * r[j].im;
-                    acc[i][j][3] += v[i].im * r[j].re;
-                }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < IB; ++i)
-#pragma unroll
-        for (int j = 0; j < IB; ++j) {
-            const int l = l0 + ty + 16 * i, r = r0 + tx + 16 * j;
-            if (l < nl && r < nr) {
-                double* o = out + ((long long)l * nr + r) * 4;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) atomicAdd(o + q, acc[i][j][q]);
-            }
-        }
-}
-
-// Grid-API scatter of a dense density into the "every cell is an atom" list is the identity;
-// its dot product reuses k_gram with nl = nr = 1.
-
 // Widening / narrowing copies for the standalone FFT entry point.
 template <typename T>
 __global__ void k_narrow(const cx<double>* __restrict__ in, cx<T>* __restrict__ out, long long n) {
