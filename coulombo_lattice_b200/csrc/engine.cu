@@ -278,8 +278,8 @@ struct cl_ctx {
 
     bool kernel_ready = false;
     DevBuf<double> ghat;
-    DevBuf<double> khat64[8];
-    DevBuf<float> khat32[8];
+    DevBuf<double> khat64;  // the 8 rounds' Khat_kappa, one after another
+    DevBuf<float> khat32;
 
     // grid API ("every cell is an atom")
     DevBuf<int> grid_cell, grid_row_ptr;
@@ -413,13 +413,13 @@ void build_khat(cl_ctx* c) {
     for (int r = 0; r < 8; ++r) {
         const int kx = r & 1, ky = (r >> 1) & 1, kz = (r >> 2) & 1;
         if (fp64_form(c)) {
-            c->khat64[r].alloc(c->M);
+            c->khat64.alloc(8 * c->M);
             clk::k_khat<double><<<grid_for(c->M), 256, 0, c->stream>>>(c->ghat.p, nx, ny, nz, kx, ky, kz, denom,
-                                                                       c->khat64[r].p);
+                                                                       c->khat64.p + r * c->M);
         } else {
-            c->khat32[r].alloc(c->M);
+            c->khat32.alloc(8 * c->M);
             clk::k_khat<float><<<grid_for(c->M), 256, 0, c->stream>>>(c->ghat.p, nx, ny, nz, kx, ky, kz, denom,
-                                                                      c->khat32[r].p);
+                                                                      c->khat32.p + r * c->M);
         }
         CL_LAUNCHED();
     }
@@ -685,11 +685,20 @@ void run_rounds(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, const
     size_t by_mem = std::max<size_t>(1, budget / (grid_bytes + round_bytes));
     size_t by_l2 = l2_budget / grid_bytes;
     int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)np, by_l2 >= 2 ? by_l2 : by_mem));
-    c->work.alloc(std::max(c->work.n, (size_t)chunk * grid_bytes));
+    // All rounds in one launch of each pass where their grids take at most 512 MB: 8 rounds of launches
+    // become one, and a small grid's rounds fill the SMs together (B200, a request's kernels: 32^3 in FP64,
+    // 10 densities, 0.388 -> 0.120 ms; 45^3 in FP32, 10 densities, 0.471 -> 0.183; 64^3 in FP64, one
+    // density, 0.360 -> 0.127).  Larger grids fill the SMs round by round and keep one
+    // round's buffers.
+    const size_t all_rounds = (size_t)np * n_rounds * grid_bytes;
+    const bool together = chunk == np && all_rounds <= std::min<size_t>(512ull << 20, budget / 2) &&
+                          l2_budget == 0 && np * n_rounds <= 65535;  // grids of a launch (gridDim.y)
+    const int per_launch = together ? n_rounds : 1;
+    c->work.alloc(std::max(c->work.n, together ? all_rounds : (size_t)chunk * grid_bytes));
     c->rounds.alloc(std::max(c->rounds.n, (size_t)chunk * round_bytes));
     cx<T>* buf = reinterpret_cast<cx<T>*>(c->work.p);
     cx<T>* tr = reinterpret_cast<cx<T>*>(c->rounds.p);
-    const long long tr_slot = (long long)chunk * n_at;  // elements per round slot
+    const T* kh = sizeof(T) == 4 ? (const T*)c->khat32.p : (const T*)c->khat64.p;
 
     const Axis& X = c->ax[0];
     const Axis& Y = c->ax[1];
@@ -723,8 +732,7 @@ void run_rounds(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, const
     // the request's own passes overwrite afterwards.
     if (autotune_enabled() && !std::getenv("CL_TUNE_FORCE") && np > 0 && !stream_capturing(c->stream)) {
         const int cnt_t = (int)std::max<size_t>(1, std::min<size_t>((size_t)chunk, (512ull << 20) / grid_bytes));
-        const clk::RoundPhase rp0{c->ax[0].phase.p, c->ax[1].phase.p, c->ax[2].phase.p, 0, 0, 0};
-        const T* kh0 = sizeof(T) == 4 ? (const T*)c->khat32[0].p : (const T*)c->khat64[0].p;
+        const clk::RoundPhase rp0{c->ax[0].phase.p, c->ax[1].phase.p, c->ax[2].phase.p, 0, 0, 0, 0, 1, 0};
         const int* rp_skip = skip_empty ? row_ptr : nullptr;
         if (reg_x)
             tune_pass(c, clp::kXFwd, fp32, nx, [&](clp::Variant v) {
@@ -741,7 +749,7 @@ void run_rounds(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, const
         }
         if (reg_z)
             tune_pass(c, clp::kZConv, fp32, nz, [&](clp::Variant v) {
-                clp::zconv<T>(c->stream, v, buf, c->M, twz, kh0, nxy, nz, cnt_t);
+                clp::zconv<T>(c->stream, v, buf, c->M, twz, kh, nxy, nz, cnt_t, clp::Rounds{});
             });
         if (reg_x)
             tune_pass(c, clp::kXInv, fp32, nx, [&](clp::Variant v) {
@@ -772,63 +780,69 @@ void run_rounds(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, const
         const int cnt = std::min(chunk, np - p0);
         const cx<T>* rho_c = rho + (long long)p0 * rho_stride;
         cx<double>* V_c = V + (long long)p0 * v_stride;
-        int slot = 0;
+        const long long tr_slot = (long long)cnt * n_at;  // elements per round
+        int done = 0;                                      // rounds of the mask launched so far
         for (int r = 0; r < 8; ++r) {
             if (!((round_mask >> r) & 1)) continue;
-            cx<T>* tr_r = tr + slot++ * tr_slot;
-            clk::RoundPhase rp{c->ax[0].phase.p, c->ax[1].phase.p, c->ax[2].phase.p, r & 1, (r >> 1) & 1,
-                               (r >> 2) & 1};
-            const T* kh = sizeof(T) == 4 ? (const T*)c->khat32[r].p : (const T*)c->khat64[r].p;
+            clp::Rounds rounds{0, 0, (long long)cnt * c->M};
+            for (; r < 8 && rounds.n < per_launch; ++r)
+                if ((round_mask >> r) & 1) rounds.list |= (unsigned)r << (4 * rounds.n++);
+            --r;
+            const int grids = cnt * rounds.n;  // one after another, a round's densities together
+            cx<T>* tr_r = tr + done * tr_slot;
+            done += rounds.n;
+            const clk::RoundPhase rp{c->ax[0].phase.p, c->ax[1].phase.p, c->ax[2].phase.p, 0, 0, 0,
+                                     rounds.list,      rounds.n,          rounds.stride};
             cudaEvent_t e = prof_begin(c);
             if (xy_fwd) {
                 clp::xyfwd<T>(c->stream, rho_c, rho_stride, row_ptr, cell, buf, c->M, twx, rp, nx, ny, nz, cnt);
             } else if (!(reg_x && clp::xfwd<T>(c->stream, v_xf, rho_c, rho_stride, row_ptr, cell, buf, c->M, twx,
                                                 rp, nx, ny, nrows, cnt, skip_empty))) {
-                clk::k_xfwd<T><<<xblocks, 256, xt.smem, c->stream>>>(rho_c, rho_stride, row_ptr, cell, buf, c->M,
-                                                                     X.plan, twx, rp, nx, ny, nrows, xt.rows, xt.ld,
-                                                                     cnt);
+                clk::k_xfwd<T><<<dim3(xblocks, 1, rounds.n), 256, xt.smem, c->stream>>>(
+                    rho_c, rho_stride, row_ptr, cell, buf, c->M, X.plan, twx, rp, nx, ny, nrows, xt.rows, xt.ld, cnt);
             }
             CL_LAUNCHED();
             prof_end(c, e, CL_KCLASS_XFWD,
-                     cnt * (atoms * (double)sizeof(cx<T>) + (xy_fwd ? 1.0 : live) * gbytes) + atoms * 4.0);
+                     grids * (atoms * (double)sizeof(cx<T>) + (xy_fwd ? 1.0 : live) * gbytes) + atoms * 4.0);
             if (!xy_fwd) {
                 e = prof_begin(c);
-                if (!(reg_y &&
-                      clp::ycol<-1, T>(c->stream, v_yf, buf, c->M, twy, nx, ny, nz, cnt, skip_empty ? row_ptr : nullptr)))
-                    clk::k_ypass<-1, T><<<dim3(ychunks * nz, cnt), 256, yt.smem, c->stream>>>(buf, c->M, Y.plan, twy,
-                                                                                              nx, ny, yt.W, ychunks);
+                if (!(reg_y && clp::ycol<-1, T>(c->stream, v_yf, buf, c->M, twy, nx, ny, nz, grids,
+                                                 skip_empty ? row_ptr : nullptr)))
+                    clk::k_ypass<-1, T><<<dim3(ychunks * nz, grids), 256, yt.smem, c->stream>>>(
+                        buf, c->M, Y.plan, twy, nx, ny, yt.W, ychunks);
                 CL_LAUNCHED();
-                prof_end(c, e, CL_KCLASS_YPASS, cnt * (1.0 + live) * gbytes);
+                prof_end(c, e, CL_KCLASS_YPASS, grids * (1.0 + live) * gbytes);
             }
             e = prof_begin(c);
-            if (!(reg_z && clp::zconv<T>(c->stream, v_z, buf, c->M, twz, kh, nxy, nz, cnt)))
-                clk::k_zpass<T><<<dim3((unsigned)zblocks, zgroups(zblocks, cnt)), 256, zt.smem, c->stream>>>(
-                    buf, c->M, Z.plan, twz, kh, nxy, nz, zt.W, cnt, 0);
+            if (!(reg_z && clp::zconv<T>(c->stream, v_z, buf, c->M, twz, kh, nxy, nz, cnt, rounds)))
+                clk::k_zpass<T><<<dim3((unsigned)zblocks, zgroups(zblocks * rounds.n, cnt), rounds.n), 256, zt.smem,
+                                  c->stream>>>(buf, c->M, Z.plan, twz, kh, nxy, nz, zt.W, cnt, 0, rounds.list,
+                                               rounds.stride);
             CL_LAUNCHED();
-            prof_end(c, e, CL_KCLASS_ZPASS, cnt * 2.0 * gbytes + (double)c->M * sizeof(T));
+            prof_end(c, e, CL_KCLASS_ZPASS, grids * 2.0 * gbytes + rounds.n * (double)c->M * sizeof(T));
             if (!xy_inv) {
                 e = prof_begin(c);
-                if (!(reg_y &&
-                      clp::ycol<+1, T>(c->stream, v_yi, buf, c->M, twy, nx, ny, nz, cnt, skip_empty ? row_ptr : nullptr)))
-                    clk::k_ypass<+1, T><<<dim3(ychunks * nz, cnt), 256, yt.smem, c->stream>>>(buf, c->M, Y.plan, twy,
-                                                                                              nx, ny, yt.W, ychunks);
+                if (!(reg_y && clp::ycol<+1, T>(c->stream, v_yi, buf, c->M, twy, nx, ny, nz, grids,
+                                                 skip_empty ? row_ptr : nullptr)))
+                    clk::k_ypass<+1, T><<<dim3(ychunks * nz, grids), 256, yt.smem, c->stream>>>(
+                        buf, c->M, Y.plan, twy, nx, ny, yt.W, ychunks);
                 CL_LAUNCHED();
-                prof_end(c, e, CL_KCLASS_YPASS, cnt * (1.0 + live) * gbytes);
+                prof_end(c, e, CL_KCLASS_YPASS, grids * (1.0 + live) * gbytes);
             }
             e = prof_begin(c);
             if (xy_inv) {
-                clp::xyinv<T>(c->stream, buf, c->M, twx, row_ptr, cell, tr_r, n_at, nx, ny, nz, cnt);
+                clp::xyinv<T>(c->stream, buf, c->M, twx, row_ptr, cell, tr_r, n_at, nx, ny, nz, grids);
             } else if (!(reg_x && clp::xinv<T>(c->stream, v_xi, buf, c->M, twx, row_ptr, cell, tr_r, n_at, nx, nrows,
-                                                cnt))) {
+                                                grids))) {
                 clk::k_xinv<T><<<xblocks, 256, xt.smem, c->stream>>>(buf, c->M, X.plan, twx, row_ptr, cell, tr_r,
-                                                                     n_at, nx, nrows, xt.rows, xt.ld, cnt);
+                                                                     n_at, nx, nrows, xt.rows, xt.ld, grids);
             }
             CL_LAUNCHED();
             prof_end(c, e, CL_KCLASS_XINV,
-                     cnt * ((xy_inv ? 1.0 : row_side) * gbytes + atoms * (double)sizeof(cx<T>)) + atoms * 4.0);
+                     grids * ((xy_inv ? 1.0 : row_side) * gbytes + atoms * (double)sizeof(cx<T>)) + atoms * 4.0);
         }
         if (n_rounds > 0) {
-            const clk::RoundPhase base{c->ax[0].phase.p, c->ax[1].phase.p, c->ax[2].phase.p, 0, 0, 0};
+            const clk::RoundPhase base{c->ax[0].phase.p, c->ax[1].phase.p, c->ax[2].phase.p, 0, 0, 0, 0, 1, 0};
             const long long blocks = std::min<long long>((n_at + 255) / 256, 148LL * 16);
             cudaEvent_t e = prof_begin(c);
             clk::k_round_sum<T><<<dim3((unsigned)blocks, zgroups(blocks, cnt)), 256, 0, c->stream>>>(
@@ -1045,7 +1059,7 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
     // CL_NO_QPLANE=1 keeps the general one
     const bool qplane = clp::quadrant_supported(fp32, nx, ny) && !std::getenv("CL_NO_QPLANE");
     // no phase in any pass: the rounds' phase tables are never read with kappa = 0
-    const clk::RoundPhase rp0{c->ax[0].phase.p, c->ax[1].phase.p, c->ax[2].phase.p, 0, 0, 0};
+    const clk::RoundPhase rp0{c->ax[0].phase.p, c->ax[1].phase.p, c->ax[2].phase.p, 0, 0, 0, 0, 1, 0};
     cx<T>* out0 = via_tr ? tr : static_cast<cx<T>*>(V_any);
     const long long out_stride = via_tr ? n_at : v_stride;
     if (autotune_enabled() && !std::getenv("CL_TUNE_FORCE") && np > 0 && !stream_capturing(c->stream)) {
@@ -3037,7 +3051,7 @@ int cl_fft3d(int nx, int ny, int nz, int batch, int sign, int fp32, double* data
             }
             ensure_smem(clk::k_zpass<T>, zt.smem);
             clk::k_zpass<T><<<(unsigned)zblocks, 256, zt.smem, c->stream>>>(buf, M, Z.plan, twz, nullptr, nxy, nz,
-                                                                             zt.W, batch, sign);
+                                                                             zt.W, batch, sign, 0u, 0LL);
             CL_LAUNCHED();
             if constexpr (sizeof(T) == 4) {
                 clk::k_widen<float><<<grid_for((long long)n), 256, 0, c->stream>>>(dT.p, d64.p, (long long)n);

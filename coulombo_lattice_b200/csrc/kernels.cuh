@@ -28,7 +28,23 @@ struct RoundPhase {
     const cx<double>* py;
     const cx<double>* pz;
     int kx, ky, kz;
+    // Rounds of a launch, one per blockIdx.z: round z is (rounds >> 4 z) & 7 and its grids start z * stride
+    // elements on.  Small boxes run all their rounds in one launch: one round of a 32^3 grid and 10
+    // densities occupies a pass for about 5 us, most of it the launch.
+    unsigned rounds;
+    int n_rounds;
+    long long stride;
 };
+
+__device__ __forceinline__ int block_round(unsigned rounds) { return (int)((rounds >> (4 * blockIdx.z)) & 7u); }
+// The launch's phases with this block's round.
+__device__ __forceinline__ RoundPhase block_phase(RoundPhase rp) {
+    const int r = block_round(rp.rounds);
+    rp.kx = r & 1;
+    rp.ky = (r >> 1) & 1;
+    rp.kz = (r >> 2) & 1;
+    return rp;
+}
 
 __device__ __forceinline__ cx<double> round_phase(const RoundPhase& rp, int x, int y, int z) {
     cx<double> p = mk(1.0, 0.0);
@@ -494,6 +510,8 @@ __global__ void __launch_bounds__(256) k_xfwd(const cx<T>* __restrict__ rho, lon
     cx<T>* tw = reinterpret_cast<cx<T>*>(smem_raw);
     cx<T>* a = tw + nx;
     cx<T>* b = a + (size_t)nx * ld;
+    rp = block_phase(rp);
+    out += blockIdx.z * rp.stride;
     const int r0 = blockIdx.x * rows;
     const int nr = min(rows, nrows - r0);
     for (int i = threadIdx.x; i < nx; i += blockDim.x) tw[i] = tw_g[i];
@@ -574,14 +592,18 @@ __global__ void __launch_bounds__(256) k_ypass(cx<T>* __restrict__ buf, long lon
 
 // ---------------------------------------------------------------------------------------
 // Pass along z: forward FFT, x Khat_kappa (tile loaded once per block and reused for all
-// densities), inverse FFT.  With khat == nullptr only the forward (S<0) or backward
+// densities), inverse FFT; blockIdx.z: round (see RoundPhase; khat holds the 8 rounds' one after another).
+// With khat == nullptr only the forward (S<0) or backward
 // transform is done (standalone FFT).  Block = W consecutive xy positions, all z.
 // ---------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256) k_zpass(cx<T>* __restrict__ buf, long long stride, FftPlan plan,
                                               const cx<T>* __restrict__ tw_g, const T* __restrict__ khat,
-                                              long long nxy, int nz, int W, int np, int sign) {
+                                              long long nxy, int nz, int W, int np, int sign, unsigned rounds,
+                                              long long round_stride) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    buf += blockIdx.z * round_stride;
+    if (khat) khat += block_round(rounds) * nxy * nz;
     cx<T>* tw = reinterpret_cast<cx<T>*>(smem_raw);
     cx<T>* a = tw + nz;
     cx<T>* b = a + (size_t)nz * W;

@@ -122,7 +122,7 @@ void run(int nx, int ny, int nz, int batch, clk::cx<double>* data, const clk::cx
         clk::k_ypass<S, double><<<dim3(ychunks * nz, nb), 256, ys>>>(slice, M, py, twy, nx, ny, wy, ychunks);
         NA_CUDA(cudaGetLastError());
     }
-    clk::k_zpass<double><<<(unsigned)((nxy + wz - 1) / wz), 256, zs>>>(data, M, pz, twz, nullptr, nxy, nz, wz, batch, S);
+    clk::k_zpass<double><<<(unsigned)((nxy + wz - 1) / wz), 256, zs>>>(data, M, pz, twz, nullptr, nxy, nz, wz, batch, S, 0u, 0LL);
     NA_CUDA(cudaGetLastError());
 }
 

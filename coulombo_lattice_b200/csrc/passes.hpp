@@ -46,18 +46,25 @@ int split_variants(int n);
 // while each block still reuses its per-block setup for a run of densities.
 unsigned density_groups(long long blocks, int cnt);
 
-// z pass: forward FFT along z, x Khat, inverse FFT along z (in place).
+// Rounds of a launch (see clk::RoundPhase): their list, count and the distance of their grids.
+struct Rounds {
+    unsigned list = 0;
+    int n = 1;
+    long long stride = 0;
+};
+
+// z pass: forward FFT along z, x Khat, inverse FFT along z (in place); kh: the 8 rounds' Khat.
 template <typename T>
 bool zconv(cudaStream_t s, Variant v, cx<T>* buf, long long M, const cx<T>* tw, const T* kh, long long nxy, int nz,
-           int cnt);
+           int cnt, const Rounds& rounds);
 
 // y pass of direction S (in place); row_ptr (or nullptr) marks the rows without atoms.
 template <int S, typename T>
 bool ycol(cudaStream_t s, Variant v, cx<T>* buf, long long M, const cx<T>* tw, int nx, int ny, int nz, int cnt,
           const int* row_ptr);
 
-// forward x pass: scatter of the atoms x conj(phase), FFT along x, rows stored; the pair
-// densities rho are in the pass precision.
+// forward x pass: scatter of the atoms x conj(phase), FFT along x, rows stored, for every round of rp;
+// the pair densities rho are in the pass precision.
 template <typename T>
 bool xfwd(cudaStream_t s, Variant v, const cx<T>* rho, long long rho_stride, const int* row_ptr,
           const int* cell, cx<T>* buf, long long M, const cx<T>* tw, const clk::RoundPhase& rp, int nx, int ny,

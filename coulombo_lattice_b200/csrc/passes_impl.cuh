@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "passes.hpp"
@@ -39,7 +40,7 @@ void with_lines(const Variant& v, F&& f) {
 
 template <typename T>
 bool zconv(cudaStream_t s, Variant v, cx<T>* buf, long long M, const cx<T>* tw, const T* kh, long long nxy, int nz,
-           int cnt) {
+           int cnt, const Rounds& rounds) {
     return clk::with_split2(
         nz,
         [&](auto tag) {
@@ -51,8 +52,8 @@ bool zconv(cudaStream_t s, Variant v, cx<T>* buf, long long M, const cx<T>* tw, 
                 const size_t smem = clk::ZconvLayout<T, Tag::r1, Tag::r2, L>::smem;
                 set_smem(kern, smem);
                 const long long blocks = (nxy + L - 1) / L;
-                kern<<<dim3((unsigned)blocks, density_groups(blocks, cnt)), L * P, smem, s>>>(buf, M, tw, kh, nxy,
-                                                                                              cnt);
+                kern<<<dim3((unsigned)blocks, density_groups(blocks * rounds.n, cnt), rounds.n), L * P, smem, s>>>(
+                    buf, M, tw, kh, nxy, cnt, rounds.list, rounds.stride);
             });
         },
         v.split);
@@ -98,7 +99,8 @@ bool xfwd(cudaStream_t s, Variant v, const cx<T>* rho, long long rho_stride, con
                         sizeof(cx<T>) * clk::XfwdPitch<Tag::r1, Tag::r2, LR, PAD, sizeof(cx<T>)>::elems;
                     set_smem(kern, smem);
                     const long long blocks = (nrows + LR - 1) / LR;
-                    kern<<<dim3((unsigned)blocks, density_groups(blocks, cnt)), LR * Q, smem, s>>>(
+                    const int nr = std::max(1, rp.n_rounds);
+                    kern<<<dim3((unsigned)blocks, density_groups(blocks * nr, cnt), nr), LR * Q, smem, s>>>(
                         rho, rho_stride, row_ptr, cell, buf, M, tw, rp, ny, nrows, cnt, skip_empty);
                 };
                 if constexpr (sizeof(T) == 4) {

@@ -45,8 +45,9 @@ bool xyfwd(cudaStream_t s, const cx<T>* rho, long long rho_stride, const int* ro
         auto kern = clk::k_xyfwd_plane<T, Tag::r1, Tag::r2, TH, MB>;
         const size_t smem = clk::PlaneSmem<T, Tag::r1, Tag::r2, TH, true, MB>::bytes;
         set_smem(kern, smem);
-        kern<<<dim3((unsigned)nz, plane_groups(nz, cnt, MB)), TH, smem, s>>>(rho, rho_stride, row_ptr, cell, buf, M,
-                                                                             tw, rp, cnt);
+        const int nr = std::max(1, rp.n_rounds);
+        kern<<<dim3((unsigned)nz, plane_groups(nz * nr, cnt, MB), nr), TH, smem, s>>>(rho, rho_stride, row_ptr, cell,
+                                                                                     buf, M, tw, rp, cnt);
     });
 }
 

@@ -18,8 +18,8 @@ unsigned density_groups(long long blocks, int cnt) {
 }
 
 template bool zconv<float>(cudaStream_t, Variant, cx<float>*, long long, const cx<float>*, const float*, long long,
-                           int, int);
+                           int, int, const Rounds&);
 template bool zconv<double>(cudaStream_t, Variant, cx<double>*, long long, const cx<double>*, const double*,
-                            long long, int, int);
+                            long long, int, int, const Rounds&);
 
 }  // namespace clp

@@ -276,6 +276,8 @@ __global__ void __launch_bounds__(THREADS, MINB)
     k_xyfwd_plane(const cx<T>* __restrict__ rho, long long rho_stride, const int* __restrict__ row_ptr,
                   const int* __restrict__ cell, cx<T>* __restrict__ out, long long out_stride,
                   const cx<T>* __restrict__ tw_g, RoundPhase rp, int np) {
+    rp = block_phase(rp);
+    out += blockIdx.z * rp.stride;
     using L = PlaneLayout<T, R1, R2>;
     using Sm = PlaneSmem<T, R1, R2, THREADS, true, MINB>;
     static_assert(R1 <= 8 && R2 <= 16 && L::N <= 128, "plane stages serve 16 lanes a row (phase A) and 8 (phase B)");

@@ -117,7 +117,7 @@ struct YcolLayout {
 template <typename T, int R1, int R2, int L>
 __global__ void __launch_bounds__(L * ColShape<R1, R2>::P, colp_min_blocks<T, R1, R2, L * ColShape<R1, R2>::P>::value)
     k_zconv_rf(cx<T>* __restrict__ buf, long long stride, const cx<T>* __restrict__ tw_g,
-               const T* __restrict__ khat, long long nxy, int np) {
+               const T* __restrict__ khat, long long nxy, int np, unsigned rounds, long long round_stride) {
     using S = ColShape<R1, R2>;
     using Lay = ZconvLayout<T, R1, R2, L>;
     constexpr int N = R1 * R2, P = S::P, IA = S::IA, IB = S::IB, LP0 = Lay::LP0, LP1 = Lay::LP1;
@@ -129,6 +129,8 @@ __global__ void __launch_bounds__(L * ColShape<R1, R2>::P, colp_min_blocks<T, R1
     const int qt = threadIdx.x / L;
     const long long c = (long long)blockIdx.x * L + line;
     const bool valid = c < nxy;
+    buf += blockIdx.z * round_stride;  // blockIdx.z: round (see RoundPhase)
+    khat += block_round(rounds) * nxy * N;
     for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = tw_g[i];
     // Khat of the positions q + r*R1 that phase-B item q holds, for all densities
     T kv[IB][R2];
@@ -438,6 +440,8 @@ __global__ void __launch_bounds__(LR * cmax<R1, R2>::value, col_min_blocks<R1, R
     cx<T>* tw = reinterpret_cast<cx<T>*>(smem_raw);
     cx<T>* tile = tw + N;
     cx<T>* ex = tile + Tile::points * TP;
+    rp = block_phase(rp);
+    out += blockIdx.z * rp.stride;
     const int r0 = blockIdx.x * LR;
     const int nr = min(LR, nrows - r0);
     // twiddles laid out [r][j] = W_N^(r j), so that phase B's lanes on consecutive j read
