@@ -1055,14 +1055,16 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
     const bool reg_y = register_passes_enabled() && clp::split_variants(ny) > 0;
     const int skip_empty = (reg_x && reg_y && !std::getenv("CL_NO_ROW_SKIP")) ? 1 : 0;
     const bool plane_ok = reg_x && reg_y && clp::plane_supported(fp32, nx, ny);
-    // 128 x 128 FP32 class planes: the quadrant forward plane pass (two blocks an SM);
-    // CL_NO_QPLANE=1 keeps the general one
-    const bool qplane = clp::quadrant_supported(fp32, nx, ny) && !std::getenv("CL_NO_QPLANE");
+    // FP32 square class planes: the quadrant plane passes, at every length compiled the fastest measured
+    // (36 densities of 128 x 128 planes: 0.57 ms forward and 0.74 inverse, the general plane passes 0.94
+    // and 0.89; 820 of 64 x 64: 1.37 and 1.58, 1.94 and 1.89; 78 of 48 x 48: 0.082 and 0.081, the
+    // separate passes 0.159 and 0.165); CL_NO_QPLANE=1 keeps the general ones
+    const bool qplane = fp32 && clp::quadrant_supported(nx, ny) && !std::getenv("CL_NO_QPLANE");
     // no phase in any pass: the rounds' phase tables are never read with kappa = 0
     const clk::RoundPhase rp0{c->ax[0].phase.p, c->ax[1].phase.p, c->ax[2].phase.p, 0, 0, 0, 0, 1, 0};
     cx<T>* out0 = via_tr ? tr : static_cast<cx<T>*>(V_any);
     const long long out_stride = via_tr ? n_at : v_stride;
-    if (autotune_enabled() && !std::getenv("CL_TUNE_FORCE") && np > 0 && !stream_capturing(c->stream)) {
+    if (autotune_enabled() && !std::getenv("CL_TUNE_FORCE") && np > 0 && !qplane && !stream_capturing(c->stream)) {
         const int cnt_t = (int)std::max<size_t>(1, std::min<size_t>((size_t)chunk, (512ull << 20) / grid_bytes));
         const int* rp_skip = skip_empty ? row_ptr : nullptr;
         if (reg_x)
@@ -1107,8 +1109,8 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
         cx<T>* out_c = via_tr ? tr : static_cast<cx<T>*>(V_any) + (long long)p0 * v_stride;
         cudaEvent_t e = prof_begin(c);
         if (qplane) {
-            clp::qfwd(c->stream, reinterpret_cast<const cx<float>*>(rho_c), rho_stride, row_ptr, cell,
-                      reinterpret_cast<cx<float>*>(buf), vM, reinterpret_cast<const cx<float>*>(twx), nz, cnt);
+            clp::pfwd(c->stream, reinterpret_cast<const cx<float>*>(rho_c), rho_stride, row_ptr, cell,
+                      reinterpret_cast<cx<float>*>(buf), vM, reinterpret_cast<const cx<float>*>(twx), nx, nz, cnt);
         } else if (xy_fwd) {
             clp::xyfwd<T>(c->stream, rho_c, rho_stride, row_ptr, cell, buf, vM, twx, rp0, nx, ny, nz, cnt);
         } else if (!(reg_x && clp::xfwd<T>(c->stream, v_xf, rho_c, rho_stride, row_ptr, cell, buf, vM, twx, rp0, nx,
@@ -1143,7 +1145,7 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
             cl::fail(CL_ERR_UNSUPPORTED, "no sub-lattice z pass for %d points", sl.pad[2]);
         CL_LAUNCHED();
         prof_end(c, e, CL_KCLASS_ZPASS, cnt * 2.0 * gbytes + h_bytes);
-        if (!xy_inv) {
+        if (!xy_inv && !qplane) {
             e = prof_begin(c);
             if (!(reg_y && clp::ycol<+1, T>(c->stream, v_yi, buf, vM, twy, nx, ny, nz, cnt,
                                              skip_empty ? row_ptr : nullptr)))
@@ -1153,7 +1155,10 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
             prof_end(c, e, CL_KCLASS_YPASS, cnt * (1.0 + live) * gbytes);
         }
         e = prof_begin(c);
-        if (xy_inv) {
+        if (qplane) {
+            clp::pinv(c->stream, reinterpret_cast<const cx<float>*>(buf), vM, reinterpret_cast<const cx<float>*>(twx),
+                      row_ptr, cell, reinterpret_cast<cx<float>*>(out_c), out_stride, nx, nz, cnt);
+        } else if (xy_inv) {
             clp::xyinv<T>(c->stream, buf, vM, twx, row_ptr, cell, out_c, out_stride, nx, ny, nz, cnt);
         } else if (!(reg_x && clp::xinv<T>(c->stream, v_xi, buf, vM, twx, row_ptr, cell, out_c, out_stride, nx, nrows,
                                             cnt))) {
@@ -1162,7 +1167,7 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
         }
         CL_LAUNCHED();
         prof_end(c, e, CL_KCLASS_XINV,
-                 cnt * ((xy_inv ? 1.0 : row_side) * gbytes + atoms * (double)sizeof(cx<T>)) + atoms * 4.0);
+                 cnt * ((xy_inv || qplane ? 1.0 : row_side) * gbytes + atoms * (double)sizeof(cx<T>)) + atoms * 4.0);
         if (via_tr) {
             e = prof_begin(c);
             clk::k_sl_widen<T><<<dim3((unsigned)std::min<long long>((n_at + 255) / 256, 148LL * 8), cnt), 256, 0,

@@ -45,6 +45,8 @@ int split_variants(int n);
 // Density groups of a launch (gridDim.y): enough blocks to fill every SM several times over,
 // while each block still reuses its per-block setup for a run of densities.
 unsigned density_groups(long long blocks, int cnt);
+// The same for the plane passes (one block a plane, min_blocks of them an SM).
+unsigned plane_groups(int nz, int cnt, int min_blocks);
 
 // Rounds of a launch (see clk::RoundPhase): their list, count and the distance of their grids.
 struct Rounds {
@@ -80,11 +82,13 @@ bool xinv(cudaStream_t s, Variant v, cx<T>* buf, long long M, const cx<T>* tw, c
 // transformed along x and y and every plane is stored; inverse: planes are transformed back
 // along y and x and the round's values at the atoms are written to out.
 bool plane_supported(bool fp32, int nx, int ny);
-// Quadrant forward plane pass (plane_q.cuh): FP32 128 x 128 sub-lattice planes, atoms in
-// [0, 64)^2.
-bool quadrant_supported(bool fp32, int nx, int ny);
-bool qfwd(cudaStream_t s, const cx<float>* rho, long long rho_stride, const int* row_ptr, const int* cell,
-          cx<float>* buf, long long M, const cx<float>* tw, int nz, int cnt);
+// Quadrant plane passes of the FP32 sub-lattice forms (plane_w.cuh): n x n planes with atoms in their
+// [0, n/2)^2 quadrant, x and y transforms both in one launch.
+bool quadrant_supported(int nx, int ny);
+bool pfwd(cudaStream_t s, const cx<float>* rho, long long rho_stride, const int* row_ptr, const int* cell,
+          cx<float>* buf, long long M, const cx<float>* tw, int n, int nz, int cnt);
+bool pinv(cudaStream_t s, const cx<float>* buf, long long M, const cx<float>* tw, const int* row_ptr, const int* cell,
+          cx<float>* out, long long o_stride, int n, int nz, int cnt);
 template <typename T>
 bool xyfwd(cudaStream_t s, const cx<T>* rho, long long rho_stride, const int* row_ptr, const int* cell, cx<T>* buf,
            long long M, const cx<T>* tw, const clk::RoundPhase& rp, int nx, int ny, int nz, int cnt);
