@@ -285,7 +285,7 @@ class CoulombCalculator:
         s = np.ascontiguousarray(np.asarray(specs, dtype=np.int16).reshape(-1, 4))
         out = np.zeros(2 * s.shape[0])
         _check(lib().cl_compute(self._h, s.shape[0], _ptr(s, ctypes.c_int16), _ptr(out)))
-        return out[0::2] + 1j * out[1::2]
+        return out.view(np.complex128)
 
     def compute_states(self, states, cells, n_holes, specs):
         """cl_compute_states: set_states + compute in one call, the coefficient upload
@@ -298,7 +298,7 @@ class CoulombCalculator:
         _check(lib().cl_compute_states(self._h, n, int(n_holes), a, o, _ptr(c.view(np.float64)),
                                        _ptr(cl_, ctypes.c_int64), s.shape[0], _ptr(s, ctypes.c_int16), _ptr(out)))
         self.n_states, self.n_atoms = n, a
-        return out[0::2] + 1j * out[1::2]
+        return out.view(np.complex128)
 
     def compute_states_raw(self, n_states, n_holes, n_atoms, n_orb, coeff_ptr, cells_ptr, n_int, spec_ptr,
                            out_ptr):
@@ -315,7 +315,7 @@ class CoulombCalculator:
         s = np.ascontiguousarray(np.asarray(specs, dtype=np.int16).reshape(-1, 4))
         out = np.zeros(2 * s.shape[0])
         _check(lib().cl_compute_rounds(self._h, s.shape[0], _ptr(s, ctypes.c_int16), int(round_mask), _ptr(out)))
-        return out[0::2] + 1j * out[1::2]
+        return out.view(np.complex128)
 
     def compute_shard(self, specs, shard, n_shards):
         """cl_compute_shard: the integrals whose left density is dealt to `shard` of `n_shards`
@@ -324,7 +324,7 @@ class CoulombCalculator:
         out = np.zeros(2 * s.shape[0])
         _check(lib().cl_compute_shard(self._h, s.shape[0], _ptr(s, ctypes.c_int16), int(shard), int(n_shards),
                                       _ptr(out)))
-        return out[0::2] + 1j * out[1::2]
+        return out.view(np.complex128)
 
     def set_profiling(self, on=True):
         _check(lib().cl_set_profiling(self._h, int(bool(on))))
@@ -360,7 +360,7 @@ class CoulombCalculator:
         return Request(self, specs, shard, n_shards)
 
     def potentials(self):
-        out = np.zeros((self.n_states, self.n_atoms))
+        out = np.empty((self.n_states, self.n_atoms))
         _check(lib().cl_potentials(self._h, _ptr(out)))
         return out
 
@@ -391,7 +391,7 @@ class Request:
 
     def run(self):
         _check(lib().cl_request_run(self._h, _ptr(self.out)))
-        return self.out[0::2] + 1j * self.out[1::2]
+        return self.out.view(np.complex128).copy()
 
     def close(self):
         if getattr(self, "_h", None) is not None and self._h.value:
@@ -419,7 +419,7 @@ class Batch:
 
     def run(self):
         _check(lib().cl_batch_run(self._h, self._outs))
-        return [r.out[0::2] + 1j * r.out[1::2] for r in self.requests]
+        return [r.out.view(np.complex128).copy() for r in self.requests]
 
     def last_ms(self):
         ms = ctypes.c_double()

@@ -260,6 +260,8 @@ struct Sublattice {
     long long tables_version = -1;        // kernel version the tables were built from
 };
 
+struct PairSetup;
+
 struct cl_ctx {
     int device = 0;
     int mode = CL_MODE_FP64_PLAIN;
@@ -294,7 +296,7 @@ struct cl_ctx {
     DevBuf<int> cell_sorted, orig_sorted, row_ptr;
     DevBuf<cx<double>> coeff_stage;  // two states of caller coefficients, input atom order
     long long live_rows = 0;           // rows (y, z) holding at least one atom
-    std::vector<long long> atom_slot;  // input atom -> sorted (deduplicated) slot
+    std::vector<int> atom_slot;        // input atom -> sorted (deduplicated) slot
     std::vector<int64_t> cells_seen;   // the cells of the last load (an identical list skips the sort)
     cudaStream_t copy_stream = nullptr;  // coefficient uploads of cl_compute_states
     std::vector<cudaEvent_t> state_ev;   // one per state: its coefficients are on the device
@@ -306,6 +308,9 @@ struct cl_ctx {
     DevBuf<double> req_o4;
     DevBuf<int> req_ridx;
     DevBuf<float> tc_buf;  // TF32 hi/lo operands of the tensor-core Gram
+    std::unique_ptr<PairSetup, void (*)(PairSetup*)> eager_pairs{nullptr, nullptr};  // lists of the last eager call
+    DevBuf<int> slot_of_atom;      // input atom -> sorted slot (the potentials' gather)
+    DevBuf<double> pot;            // potentials in input atom order
     double timings[4] = {0, 0, 0, 0};
 
     // per-kernel profiling (events recorded around launches on `stream`)
@@ -681,18 +686,22 @@ void run_rounds(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, const
     }
     const size_t round_bytes = sizeof(cx<T>) * (size_t)n_at * n_rounds;  // per density
     const size_t l2_budget = l2_chunk_bytes();
-    size_t budget = (size_t)(0.6 * (double)(free_device_bytes() + c->work.n + c->rounds.n));
-    size_t by_mem = std::max<size_t>(1, budget / (grid_bytes + round_bytes));
-    size_t by_l2 = l2_budget / grid_bytes;
-    int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)np, by_l2 >= 2 ? by_l2 : by_mem));
+    const size_t by_l2 = l2_budget / grid_bytes;
+    const size_t all_rounds = (size_t)np * n_rounds * grid_bytes;
+    const bool few = all_rounds <= (512ull << 20) && l2_budget == 0 && np * n_rounds <= 65535;  // gridDim.y
+    int chunk = std::max(np, 1);
+    size_t budget = SIZE_MAX;  // of this request; the free memory is asked for only when its buffers must grow
+    if (l2_budget != 0 || c->work.n < (few ? all_rounds : np * grid_bytes) || c->rounds.n < np * round_bytes) {
+        budget = (size_t)(0.6 * (double)(free_device_bytes() + c->work.n + c->rounds.n));
+        const size_t by_mem = std::max<size_t>(1, budget / (grid_bytes + round_bytes));
+        chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)chunk, by_l2 >= 2 ? by_l2 : by_mem));
+    }
     // All rounds in one launch of each pass where their grids take at most 512 MB: 8 rounds of launches
     // become one, and a small grid's rounds fill the SMs together (B200, a request's kernels: 32^3 in FP64,
     // 10 densities, 0.388 -> 0.120 ms; 45^3 in FP32, 10 densities, 0.471 -> 0.183; 64^3 in FP64, one
     // density, 0.360 -> 0.127).  Larger grids fill the SMs round by round and keep one
     // round's buffers.
-    const size_t all_rounds = (size_t)np * n_rounds * grid_bytes;
-    const bool together = chunk == np && all_rounds <= std::min<size_t>(512ull << 20, budget / 2) &&
-                          l2_budget == 0 && np * n_rounds <= 65535;  // grids of a launch (gridDim.y)
+    const bool together = few && chunk == np && all_rounds <= budget / 2;
     const int per_launch = together ? n_rounds : 1;
     c->work.alloc(std::max(c->work.n, together ? all_rounds : (size_t)chunk * grid_bytes));
     c->rounds.alloc(std::max(c->rounds.n, (size_t)chunk * round_bytes));
@@ -1024,8 +1033,13 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
     // potentials (v32); otherwise through the rounds buffer, widened to V
     const bool via_tr = fp32 && !v32;
     const size_t at_bytes = via_tr ? sizeof(cx<T>) * (size_t)n_at : 0;
-    size_t budget = (size_t)(0.6 * (double)(free_device_bytes() + c->work.n + c->rounds.n));
-    int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)std::max(np, 1), budget / (grid_bytes + at_bytes)));
+    // the whole request where the buffers kept from the last one hold it (asking the driver for the free
+    // memory takes longer than a small request's launches), else as much as 60% of the free memory holds
+    int chunk = std::max(np, 1);
+    if (c->work.n < chunk * grid_bytes || (via_tr && c->rounds.n < chunk * at_bytes)) {
+        const size_t budget = (size_t)(0.6 * (double)(free_device_bytes() + c->work.n + c->rounds.n));
+        chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)chunk, budget / (grid_bytes + at_bytes)));
+    }
     c->work.alloc(std::max(c->work.n, (size_t)chunk * grid_bytes));
     if (via_tr) c->rounds.alloc(std::max(c->rounds.n, (size_t)chunk * at_bytes));
     cx<T>* buf = reinterpret_cast<cx<T>*>(c->work.p);
@@ -1607,6 +1621,7 @@ void gram(cl_ctx* c, const void* V_any, bool v_f32, long long v_stride, const vo
 // Pair densities rho[p][atom] for products (fl[p], fr[p]) (0-based state indices): the
 // device lists and launch shape are set up once (setup synchronises), the launch itself only
 // enqueues (it can be captured in a CUDA graph).
+}  // namespace
 struct PairSetup {
     DevBuf<clk::PairSeg> segs;  // products grouped by left state, indices into `states` (FP64 kernel)
     clk::PairTri tri{};  // products over at most 12 states (register kernel)
@@ -1621,6 +1636,7 @@ struct PairSetup {
     int np = 0, n_segs = 0, n_used = 0, chunk = 1, blocks = 1;
     size_t smem = 0;
 };
+namespace {
 
 // Tables of the 4 x 4-state tile kernel: used states ascending, padded to a multiple of 4
 // (-1: zero rows); the requested tiles (bi | bj << 16, bi >= bj); and per ordered state pair
@@ -1828,10 +1844,12 @@ void pair_launch(cl_ctx* c, const PairSetup& ps, void* rho) {
 }
 
 void pair_densities(cl_ctx* c, const std::vector<int2>& fl, void* rho) {
-    PairSetup ps;
+    // the lists stay with the context until its next eager call (stream-ordered after this one's launch)
+    if (!c->eager_pairs) c->eager_pairs = {new PairSetup(), [](PairSetup* p) { delete p; }};
+    PairSetup& ps = *c->eager_pairs;
+    ps.reg_ok = ps.tile_ok = false;
     pair_setup(c, fl, ps);
     pair_launch(c, ps, rho);
-    CL_CUDA(cudaStreamSynchronize(c->stream));  // device lists go out of scope
 }
 
 // Device buffer of at least `count` elements, reallocated only when it must grow.
@@ -2131,7 +2149,7 @@ void load_cells(cl_ctx* c, int64_t n_atoms, const int64_t* cells) {
             cell_s.push_back((int)cells[a]);
             orig_s.push_back(a);
         }
-        c->atom_slot[a] = (long long)cell_s.size() - 1;
+        c->atom_slot[a] = (int)cell_s.size() - 1;
     }
     plan_sublattice(c, cell_s);
     int nx = c->n[0];
@@ -2173,6 +2191,7 @@ void load_cells(cl_ctx* c, int64_t n_atoms, const int64_t* cells) {
     c->cell_sorted.upload(cell_s.data(), cell_s.size(), c->stream);
     c->orig_sorted.upload(orig_s.data(), orig_s.size(), c->stream);
     c->row_ptr.upload(rp.data(), rp.size(), c->stream);
+    c->slot_of_atom.upload(c->atom_slot.data(), c->atom_slot.size(), c->stream);
     CL_CUDA(cudaStreamSynchronize(c->stream));
     c->cells_seen.assign(cells, cells + n_atoms);
 }
@@ -2347,38 +2366,53 @@ DensityLayout layout_densities(const std::vector<cl::PlanStep>& plan, int n_stat
     return d;
 }
 
-// Step values (coulombo.cpp:199-207): step s takes the Gram entry of its (left, right) pair,
-// combined for the pair's conjugation flags and conjugated when the left product is.  Long
-// integral lists are mapped on several host threads.
-void map_step_values(const std::vector<cl::PlanStep>& plan, const DensityLayout& d, const double* h, double* out) {
-    const int nr = d.gram.nr;
-    const auto work = [&](size_t i0, size_t i1) {
+// f(begin, end) over [0, n) on several host threads where there is enough to share.
+template <typename F>
+void share_range(size_t n, F&& f) {
+    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t nt = std::min<size_t>(std::min<size_t>(hw, 32), n / 65536 + 1);
+    if (nt <= 1) {
+        f(size_t{0}, n);
+        return;
+    }
+    std::vector<std::thread> pool;
+    for (size_t t = 0; t < nt; ++t) pool.emplace_back([&, t] { f(n * t / nt, n * (t + 1) / nt); });
+    for (auto& th : pool) th.join();
+}
+
+// Where a step's value comes from (coulombo.cpp:199-207): the Gram entry of its (left, right) pair,
+// combined for the pair's conjugation flags and conjugated when the left product is.
+struct StepValue {
+    uint64_t entry : 61, turned : 1, mixed : 1, conj : 1;
+};
+std::vector<StepValue> step_values(const std::vector<cl::PlanStep>& plan, const DensityLayout& d) {
+    std::vector<StepValue> v(plan.size());
+    share_range(plan.size(), [&](size_t i0, size_t i1) {
         for (size_t i = i0; i < i1; ++i) {
             const auto& st = plan[i];
             // a symmetric block holds the pairs with the larger product on the left
             const bool turned = d.sym[st.left.product] && st.left.product < st.right.product;
             const int l = d.slot[turned ? st.right.product : st.left.product];
             const int r = d.rcol[turned ? st.left.product : st.right.product];
-            const double* q = &h[((size_t)l * nr + r) * 4];
-            const double ad = turned ? q[3] : q[2], bc = turned ? q[2] : q[3];
-            const bool rconj = st.left.conjugate != st.right.conjugate;
-            const double re = rconj ? q[0] + q[1] : q[0] - q[1];
-            double im = rconj ? bc - ad : ad + bc;
-            if (st.left.conjugate) im = -im;
-            out[2 * st.id] = re;
-            out[2 * st.id + 1] = im;
+            v[i] = StepValue{(uint64_t)l * d.gram.nr + r, turned, st.left.conjugate != st.right.conjugate,
+                             st.left.conjugate != 0};
         }
-    };
-    const size_t n = plan.size();
-    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
-    const size_t nt = std::min<size_t>(std::min<size_t>(hw, 32), n / 65536 + 1);
-    if (nt <= 1) {
-        work(0, n);
-        return;
-    }
-    std::vector<std::thread> pool;
-    for (size_t t = 0; t < nt; ++t) pool.emplace_back([&, t] { work(n * t / nt, n * (t + 1) / nt); });
-    for (auto& th : pool) th.join();
+    });
+    return v;
+}
+void map_step_values(const std::vector<cl::PlanStep>& plan, const std::vector<StepValue>& from, const double* h,
+                     double* out) {
+    share_range(plan.size(), [&](size_t i0, size_t i1) {
+        for (size_t i = i0; i < i1; ++i) {
+            const StepValue v = from[i];
+            const double* q = h + 4 * v.entry;
+            const double ad = v.turned ? q[3] : q[2], bc = v.turned ? q[2] : q[3];
+            const double im = v.mixed ? bc - ad : ad + bc;
+            double* o = out + 2 * (size_t)plan[i].id;
+            o[0] = v.mixed ? q[0] + q[1] : q[0] - q[1];
+            o[1] = v.conj ? -im : im;
+        }
+    });
 }
 
 // The steps of shard `shard` of `n_shards`: the plan's prepared (left) densities, in ascending
@@ -2452,7 +2486,7 @@ void compute_impl(cl_ctx* c, int64_t n_int, const int16_t* spec, double* out, in
         c->timings[2] = t23;
         c->timings[3] = t03;
         prof_collect(c);
-        map_step_values(plan, lay, h.data(), out);
+        map_step_values(plan, step_values(plan, lay), h.data(), out);
     }
 }
 
@@ -2590,7 +2624,7 @@ void compute_states_impl(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, 
     c->timings[2] = t23;
     c->timings[3] = t03;
     prof_collect(c);
-    map_step_values(plan, lay, h.data(), out);
+    map_step_values(plan, step_values(plan, lay), h.data(), out);
 }
 }  // namespace
 
@@ -2655,19 +2689,28 @@ int cl_potentials(cl_ctx* c, double* out) {
         const long long As = c->n_sorted;
         std::vector<int2> fl(n);
         for (int s = 0; s < n; ++s) fl[s] = make_int2(s, s);
-        DevBuf<cx<double>> rho, V;
-        rho.alloc((size_t)n * As);
-        V.alloc((size_t)n * As);
+        DevBuf<cx<double>>& rho = c->req_rho;
+        DevBuf<cx<double>>& V = c->req_V;
+        grow(rho, (size_t)n * As);
+        grow(V, (size_t)n * As);
+        grow(c->pot, (size_t)n * c->n_atoms);
         CL_CUDA(cudaEventRecord(c->ev[0], c->stream));
         pair_densities(c, fl, rho.p);
         CL_CUDA(cudaEventRecord(c->ev[1], c->stream));
-        run_transforms(c, rho.p, As, n, V.p, As, false);
+        const bool v32 = c->sl.active && !fp64_form(c);  // as the inverse passes produce them
+        run_transforms(c, rho.p, As, n, V.p, As, v32);
         CL_CUDA(cudaEventRecord(c->ev[2], c->stream));
-        std::vector<cx<double>> h((size_t)n * As);
-        CL_CUDA(cudaMemcpyAsync(h.data(), V.p, h.size() * sizeof(cx<double>), cudaMemcpyDeviceToHost, c->stream));
+        // the real parts in the caller's atom order: half the bytes over the host link
+        const dim3 grid((unsigned)std::min<long long>((c->n_atoms + 255) / 256, 148LL * 8), n);
+        if (v32)
+            clk::k_potential_of_atoms<float><<<grid, 256, 0, c->stream>>>(reinterpret_cast<const cx<float>*>(V.p), As,
+                                                                         c->slot_of_atom.p, c->n_atoms, c->pot.p);
+        else
+            clk::k_potential_of_atoms<double><<<grid, 256, 0, c->stream>>>(V.p, As, c->slot_of_atom.p, c->n_atoms,
+                                                                          c->pot.p);
+        CL_LAUNCHED();
+        CL_CUDA(cudaMemcpyAsync(out, c->pot.p, sizeof(double) * (size_t)n * c->n_atoms, cudaMemcpyDeviceToHost, c->stream));
         CL_CUDA(cudaStreamSynchronize(c->stream));
-        for (int s = 0; s < n; ++s)
-            for (long long a = 0; a < c->n_atoms; ++a) out[(size_t)s * c->n_atoms + a] = h[(size_t)s * As + c->atom_slot[a]].re;
         float t01, t12;
         CL_CUDA(cudaEventElapsedTime(&t01, c->ev[0], c->ev[1]));
         CL_CUDA(cudaEventElapsedTime(&t12, c->ev[1], c->ev[2]));
@@ -2689,6 +2732,7 @@ struct cl_request {
     int64_t n_int = 0;
     std::vector<cl::PlanStep> plan;
     DensityLayout lay;
+    std::vector<StepValue> values;
     int nl = 0, nr = 0;
     PairSetup ps;
     DevBuf<int> ridx;
@@ -2745,7 +2789,7 @@ void request_finish(cl_request* r, double* out) {
     if (r->n_shards > 1) std::memset(out, 0, sizeof(double) * 2 * (size_t)r->n_int);
     if (r->nl == 0) return;
     check_gram_slot(r->o4_host[4 * (size_t)r->nl * r->nr]);
-    map_step_values(r->plan, r->lay, r->o4_host, out);
+    map_step_values(r->plan, r->values, r->o4_host, out);
 }
 
 }  // namespace
@@ -2781,6 +2825,7 @@ int cl_request_create_shard(cl_ctx* c, int64_t n_int, const int16_t* spec, int s
         r->lay = layout_densities(r->plan, c->n_states, symmetric_blocks(c), false);
         r->nl = r->lay.gram.nl;
         r->nr = r->lay.gram.nr;
+        r->values = step_values(r->plan, r->lay);
         const std::vector<int>& rights = r->lay.rights;
         const std::vector<int2> fl = r->lay.states();
         const long long As = c->n_sorted;

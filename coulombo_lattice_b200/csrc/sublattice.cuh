@@ -192,6 +192,17 @@ __global__ void k_sl_widen(const cx<T>* __restrict__ src, long long s_stride, cx
         d[i] = widen(s[i]);
 }
 
+// out[s][a] = Re V[s][slot[a]] for the states s = blockIdx.y and the atoms a in the caller's order.
+template <typename T>
+__global__ void k_potential_of_atoms(const cx<T>* __restrict__ V, long long v_stride, const int* __restrict__ slot,
+                                     long long n_atoms, double* __restrict__ out) {
+    const cx<T>* v = V + blockIdx.y * v_stride;
+    double* o = out + blockIdx.y * n_atoms;
+    for (long long a = blockIdx.x * (long long)blockDim.x + threadIdx.x; a < n_atoms;
+         a += (long long)gridDim.x * blockDim.x)
+        o[a] = (double)v[slot[a]].re;
+}
+
 // Shared-memory layout of k_zmix_rf: twiddles, z phases, xy phases of the block's columns, the
 // stage exchange and the spectra being mixed.  LL = 8 L lines (class-major, column-minor);
 // LPM pads the spectra so the mixing step's reads (L columns x 32/L frequencies a warp) hit
