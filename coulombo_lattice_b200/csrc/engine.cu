@@ -22,6 +22,7 @@
 #include "host/host_logic.hpp"
 #include "host/status.hpp"
 #include "kernels.cuh"
+#include "pair_mma.cuh"
 #include "passes.hpp"
 #include "gram_dmma.cuh"
 #include "gram_tc.cuh"
@@ -1624,10 +1625,13 @@ void gram(cl_ctx* c, const void* V_any, bool v_f32, long long v_stride, const vo
 }  // namespace
 struct PairSetup {
     DevBuf<clk::PairSeg> segs;  // products grouped by left state, indices into `states` (FP64 kernel)
-    clk::PairTri tri{};  // products over at most 12 states (register kernel)
-    bool reg_ok = false;
-    int grid_reg = 1;
-    // tiles of 4 x 4 states (more than 8 used states, see k_pair_density_tile)
+    // FP64 tensor cores (at most 40 used states, see k_pair_mma)
+    bool mma_ok = false;
+    clk::pm::PairMmaArgs mma{};
+    DevBuf<int> mma_prod;
+    int mma_blocks = 0, mma_grid = 1;  // blocks of 8 states; thread blocks
+    size_t mma_smem = 0;
+    // tiles of 4 x 4 states (see k_pair_density_tile)
     bool tile_ok = false;
     DevBuf<int> tile_states, tiles, tile_prod;
     int ns_pad = 0, n_tiles = 0, tile_atoms = 0, tile_threads = 0, tile_blocks = 0;
@@ -1697,6 +1701,91 @@ void pair_tile_setup(cl_ctx* c, const std::vector<int2>& fl, const std::vector<i
     ps.tile_prod.upload(prod.data(), prod.size(), c->stream);
 }
 
+// f(NB, FOLD) as integral constants for nb blocks of 8 states: FOLD from 16 orbitals on, where the products
+// it leaves out outweigh its shuffles (20 states, 10 orbitals: 0.31 ms without, 0.33 with; 20 orbitals:
+// 0.57 and 0.56; 12 states: 0.139 and 0.126).
+template <typename F>
+void with_pair_mma(int nb, int n_orb, F&& f) {
+    const auto blocks = [&](auto fold) {
+        switch (nb) {
+            case 1: f(std::integral_constant<int, 1>{}, fold); break;
+            case 2: f(std::integral_constant<int, 2>{}, fold); break;
+            case 3: f(std::integral_constant<int, 3>{}, fold); break;
+            case 4: f(std::integral_constant<int, 4>{}, fold); break;
+            default: f(std::integral_constant<int, 5>{}, fold); break;
+        }
+    };
+    if (n_orb >= 16)
+        blocks(std::true_type{});
+    else
+        blocks(std::false_type{});
+}
+
+// Tables and launch shape of the tensor-core kernel: used states ascending, the density row of each
+// product (i, j), i >= j in that order (rows are conj(c_x) c_y, x >= y).  Batches hold about 160 values a
+// state, in powers of two from one atom a warp group up -- more where one block an SM runs anyway (30
+// states: 8 atoms 0.53 ms, 4 atoms 0.60) -- two of them in shared memory; when even the smallest does not
+// fit beside the products (40 states in FP64, many orbitals) the tile kernel runs.
+void pair_mma_setup(cl_ctx* c, const std::vector<int2>& fl, const std::vector<int>& used,
+                    const std::vector<int>& where, PairSetup& ps) {
+    using namespace clk::pm;
+    const int n = (int)used.size(), nb = (n + 7) / 8;
+    if (n == 0 || nb > MAX_BLOCKS || ps.np > 32767) return;
+    PairMmaArgs& g = ps.mma;
+    g = PairMmaArgs{};
+    g.n_orb = c->n_orb;
+    g.n = c->n_sorted;
+    g.np = ps.np;
+    g.n_used = n;
+    g.stages = 2;
+    const auto bytes = [&](int at) {
+        const int pitch = state_pitch(at, c->n_orb);
+        return fp64_form(c) ? pair_mma_smem<double>(nb, n, pitch, ps.np, at, g.stages)
+                            : pair_mma_smem<float>(nb, n, pitch, ps.np, at, g.stages);
+    };
+    const size_t most = 227 * 1024;
+    int at = warps(nb) / warps_per_atom(nb);
+    if (bytes(at) > most) return;
+    while (at < 64 && (2 * at * c->n_orb <= 160 || (min_blocks(nb) == 1 && at < 16)) && bytes(2 * at) <= most) at *= 2;
+    g.at = at;
+    while ((1 << g.at_log2) < at) ++g.at_log2;
+    g.state_pitch = state_pitch(at, c->n_orb);
+    std::vector<int> order(n), pos(n);
+    std::iota(order.begin(), order.end(), 0);
+    std::sort(order.begin(), order.end(), [&](int x, int y) { return used[x] < used[y]; });
+    for (int k = 0; k < n; ++k) {
+        pos[order[k]] = k;
+        g.state[k] = used[order[k]];
+    }
+    std::vector<int> prod((size_t)64 * nb * nb, -1);
+    for (int p = 0; p < ps.np; ++p) {
+        const int i = pos[where[fl[p].x]], j = pos[where[fl[p].y]];
+        if (i < j) cl::fail(CL_ERR_STATE, "pair density with its lower state first");
+        int& row = prod[(size_t)i * 8 * nb + j];
+        if (row >= 0) return;  // the same product twice: the kernels with a row per product
+        row = p;
+    }
+    ps.mma_prod.upload(prod.data(), prod.size(), c->stream);
+    ps.mma_ok = true;
+    ps.mma_blocks = nb;
+    ps.mma_smem = bytes(at);
+    const long long batches = (g.n + at - 1) / at;
+    int resident = 1;
+    with_pair_mma(nb, c->n_orb, [&](auto k, auto fold) {
+        constexpr int NB = decltype(k)::value;
+        constexpr bool FOLD = decltype(fold)::value;
+        const auto count = [&](auto kern) {
+            ensure_smem(kern, most);
+            CL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, 32 * warps(NB), ps.mma_smem));
+        };
+        if (fp64_form(c))
+            count(k_pair_mma<NB, FOLD, double>);
+        else
+            count(k_pair_mma<NB, FOLD, float>);
+    });
+    ps.mma_grid = (int)std::max<long long>(1, std::min<long long>(batches, 148LL * std::max(1, resident)));
+}
+
 void pair_setup(cl_ctx* c, const std::vector<int2>& fl, PairSetup& ps) {
     ps.np = (int)fl.size();
     std::vector<int> used;
@@ -1722,31 +1811,10 @@ void pair_setup(cl_ctx* c, const std::vector<int2>& fl, PairSetup& ps) {
         }
     ps.n_segs = (int)segs.size();
     ps.segs.upload(segs.data(), segs.size(), c->stream);
-    // register kernel (at most 12 used states): the used states in ascending order, and the
-    // density row of each product (i, j), i >= j in that order (rows are conj(c_x) c_y, x >= y)
-    // (CL_NO_PAIR_REG12=1: at most 8, the 4 x 4-state tile kernel above that)
-    const size_t reg_max = std::getenv("CL_NO_PAIR_REG12") ? 8 : (size_t)clk::kPairRegStates;
-    ps.reg_ok = !used.empty() && used.size() <= reg_max;
-    if (ps.reg_ok) {
-        std::vector<int> order(used.size());
-        std::iota(order.begin(), order.end(), 0);
-        std::sort(order.begin(), order.end(), [&](int a, int b) { return used[a] < used[b]; });
-        std::vector<int> pos(used.size());
-        for (size_t k = 0; k < order.size(); ++k) {
-            pos[order[k]] = (int)k;
-            ps.tri.states[k] = used[order[k]];
-        }
-        for (size_t k = order.size(); k < (size_t)clk::kPairRegStates; ++k) ps.tri.states[k] = used[order[0]];
-        for (int& v : ps.tri.prod) v = -1;
-        for (int p = 0; p < ps.np; ++p) {
-            const int i = pos[where[fl[p].x]], j = pos[where[fl[p].y]];
-            if (i < j) cl::fail(CL_ERR_STATE, "pair density with its lower state first");
-            ps.tri.prod[i * (i + 1) / 2 + j] = p;
-        }
-        ps.grid_reg = (int)std::max<long long>(
-            1, std::min<long long>((c->n_sorted + clk::kPairAtoms - 1) / clk::kPairAtoms, 148LL * 2 * 4));
-    }
-    if (!ps.reg_ok && !used.empty() && !std::getenv("CL_NO_PAIR_TILE")) pair_tile_setup(c, fl, used, where, ps);
+    // CL_NO_PAIR_REG12=1: the 4 x 4-state tile kernel instead of the tensor cores; CL_NO_PAIR_TILE=1 with it:
+    // the segment kernel
+    if (!std::getenv("CL_NO_PAIR_REG12")) pair_mma_setup(c, fl, used, where, ps);
+    if (!ps.mma_ok && !used.empty() && !std::getenv("CL_NO_PAIR_TILE")) pair_tile_setup(c, fl, used, where, ps);
     ps.states.upload(used.data(), used.size(), c->stream);
     ps.n_used = (int)used.size();
     // two stages of `chunk` atoms, each up to 48 KB (about two blocks per SM)
@@ -1772,55 +1840,31 @@ void pair_setup(cl_ctx* c, const std::vector<int2>& fl, PairSetup& ps) {
     CL_CUDA(cudaStreamSynchronize(c->stream));
 }
 
-// f(std::integral_constant<int, n>) for 1 <= n <= 12 used states
-template <typename F>
-void with_states(int n, F&& f) {
-    switch (n) {
-        case 1: f(std::integral_constant<int, 1>{}); break;
-        case 2: f(std::integral_constant<int, 2>{}); break;
-        case 3: f(std::integral_constant<int, 3>{}); break;
-        case 4: f(std::integral_constant<int, 4>{}); break;
-        case 5: f(std::integral_constant<int, 5>{}); break;
-        case 6: f(std::integral_constant<int, 6>{}); break;
-        case 7: f(std::integral_constant<int, 7>{}); break;
-        case 8: f(std::integral_constant<int, 8>{}); break;
-        case 9: f(std::integral_constant<int, 9>{}); break;
-        case 10: f(std::integral_constant<int, 10>{}); break;
-        case 11: f(std::integral_constant<int, 11>{}); break;
-        default: f(std::integral_constant<int, 12>{}); break;
-    }
-}
-
 void pair_launch(cl_ctx* c, const PairSetup& ps, void* rho) {
     // the shared-memory attribute is per kernel, so another setup (of another group or
     // request) may have lowered it since this one was prepared
     cudaEvent_t e = prof_begin(c);
-    if (fp64_form(c) && ps.reg_ok) {
-        cx<double>* out = static_cast<cx<double>*>(rho);
-        const auto go = [&](auto ns) {
-            constexpr int NS = decltype(ns)::value;
-            const size_t smem = 2 * sizeof(cx<double>) * clk::pair_stage_elems(NS);
-            ensure_smem(clk::k_pair_density_reg<NS, double>, smem);
-            clk::k_pair_density_reg<NS, double><<<ps.grid_reg, clk::kPairAtoms * clk::pair_parts(NS), smem, c->stream>>>(
-                c->coeff.p, c->n_sorted, c->n_orb, nullptr, c->n_sorted, ps.tri, out);
-        };
-        with_states(ps.n_used, go);
+    if (ps.mma_ok) {
+        clk::pm::PairMmaArgs g = ps.mma;
+        g.coeff = c->coeff.p;
+        g.prod = ps.mma_prod.p;
+        with_pair_mma(ps.mma_blocks, g.n_orb, [&](auto k, auto fold) {
+            constexpr int NB = decltype(k)::value;
+            constexpr bool FOLD = decltype(fold)::value;
+            const int threads = 32 * clk::pm::warps(NB);
+            if (fp64_form(c))
+                clk::pm::k_pair_mma<NB, FOLD, double><<<ps.mma_grid, threads, ps.mma_smem, c->stream>>>(
+                    g, static_cast<cx<double>*>(rho));
+            else
+                clk::pm::k_pair_mma<NB, FOLD, float><<<ps.mma_grid, threads, ps.mma_smem, c->stream>>>(
+                    g, static_cast<cx<float>*>(rho));
+        });
     } else if (fp64_form(c) && !ps.tile_ok) {
         ensure_smem(clk::k_pair_density<double>, ps.smem);
         clk::k_pair_density<double><<<ps.blocks, 256, ps.smem, c->stream>>>(
             c->coeff.p, c->n_sorted, c->n_orb, nullptr, c->n_sorted, ps.segs.p, ps.n_segs, ps.states.p,
             ps.n_used, ps.chunk, static_cast<cx<double>*>(rho));
-    } else if (ps.reg_ok) {
-        cx<float>* out = static_cast<cx<float>*>(rho);
-        const auto go = [&](auto ns) {
-            constexpr int NS = decltype(ns)::value;
-            const size_t smem = 2 * sizeof(cx<double>) * clk::pair_stage_elems(NS);
-            ensure_smem(clk::k_pair_density_reg<NS, float>, smem);
-            clk::k_pair_density_reg<NS, float><<<ps.grid_reg, clk::kPairAtoms * clk::pair_parts(NS), smem, c->stream>>>(
-                c->coeff.p, c->n_sorted, c->n_orb, nullptr, c->n_sorted, ps.tri, out);
-        };
-        with_states(ps.n_used, go);
-    } else if (ps.tile_ok) {  // more than 12 states: 4 x 4-state tiles (FP64 sums, rounded once)
+    } else if (ps.tile_ok) {  // 4 x 4-state tiles (FP64 sums, rounded once)
         const auto go = [&](auto tag) {
             using RT = decltype(tag);
             ensure_smem(clk::k_pair_density_tile<RT>, ps.tile_smem);
@@ -1847,7 +1891,7 @@ void pair_densities(cl_ctx* c, const std::vector<int2>& fl, void* rho) {
     // the lists stay with the context until its next eager call (stream-ordered after this one's launch)
     if (!c->eager_pairs) c->eager_pairs = {new PairSetup(), [](PairSetup* p) { delete p; }};
     PairSetup& ps = *c->eager_pairs;
-    ps.reg_ok = ps.tile_ok = false;
+    ps.mma_ok = ps.tile_ok = false;
     pair_setup(c, fl, ps);
     pair_launch(c, ps, rho);
 }

@@ -276,142 +276,8 @@ __global__ void __launch_bounds__(256) k_pair_density(const cx<double>* __restri
 }
 
 // ---------------------------------------------------------------------------------------
-// Pair densities for requests over at most 12 states, summed in FP64 and rounded once to the
-// form's precision RT; products t = i (i + 1) / 2 + j of states i >= j (ascending order) go to
-// rows prod[t] of rho.
-// ---------------------------------------------------------------------------------------
-constexpr int kPairRegStates = 12;
-struct PairTri {
-    int states[kPairRegStates];                             // used states, ascending (coefficient rows)
-    int prod[kPairRegStates * (kPairRegStates + 1) / 2];    // row of product (i, j), i >= j; -1: not requested
-};
-
-// Block = 64 atoms x PARTS warp pairs: the products are split into PARTS parts (t mod PARTS),
-// each taken by the two warps of one part (the part is uniform over a warp: no predicated work;
-// at most 10 FP64 sums per thread: 4 parts up to 8 states, 8 parts up to 12).  The coefficients
-// are staged through shared memory four orbitals at a time: per (state, atom) the 64 contiguous
-// bytes of those orbitals are copied with 16-byte cp.async (coalesced; the next slice is in
-// flight while this one is used), at an 80-byte pitch per atom so that threads on consecutive
-// atoms read distinct banks.  Every coefficient leaves HBM once and each part reads the slice
-// from shared memory.  The barriers are in the kernel body, reached by every thread; only the
-// arithmetic is specialised per part.
-constexpr int kPairAtoms = 64;      // atoms per block and step
-constexpr int kPairOrbSlice = 4;    // orbitals per stage
-__host__ __device__ constexpr int pair_stage_elems(int ns) { return ns * kPairAtoms * (kPairOrbSlice + 1); }
-__host__ __device__ constexpr int pair_parts(int ns) { return ns <= 8 ? 4 : 8; }
-__host__ __device__ constexpr int pair_min_blocks(int ns) { return ns <= 8 ? 2 : 1; }  // <= 128 registers
-
-template <int NS, int PARTS, int H>
-__device__ __forceinline__ void pair_accumulate(const cx<double>* __restrict__ st, int a, double* ar, double* ai) {
-    constexpr int NT = NS * (NS + 1) / 2;
-#pragma unroll
-    for (int o = 0; o < kPairOrbSlice; ++o) {
-        cx<double> c[NS];
-#pragma unroll
-        for (int i = 0; i < NS; ++i) c[i] = st[(i * kPairAtoms + a) * (kPairOrbSlice + 1) + o];
-#pragma unroll
-        for (int i = 0; i < NS; ++i)
-#pragma unroll
-            for (int j = 0; j <= i; ++j) {
-                const int t = i * (i + 1) / 2 + j;
-                if (t % PARTS == H && t < NT) {  // compile-time after unrolling
-                    ar[t / PARTS] += c[i].re * c[j].re + c[i].im * c[j].im;  // conj(c_i) c_j
-                    ai[t / PARTS] += c[i].re * c[j].im - c[i].im * c[j].re;
-                }
-            }
-    }
-}
-
-template <int NS, int PARTS, int H, typename RT>
-__device__ __forceinline__ void pair_store(const PairTri& tri, const double* ar, const double* ai, long long slot,
-                                           long long n_sorted, cx<RT>* __restrict__ rho) {
-    constexpr int NT = NS * (NS + 1) / 2, NH = (NT - H + PARTS - 1) / PARTS;
-#pragma unroll
-    for (int k = 0; k < NH; ++k) {
-        const int p = tri.prod[PARTS * k + H];
-        if (p >= 0) rho[(long long)p * n_sorted + slot] = narrow<RT>(mk(ar[k], ai[k]));
-    }
-}
-
-// The part `part` of the thread, dispatched to the compile-time part H.
-template <int NS, int PARTS, int H = 0>
-__device__ __forceinline__ void pair_accumulate_part(int part, const cx<double>* __restrict__ st, int a, double* ar,
-                                                     double* ai) {
-    if constexpr (H < PARTS) {
-        if (part == H)
-            pair_accumulate<NS, PARTS, H>(st, a, ar, ai);
-        else
-            pair_accumulate_part<NS, PARTS, H + 1>(part, st, a, ar, ai);
-    }
-}
-template <int NS, int PARTS, typename RT, int H = 0>
-__device__ __forceinline__ void pair_store_part(int part, const PairTri& tri, const double* ar, const double* ai,
-                                                long long slot, long long n_sorted, cx<RT>* __restrict__ rho) {
-    if constexpr (H < PARTS) {
-        if (part == H)
-            pair_store<NS, PARTS, H, RT>(tri, ar, ai, slot, n_sorted, rho);
-        else
-            pair_store_part<NS, PARTS, RT, H + 1>(part, tri, ar, ai, slot, n_sorted, rho);
-    }
-}
-
-template <int NS, typename RT>
-__global__ void __launch_bounds__(kPairAtoms * pair_parts(NS), pair_min_blocks(NS))
-    k_pair_density_reg(const cx<double>* __restrict__ coeff, long long n_atoms, int n_orb,
-                       const int* __restrict__ orig, long long n_sorted, const PairTri tri,
-                       cx<RT>* __restrict__ rho) {
-    constexpr int PARTS = pair_parts(NS), THREADS = kPairAtoms * PARTS;
-    constexpr int NT = NS * (NS + 1) / 2, NHM = (NT + PARTS - 1) / PARTS;
-    constexpr int SE = pair_stage_elems(NS);
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    cx<double>* sm = reinterpret_cast<cx<double>*>(smem_raw);
-    const int part = threadIdx.x / kPairAtoms;
-    const int a = threadIdx.x % kPairAtoms;
-    const int n_slices = (n_orb + kPairOrbSlice - 1) / kPairOrbSlice;
-    // the copies of one stage: NS states x 64 atoms x 4 orbitals, 16 bytes each
-    const auto issue = [&](long long a0, int slice, cx<double>* st) {
-        const int na = (int)min((long long)kPairAtoms, n_sorted - a0);
-        for (int e = threadIdx.x; e < NS * kPairAtoms * kPairOrbSlice; e += THREADS) {
-            const int o = e % kPairOrbSlice, r = e / kPairOrbSlice;
-            const int at = r % kPairAtoms, i = r / kPairAtoms;
-            const int orb = slice * kPairOrbSlice + o;
-            cx<double>* dst = st + (i * kPairAtoms + at) * (kPairOrbSlice + 1) + o;
-            if (at < na && orb < n_orb)
-                pd_cp_async16(dst, coeff + ((long long)tri.states[i] * n_atoms + atom_of(orig, a0 + at)) * n_orb + orb);
-            else
-                *dst = mk(0.0, 0.0);
-        }
-        asm volatile("cp.async.commit_group;\n" ::);
-    };
-    const long long gstep = (long long)gridDim.x * kPairAtoms;
-    long long a0 = (long long)blockIdx.x * kPairAtoms;
-    int stage = 0;
-    if (a0 < n_sorted) issue(a0, 0, sm);
-    for (; a0 < n_sorted; a0 += gstep) {
-        double ar[NHM], ai[NHM];
-#pragma unroll
-        for (int k = 0; k < NHM; ++k) ar[k] = ai[k] = 0.0;
-        for (int sl = 0; sl < n_slices; ++sl) {
-            // next stage: this group's next slice, or the next group's first one
-            const long long na0 = sl + 1 < n_slices ? a0 : a0 + gstep;
-            if (na0 < n_sorted) {
-                issue(na0, sl + 1 < n_slices ? sl + 1 : 0, sm + (stage ^ 1) * SE);
-                asm volatile("cp.async.wait_group 1;\n" ::);
-            } else {
-                asm volatile("cp.async.wait_group 0;\n" ::);
-            }
-            __syncthreads();
-            pair_accumulate_part<NS, PARTS>(part, sm + stage * SE, a, ar, ai);
-            __syncthreads();  // the stage is refilled two slices on
-            stage ^= 1;
-        }
-        const long long slot = a0 + a;
-        if (slot < n_sorted) pair_store_part<NS, PARTS, RT>(part, tri, ar, ai, slot, n_sorted, rho);
-    }
-}
-
-// ---------------------------------------------------------------------------------------
-// Pair densities for requests over more than 8 states, in tiles of 4 x 4 states.  The used
+// Pair densities for requests that the tensor-core kernel (pair_mma.cuh) does not hold, in tiles of 4 x 4
+// states.  The used
 // states, ascending and padded to a multiple of 4 (padding rows are zero), form blocks of 4;
 // tile (bi, bj), bi >= bj, holds the products conj(c_i) c_j, i = 4 bi + u, j = 4 bj + v, of
 // which prod[i * ns_pad + j] names the density row (2 p, or 2 p + 1 where the row is the
