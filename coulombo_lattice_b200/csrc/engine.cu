@@ -1318,16 +1318,16 @@ enum class GramKind {
 };
 // FP32 potentials and densities can take either TF32x3 Gram: the fused one splits the operands of its
 // tile (at most 64 x 40 densities) itself, once per tile, the other reads split operands that a pass of
-// their own writes.  Per k-tile of 32 atoms an SM takes 1.06 us for a fused tile and 1.17 us for a
+// their own writes.  Per k-tile of 32 atoms an SM takes 1.06 us for a fused tile and 1.10 us for a
 // 64 x 64 tile after the split, whose pass costs 0.019 us a density (36 densities a side over 2.1M
-// atoms: 0.47 ms in one fused tile; 820: 11.0 ms in 169 tiles, and 1.64 ms the split).  CL_TC_SPLIT=1
+// atoms: 0.47 ms in one fused tile; 820: 5.56 ms in 91 tiles, and 1.64 ms the split).  CL_TC_SPLIT=1
 // keeps the split pass everywhere; CL_TC_FUSED=1 takes the fused Gram at any tile count.
 GramKind gram_kind(const cl_ctx* c, const GramPlan& g, bool v_f32, bool rho_f32, long long n_atoms) {
     if (!use_tc_gram(c) || small_gram(c, n_atoms)) return GramKind::kFp64;
     if (!v_f32 || !rho_f32 || std::getenv("CL_TC_SPLIT")) return GramKind::kSplit;
     if (std::getenv("CL_TC_FUSED")) return GramKind::kFused;
     const double fused = 1.06 * clk::gram_tile_count(tc_tiles(g, clk::tc::BM / 2, clk::tc::WS_MAX_NB / 2));
-    const double split = 1.17 * clk::gram_tile_count(tc_tiles(g, clk::tc::BM / 2, clk::tc::BN / 2)) +
+    const double split = 1.10 * clk::gram_tile_count(tc_tiles(g, clk::tc::BM / 2, clk::tc::BN / 2)) +
                          0.019 * (g.nl + g.nr);
     return fused <= split ? GramKind::kFused : GramKind::kSplit;
 }

@@ -19,7 +19,7 @@
 // the rounding of the parts are ~2^-22 of each product.
 //
 // Operands are staged by TMA (no multicast) into 128-byte-swizzled shared-memory tiles: one
-// warp issues the copies, one lane issues the MMAs, eight warps drain the accumulator.
+// warp issues the copies, one lane issues the MMAs, sixteen warps drain the accumulator.
 // Every wait is bounded by a clock deadline; on expiry the block records an error in the
 // slot after the results, waits (again bounded) for its own copies and MMAs, frees its
 // tensor memory and returns.
@@ -43,7 +43,10 @@ constexpr int A_BYTES = BM * BK * 4;
 constexpr int B_BYTES = BN * BK * 4;
 constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;  // hi and lo of both operands
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
-constexpr int EPI_WARPS = 8;
+// Sixteen warps hide each other's tensor-memory waits: the 40-state Gram took 6.03 ms with eight.  What is
+// left per k-tile (1.10 us) is near the 64 KB of operands each SM draws from L2 (8.8 TB/s over all SMs).
+constexpr int EPI_WARPS = 16;
+constexpr int EPI_COLS = 4 * BN / EPI_WARPS;  // accumulator columns a warp drains (of its 32 lanes)
 constexpr int THREADS = 32 * (2 + EPI_WARPS);
 constexpr uint32_t TMEM_COLS = 4 * BN;  // main x double buffer, correction, unused; FP32
 constexpr long long TIMEOUT_CYCLES = 1LL << 32;  // ~2 s at B200 clocks
@@ -146,6 +149,24 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// Issues the load of 8 consecutive FP32 accumulator columns of this thread's lane (no wait).
+__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+// Waits for this thread's tensor-memory loads; the 16 destination registers pass through the
+// wait, so that no use of them is scheduled before it.
+__device__ __forceinline__ void tmem_wait_ld16(uint32_t* r) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
+                   "+r"(r[15])
+                 :
+                 : "memory");
 }
 
 __device__ __forceinline__ float tf32_rn(float x) {
@@ -315,11 +336,23 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
     } else {
         // ---- epilogue: FP32 accumulator -> FP64 registers ----
-        const int q = warp & 3;             // tensor-memory lane quarter this warp may read
-        const int h = (warp - 2) >> 2;      // column half
-        double acc[64];
+        const int q = warp & 3;                      // tensor-memory lane quarter this warp may read
+        const int c0 = ((warp - 2) >> 2) * EPI_COLS;  // first of its columns
+        double acc[EPI_COLS];
 #pragma unroll
-        for (int i = 0; i < 64; ++i) acc[i] = 0.0;
+        for (int i = 0; i < EPI_COLS; ++i) acc[i] = 0.0;
+        const uint32_t lanes = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)c0;
+        const auto drain = [&](uint32_t col) {
+#pragma unroll
+            for (int j = 0; j < EPI_COLS / 16; ++j) {
+                uint32_t v[16];
+                tmem_ld8_issue(lanes + col + 16 * j, v);
+                tmem_ld8_issue(lanes + col + 16 * j + 8, v + 8);
+                tmem_wait_ld16(v);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) acc[16 * j + i] += (double)__uint_as_float(v[i]);
+            }
+        };
         bool ok = true;
         for (int ch = 0; ch < nchunks; ++ch) {
             const int b = ch & 1;
@@ -330,14 +363,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 break;
             }
             fence_after();
-            const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(b * BN + h * 64);
-            float v[32];
-            tmem_ld32(ta, v);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) acc[i] += (double)v[i];
-            tmem_ld32(ta + 32, v);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) acc[32 + i] += (double)v[i];
+            drain((uint32_t)(b * BN));
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(ACCE + b));
@@ -345,23 +371,14 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (ok) {
             // the correction accumulator is complete with the last chunk's commit
             fence_after();
-            const uint32_t tc_ = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(2 * BN + h * 64);
-            float v[32];
-            tmem_ld32(tc_, v);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) acc[i] += (double)v[i];
-            tmem_ld32(tc_ + 32, v);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) acc[32 + i] += (double)v[i];
-        }
-        if (ok) {
+            drain((uint32_t)(2 * BN));
             const int R = 32 * q + lane;
             const int l = R >> 1, pa = R & 1;
             if (l < tile.nl) {
                 double* row = out4 + ((long long)(tile.l0 + l) * tiles.ldr + tile.r0) * 4;
 #pragma unroll
-                for (int j = 0; j < 64; ++j) {
-                    const int Cg = h * 64 + j;
+                for (int j = 0; j < EPI_COLS; ++j) {
+                    const int Cg = c0 + j;
                     const int r = Cg >> 1, pc = Cg & 1;
                     if (r < tile.nr) {
                         const int qi = (pa == pc) ? pa : 2 + pa;  // ac, bd, ad, bc
@@ -741,24 +758,6 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// Issues the load of 8 consecutive FP32 accumulator columns of this thread's lane (no wait).
-__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t* r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
-}
-// Waits for this thread's tensor-memory loads; the 16 destination registers pass through the
-// wait, so that no use of them is scheduled before it.
-__device__ __forceinline__ void tmem_wait_ld16(uint32_t* r) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
-                   "+r"(r[15])
-                 :
-                 : "memory");
 }
 
 template <int AHEAD>
