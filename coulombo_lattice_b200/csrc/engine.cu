@@ -1070,7 +1070,7 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
     const bool reg_y = register_passes_enabled() && clp::split_variants(ny) > 0;
     const int skip_empty = (reg_x && reg_y && !std::getenv("CL_NO_ROW_SKIP")) ? 1 : 0;
     const bool plane_ok = reg_x && reg_y && clp::plane_supported(fp32, nx, ny);
-    // FP32 square class planes: the quadrant plane passes, at every length compiled the fastest measured
+    // FP32 class planes: the quadrant plane passes, at every length compiled the fastest measured
     // (36 densities of 128 x 128 planes: 0.57 ms forward and 0.74 inverse, the general plane passes 0.94
     // and 0.89; 820 of 64 x 64: 1.37 and 1.58, 1.94 and 1.89; 78 of 48 x 48: 0.082 and 0.081, the
     // separate passes 0.159 and 0.165); CL_NO_QPLANE=1 keeps the general ones
@@ -1124,8 +1124,13 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
         cx<T>* out_c = via_tr ? tr : static_cast<cx<T>*>(V_any) + (long long)p0 * v_stride;
         cudaEvent_t e = prof_begin(c);
         if (qplane) {
-            clp::pfwd(c->stream, reinterpret_cast<const cx<float>*>(rho_c), rho_stride, row_ptr, cell,
-                      reinterpret_cast<cx<float>*>(buf), vM, reinterpret_cast<const cx<float>*>(twx), nx, nz, cnt);
+            const auto* r32 = reinterpret_cast<const cx<float>*>(rho_c);
+            auto* b32 = reinterpret_cast<cx<float>*>(buf);
+            const auto *tx = reinterpret_cast<const cx<float>*>(twx), *ty = reinterpret_cast<const cx<float>*>(twy);
+            if (nx == ny)
+                clp::pfwd(c->stream, r32, rho_stride, row_ptr, cell, b32, vM, tx, nx, nz, cnt);
+            else
+                clp::pfwd_xy(c->stream, r32, rho_stride, row_ptr, cell, b32, vM, tx, ty, nx, ny, nz, cnt);
         } else if (xy_fwd) {
             clp::xyfwd<T>(c->stream, rho_c, rho_stride, row_ptr, cell, buf, vM, twx, rp0, nx, ny, nz, cnt);
         } else if (!(reg_x && clp::xfwd<T>(c->stream, v_xf, rho_c, rho_stride, row_ptr, cell, buf, vM, twx, rp0, nx,
@@ -1171,8 +1176,13 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
         }
         e = prof_begin(c);
         if (qplane) {
-            clp::pinv(c->stream, reinterpret_cast<const cx<float>*>(buf), vM, reinterpret_cast<const cx<float>*>(twx),
-                      row_ptr, cell, reinterpret_cast<cx<float>*>(out_c), out_stride, nx, nz, cnt);
+            const auto* b32 = reinterpret_cast<const cx<float>*>(buf);
+            auto* o32 = reinterpret_cast<cx<float>*>(out_c);
+            const auto *tx = reinterpret_cast<const cx<float>*>(twx), *ty = reinterpret_cast<const cx<float>*>(twy);
+            if (nx == ny)
+                clp::pinv(c->stream, b32, vM, tx, row_ptr, cell, o32, out_stride, nx, nz, cnt);
+            else
+                clp::pinv_xy(c->stream, b32, vM, tx, ty, row_ptr, cell, o32, out_stride, nx, ny, nz, cnt);
         } else if (xy_inv) {
             clp::xyinv<T>(c->stream, buf, vM, twx, row_ptr, cell, out_c, out_stride, nx, ny, nz, cnt);
         } else if (!(reg_x && clp::xinv<T>(c->stream, v_xi, buf, vM, twx, row_ptr, cell, out_c, out_stride, nx, nrows,

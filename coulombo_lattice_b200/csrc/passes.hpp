@@ -82,9 +82,14 @@ bool xinv(cudaStream_t s, Variant v, cx<T>* buf, long long M, const cx<T>* tw, c
 // transformed along x and y and every plane is stored; inverse: planes are transformed back
 // along y and x and the round's values at the atoms are written to out.
 bool plane_supported(bool fp32, int nx, int ny);
-// Quadrant plane passes of the FP32 sub-lattice forms (plane_w.cuh): n x n planes with atoms in their
-// [0, n/2)^2 quadrant, x and y transforms both in one launch.
+// Quadrant plane passes of the FP32 sub-lattice forms (plane_w.cuh): planes with atoms in their
+// [0, nx/2) x [0, ny/2) quadrant, x and y transforms both in one launch; pfwd and pinv on n x n planes,
+// pfwd_xy and pinv_xy on planes of two lengths (plane_xy.cuh).
 bool quadrant_supported(int nx, int ny);
+bool pfwd_xy(cudaStream_t s, const cx<float>* rho, long long rho_stride, const int* row_ptr, const int* cell,
+             cx<float>* buf, long long M, const cx<float>* twx, const cx<float>* twy, int nx, int ny, int nz, int cnt);
+bool pinv_xy(cudaStream_t s, const cx<float>* buf, long long M, const cx<float>* twx, const cx<float>* twy,
+             const int* row_ptr, const int* cell, cx<float>* out, long long o_stride, int nx, int ny, int nz, int cnt);
 bool pfwd(cudaStream_t s, const cx<float>* rho, long long rho_stride, const int* row_ptr, const int* cell,
           cx<float>* buf, long long M, const cx<float>* tw, int n, int nz, int cnt);
 bool pinv(cudaStream_t s, const cx<float>* buf, long long M, const cx<float>* tw, const int* row_ptr, const int* cell,

@@ -7,7 +7,7 @@
 namespace clp {
 
 bool quadrant_supported(int nx, int ny) {
-    return nx == ny && clk::pw::with_plane_w(nx, [](auto) {});
+    return clk::pw::with_plane_w(nx, [](auto) {}) && clk::pw::with_plane_w(ny, [](auto) {});
 }
 
 bool pfwd(cudaStream_t s, const cx<float>* rho, long long rho_stride, const int* row_ptr, const int* cell,

@@ -58,24 +58,23 @@ struct Occupancy {
     unsigned* base;  // [Q], from the plane's first atom
     bool full;       // every quadrant point, in order
 };
-template <int Q, int N, int THREADS>
+// (qx, qy): the quadrant; (nx, ny): the plane.
 __device__ __forceinline__ Occupancy plane_occupancy(unsigned* mem, const int* row_ptr, const int* cell, int z, int a0,
-                                                     int a1) {
-    Occupancy o{mem, mem + 2 * Q, a1 - a0 == Q * Q};
-    for (int i = threadIdx.x; i < 2 * Q; i += THREADS) o.mask[i] = 0;
-    for (int y = threadIdx.x; y < Q; y += THREADS) o.base[y] = row_ptr[z * N + y] - a0;
+                                                     int a1, int qx, int qy, int nx, int ny) {
+    Occupancy o{mem, mem + 2 * qy, a1 - a0 == qx * qy};
+    for (int i = threadIdx.x; i < 2 * qy; i += blockDim.x) o.mask[i] = 0;
+    for (int y = threadIdx.x; y < qy; y += blockDim.x) o.base[y] = row_ptr[z * ny + y] - a0;
     __syncthreads();
     if (!o.full)
-        for (int i = a0 + threadIdx.x; i < a1; i += THREADS) {
-            const int x = cell[i] % N, y = cell[i] / N % N;
+        for (int i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
+            const int x = cell[i] % nx, y = cell[i] / nx % ny;
             atomicOr(&o.mask[2 * y + (x >> 5)], 1u << (x & 31));
         }
     __syncthreads();
     return o;
 }
-// Index (from the plane's first atom) of the atom at (x, y), or -1.
-template <int Q>
-__device__ __forceinline__ int atom_at(const Occupancy& o, int x, int y) {
+// Index (from the plane's first atom) of the atom at (x, y) of a quadrant Q wide, or -1.
+__device__ __forceinline__ int atom_at(const Occupancy& o, int x, int y, int Q) {
     if (o.full) return y * Q + x;
     const unsigned w0 = o.mask[2 * y], w = x < 32 ? w0 : o.mask[2 * y + 1];
     if (!((w >> (x & 31)) & 1u)) return -1;
@@ -96,7 +95,7 @@ __global__ void __launch_bounds__(PlaneW<H, R2, true>::THREADS, PlaneW<H, R2, tr
     const int tid = threadIdx.x, z = blockIdx.x;
     for (int i = tid; i < N; i += THREADS) tw[i] = tw_g[(i / R1) * (i % R1)];  // [t][q]: W^(t q)
     const int a0 = row_ptr[z * N], a1 = row_ptr[z * N + N];
-    const Occupancy occ = plane_occupancy<Q, N, THREADS>(reinterpret_cast<unsigned*>(tw + N), row_ptr, cell, z, a0, a1);
+    const Occupancy occ = plane_occupancy(reinterpret_cast<unsigned*>(tw + N), row_ptr, cell, z, a0, a1, Q, Q, N, N);
     const int per = (np + gridDim.y - 1) / gridDim.y;
     const int p_begin = blockIdx.y * per, p_end = min(np, p_begin + per);
     const bool pairs = occ.full && Q % 2 == 0 && PQ % 2 == 0 && rho_stride % 2 == 0 &&
@@ -111,7 +110,7 @@ __global__ void __launch_bounds__(PlaneW<H, R2, true>::THREADS, PlaneW<H, R2, tr
         } else {
             for (int e = tid; e < Q * Q; e += THREADS) {
                 const int y = e / Q, x = e % Q;
-                const int i = atom_at<Q>(occ, x, y);
+                const int i = atom_at(occ, x, y, Q);
                 if (i >= 0)
                     cp_async<8>(I + y * PQ + x, src + i);
                 else
@@ -211,7 +210,7 @@ __global__ void __launch_bounds__(PlaneW<H, R2, false>::THREADS, PlaneW<H, R2, f
     const int tid = threadIdx.x, z = blockIdx.x;
     for (int i = tid; i < N; i += THREADS) tw[i] = tw_g[(i / R1) * (i % R1)];  // [t][q]: W^(t q)
     const int a0 = row_ptr[z * N], a1 = row_ptr[z * N + N];
-    const Occupancy occ = plane_occupancy<Q, N, THREADS>(reinterpret_cast<unsigned*>(tw + N), row_ptr, cell, z, a0, a1);
+    const Occupancy occ = plane_occupancy(reinterpret_cast<unsigned*>(tw + N), row_ptr, cell, z, a0, a1, Q, Q, N, N);
     const int per = (np + gridDim.y - 1) / gridDim.y;
     const int p_begin = blockIdx.y * per, p_end = min(np, p_begin + per);
     cx<float> v[IX][R2];
@@ -291,7 +290,7 @@ __global__ void __launch_bounds__(PlaneW<H, R2, false>::THREADS, PlaneW<H, R2, f
             idft_first_half<H>(ev, od);
 #pragma unroll
             for (int n = 0; n < H; ++n) {
-                const int i = atom_at<Q>(occ, x, t + R2 * n);
+                const int i = atom_at(occ, x, t + R2 * n, Q);
                 if (i >= 0) op[i] = ev[n];
             }
         }
@@ -299,37 +298,27 @@ __global__ void __launch_bounds__(PlaneW<H, R2, false>::THREADS, PlaneW<H, R2, f
     }
 }
 
-// The compiled split N = 2 H R2 of a plane length; f is called with (H, R2) as SplitTag<H, R2>.
-template <typename F>
-bool with_plane_w(int n, F&& f) {
-    switch (n) {
-#define CLK_PW(N, A, B)      \
+// The compiled splits N = 2 H R2 of the plane lengths; f is called with (H, R2) as SplitTag<H, R2>.
+#define CLK_PW_LENGTHS(X)                                                                              \
+    X(12, 3, 2) X(16, 4, 2) X(18, 3, 3) X(20, 5, 2) X(24, 4, 3) X(30, 5, 3) \
+    X(32, 4, 4) X(36, 6, 3) X(40, 5, 4) X(48, 8, 3) X(50, 5, 5) X(54, 9, 3) \
+    X(60, 6, 5) X(64, 8, 4) X(72, 9, 4) X(80, 8, 5) X(90, 9, 5) X(96, 8, 6) \
+    X(100, 10, 5) X(108, 9, 6) X(120, 10, 6) X(128, 8, 8)
+#define CLK_PW_CASE(N, A, B) \
     case N:                  \
         f(SplitTag<A, B>{}); \
         return true;
-        CLK_PW(12, 3, 2)
-        CLK_PW(16, 4, 2)
-        CLK_PW(18, 3, 3)
-        CLK_PW(20, 5, 2)
-        CLK_PW(24, 4, 3)
-        CLK_PW(30, 5, 3)
-        CLK_PW(32, 4, 4)
-        CLK_PW(36, 6, 3)
-        CLK_PW(40, 5, 4)
-        CLK_PW(48, 8, 3)
-        CLK_PW(50, 5, 5)
-        CLK_PW(54, 9, 3)
-        CLK_PW(60, 6, 5)
-        CLK_PW(64, 8, 4)
-        CLK_PW(72, 9, 4)
-        CLK_PW(80, 8, 5)
-        CLK_PW(90, 9, 5)
-        CLK_PW(96, 8, 6)
-        CLK_PW(100, 10, 5)
-        CLK_PW(108, 9, 6)
-        CLK_PW(120, 10, 6)
-        CLK_PW(128, 8, 8)
-#undef CLK_PW
+template <typename F>
+bool with_plane_w(int n, F&& f) {
+    switch (n) {
+        CLK_PW_LENGTHS(CLK_PW_CASE)
+        default: return false;
+    }
+}
+template <typename F>
+__device__ __forceinline__ bool with_plane_w_device(int n, F&& f) {
+    switch (n) {
+        CLK_PW_LENGTHS(CLK_PW_CASE)
         default: return false;
     }
 }

@@ -51,3 +51,32 @@ def test_lengths(n, drop, monkeypatch):
         cc.set_states(st, cells, 1)
         ref = cc.potentials()
     assert np.abs(pot - ref).max() <= 1e-6 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("drop", [0.0, 0.25])
+@pytest.mark.parametrize("k", range(len(LENGTHS)))
+def test_two_lengths(k, drop):
+    """Planes of two lengths: every length once as x and once as y (against one 7 places on, shorter and
+    longer), two grids of two classes among them when neither length divides by 4."""
+    nx, ny = LENGTHS[k], LENGTHS[(k + 7) % len(LENGTHS)]
+    dims = (2 * nx, 2 * ny, 24)
+    lat = synth.zincblende_lattice((nx // 2, ny // 2, 6))
+    lat = lat[lat[:, 2] < (24 if nx * ny <= 1024 else 4)]
+    rng = np.random.default_rng(k)
+    if drop:
+        lat = lat[rng.random(len(lat)) >= drop]
+    n_states = 4 if nx * ny <= 1024 else 2
+    st = rng.standard_normal((n_states, len(lat), 2)) + 1j * rng.standard_normal((n_states, len(lat), 2))
+    st /= np.sqrt(np.sum(np.abs(st) ** 2, axis=(1, 2), keepdims=True))
+    cells = synth.cell_indices(lat, dims)
+    specs = [tuple(int(v) for v in s) for s in cl.enumerate_integrals("****", n_states, 1)]
+    step = (synth.A_ZB / 4,) * 3
+    want = np.array(H.compute_integrals(list(st), cells, dims, step, specs, dielectric=10.89, onsite=3.0))
+    with cl.CoulombCalculator(dims, step, cl.MODE_FP32_SUBLATTICE) as cc:
+        cc.initialize(dielectric=10.89, onsite=3.0)
+        cc.set_states(st, cells, 1)
+        assert cc.form_info()["lengths"][:2] == (nx, ny)
+        cc.set_profiling(True)
+        got = cc.compute(specs)
+        assert "y_pass" not in cc.kernel_profile()
+    assert np.abs(got - want).max() <= 1e-6 * np.abs(want).max()
