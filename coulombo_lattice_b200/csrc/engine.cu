@@ -254,10 +254,9 @@ struct Sublattice {
     Axis ax[3];                           // plans and twiddles of the transform lengths
     DevBuf<cx<double>> H64, phxy64, phz64;
     DevBuf<cx<float>> H32, phxy32, phz32;
-    // FP32, zinc-blende or two classes: the tables of the z pass that mixes in registers (zmix_wht.cuh)
+    // zinc-blende or two classes: the tables of the z pass that mixes in registers (zmix_wht.cuh)
     bool zw = false;
-    DevBuf<float4> zw_tab;
-    DevBuf<cx<float>> zw_col, zw_zph;
+    DevBuf<unsigned char> zw_tab, zw_col, zw_zph;  // of the form's precision
     long long tables_version = -1;        // kernel version the tables were built from
 };
 
@@ -919,7 +918,7 @@ void ensure_sl_tables(cl_ctx* c) {
     }
     const double denom = (double)((unsigned long long)c->M * 8ull);
     const int blocks = grid_for(nq);
-    sl.zw = fp32 && (sl.zb ? clp::zw_zb_supported(pz) : sl.S == 2 && clp::zw_pair_supported(pz));
+    sl.zw = sl.zb ? clp::zw_zb_supported(pz) : sl.S == 2 && clp::zw_pair_supported(pz);
     if (sl.zb || sl.zw) {
         // raw class kernels in FP64, then their Walsh-Hadamard form (sublattice.cuh) rounded once
         DevBuf<cx<double>> raw;
@@ -944,17 +943,25 @@ void ensure_sl_tables(cl_ctx* c) {
                 // the half's offsets along the axis are its class 0's and that +- 2 (zinc-blende, mod 4)
                 for (int h = 0; h < 2; ++h) zb.sgn[h][d] = sl.off[h * half][d] < 2 ? 1 : -1;
             }
-            if (sl.zb) {
-                sl.zw_tab.alloc((size_t)3 * nq);
-                sl.zw_col.alloc((size_t)7 * nxy);
-                sl.zw_zph.alloc((size_t)2 * pz);
-                clk::k_zw_table<clk::kZwZb><<<blocks, 256, 0, c->stream>>>(raw.p, zb, sl.zw_tab.p);
-                CL_LAUNCHED();
-                clk::k_zw_columns<<<grid_for(nxy), 256, 0, c->stream>>>(zb, sl.zw_col.p, sl.zw_zph.p);
-            } else {
-                sl.zw_tab.alloc((size_t)nq);
-                clk::k_zw_table<clk::kZwPair><<<blocks, 256, 0, c->stream>>>(raw.p, zb, sl.zw_tab.p);
-            }
+            const auto build = [&](auto tag) {
+                using T = decltype(tag);
+                sl.zw_tab.alloc(sizeof(clk::Quad<T>) * (sl.zb ? 3 : 1) * nq);
+                auto* tab = reinterpret_cast<clk::Quad<T>*>(sl.zw_tab.p);
+                if (sl.zb) {
+                    sl.zw_col.alloc(sizeof(cx<T>) * 7 * nxy);
+                    sl.zw_zph.alloc(sizeof(cx<T>) * 2 * pz);
+                    clk::k_zw_table<T, clk::kZwZb><<<blocks, 256, 0, c->stream>>>(raw.p, zb, tab);
+                    CL_LAUNCHED();
+                    clk::k_zw_columns<T><<<grid_for(nxy), 256, 0, c->stream>>>(
+                        zb, reinterpret_cast<cx<T>*>(sl.zw_col.p), reinterpret_cast<cx<T>*>(sl.zw_zph.p));
+                } else {
+                    clk::k_zw_table<T, clk::kZwPair><<<blocks, 256, 0, c->stream>>>(raw.p, zb, tab);
+                }
+            };
+            if (fp32)
+                build(float{});
+            else
+                build(double{});
         } else if (fp32) {
             sl.H32.alloc((size_t)8 * nq);
             clk::k_sl_zb_wht<float><<<blocks, 256, 0, c->stream>>>(raw.p, nq, w, sl.H32.p);
@@ -1070,11 +1077,11 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
     const bool reg_y = register_passes_enabled() && clp::split_variants(ny) > 0;
     const int skip_empty = (reg_x && reg_y && !std::getenv("CL_NO_ROW_SKIP")) ? 1 : 0;
     const bool plane_ok = reg_x && reg_y && clp::plane_supported(fp32, nx, ny);
-    // FP32 class planes: the quadrant plane passes, at every length compiled the fastest measured
+    // Class planes: the quadrant plane passes, at every length compiled the fastest measured
     // (36 densities of 128 x 128 planes: 0.57 ms forward and 0.74 inverse, the general plane passes 0.94
     // and 0.89; 820 of 64 x 64: 1.37 and 1.58, 1.94 and 1.89; 78 of 48 x 48: 0.082 and 0.081, the
     // separate passes 0.159 and 0.165); CL_NO_QPLANE=1 keeps the general ones
-    const bool qplane = fp32 && clp::quadrant_supported(nx, ny) && !std::getenv("CL_NO_QPLANE");
+    const bool qplane = clp::quadrant_supported(fp32, nx, ny) && !std::getenv("CL_NO_QPLANE");
     // no phase in any pass: the rounds' phase tables are never read with kappa = 0
     const clk::RoundPhase rp0{c->ax[0].phase.p, c->ax[1].phase.p, c->ax[2].phase.p, 0, 0, 0, 0, 1, 0};
     cx<T>* out0 = via_tr ? tr : static_cast<cx<T>*>(V_any);
@@ -1116,7 +1123,7 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
     const double atoms = (double)n_at;
     const double live = skip_empty ? (double)c->live_rows / nrows : 1.0;
     const double row_side = (double)c->live_rows / nrows;
-    const double h_bytes = sl.zw ? (sl.zb ? 48.0 : 16.0) * sl.pad[2] * nxy
+    const double h_bytes = sl.zw ? (sl.zb ? 12.0 : 4.0) * sizeof(T) * sl.pad[2] * nxy
                                  : (double)sl.table.nh * sl.pad[2] * nxy * sizeof(cx<T>);
     for (int p0 = 0; p0 < np; p0 += chunk) {
         const int cnt = std::min(chunk, np - p0);
@@ -1124,13 +1131,10 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
         cx<T>* out_c = via_tr ? tr : static_cast<cx<T>*>(V_any) + (long long)p0 * v_stride;
         cudaEvent_t e = prof_begin(c);
         if (qplane) {
-            const auto* r32 = reinterpret_cast<const cx<float>*>(rho_c);
-            auto* b32 = reinterpret_cast<cx<float>*>(buf);
-            const auto *tx = reinterpret_cast<const cx<float>*>(twx), *ty = reinterpret_cast<const cx<float>*>(twy);
             if (nx == ny)
-                clp::pfwd(c->stream, r32, rho_stride, row_ptr, cell, b32, vM, tx, nx, nz, cnt);
+                clp::pfwd<T>(c->stream, rho_c, rho_stride, row_ptr, cell, buf, vM, twx, nx, nz, cnt);
             else
-                clp::pfwd_xy(c->stream, r32, rho_stride, row_ptr, cell, b32, vM, tx, ty, nx, ny, nz, cnt);
+                clp::pfwd_xy<T>(c->stream, rho_c, rho_stride, row_ptr, cell, buf, vM, twx, twy, nx, ny, nz, cnt);
         } else if (xy_fwd) {
             clp::xyfwd<T>(c->stream, rho_c, rho_stride, row_ptr, cell, buf, vM, twx, rp0, nx, ny, nz, cnt);
         } else if (!(reg_x && clp::xfwd<T>(c->stream, v_xf, rho_c, rho_stride, row_ptr, cell, buf, vM, twx, rp0, nx,
@@ -1154,10 +1158,10 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
         e = prof_begin(c);
         bool mixed;
         if (sl.zw) {
-            cx<float>* b32 = reinterpret_cast<cx<float>*>(buf);
-            const cx<float>* t32 = reinterpret_cast<const cx<float>*>(twz);
-            mixed = sl.zb ? clp::zw_zb(c->stream, b32, vM, t32, sl.zw_tab.p, sl.zw_col.p, sl.zw_zph.p, nxy, sl.pad[2], cnt)
-                          : clp::zw_pair(c->stream, b32, vM, t32, sl.zw_tab.p, nxy, sl.pad[2], cnt);
+            const auto* tab = reinterpret_cast<const clk::Quad<T>*>(sl.zw_tab.p);
+            mixed = sl.zb ? clp::zw_zb<T>(c->stream, buf, vM, twz, tab, reinterpret_cast<const cx<T>*>(sl.zw_col.p),
+                                          reinterpret_cast<const cx<T>*>(sl.zw_zph.p), nxy, sl.pad[2], cnt)
+                          : clp::zw_pair<T>(c->stream, buf, vM, twz, tab, nxy, sl.pad[2], cnt);
         } else {
             mixed = clp::zmix<T>(c->stream, buf, vM, twz, H, phxy, phz, mix, sl.zb, nxy, sl.pad[2], cnt);
         }
@@ -1176,13 +1180,10 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
         }
         e = prof_begin(c);
         if (qplane) {
-            const auto* b32 = reinterpret_cast<const cx<float>*>(buf);
-            auto* o32 = reinterpret_cast<cx<float>*>(out_c);
-            const auto *tx = reinterpret_cast<const cx<float>*>(twx), *ty = reinterpret_cast<const cx<float>*>(twy);
             if (nx == ny)
-                clp::pinv(c->stream, b32, vM, tx, row_ptr, cell, o32, out_stride, nx, nz, cnt);
+                clp::pinv<T>(c->stream, buf, vM, twx, row_ptr, cell, out_c, out_stride, nx, nz, cnt);
             else
-                clp::pinv_xy(c->stream, b32, vM, tx, ty, row_ptr, cell, o32, out_stride, nx, ny, nz, cnt);
+                clp::pinv_xy<T>(c->stream, buf, vM, twx, twy, row_ptr, cell, out_c, out_stride, nx, ny, nz, cnt);
         } else if (xy_inv) {
             clp::xyinv<T>(c->stream, buf, vM, twx, row_ptr, cell, out_c, out_stride, nx, ny, nz, cnt);
         } else if (!(reg_x && clp::xinv<T>(c->stream, v_xi, buf, vM, twx, row_ptr, cell, out_c, out_stride, nx, nrows,

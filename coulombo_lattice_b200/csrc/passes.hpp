@@ -21,6 +21,8 @@
 
 namespace clk {
 struct SlMix;
+template <typename T>
+struct Quad;
 }
 
 namespace clp {
@@ -82,18 +84,22 @@ bool xinv(cudaStream_t s, Variant v, cx<T>* buf, long long M, const cx<T>* tw, c
 // transformed along x and y and every plane is stored; inverse: planes are transformed back
 // along y and x and the round's values at the atoms are written to out.
 bool plane_supported(bool fp32, int nx, int ny);
-// Quadrant plane passes of the FP32 sub-lattice forms (plane_w.cuh): planes with atoms in their
+// Quadrant plane passes of the sub-lattice forms (plane_w.cuh): planes with atoms in their
 // [0, nx/2) x [0, ny/2) quadrant, x and y transforms both in one launch; pfwd and pinv on n x n planes,
 // pfwd_xy and pinv_xy on planes of two lengths (plane_xy.cuh).
-bool quadrant_supported(int nx, int ny);
-bool pfwd_xy(cudaStream_t s, const cx<float>* rho, long long rho_stride, const int* row_ptr, const int* cell,
-             cx<float>* buf, long long M, const cx<float>* twx, const cx<float>* twy, int nx, int ny, int nz, int cnt);
-bool pinv_xy(cudaStream_t s, const cx<float>* buf, long long M, const cx<float>* twx, const cx<float>* twy,
-             const int* row_ptr, const int* cell, cx<float>* out, long long o_stride, int nx, int ny, int nz, int cnt);
-bool pfwd(cudaStream_t s, const cx<float>* rho, long long rho_stride, const int* row_ptr, const int* cell,
-          cx<float>* buf, long long M, const cx<float>* tw, int n, int nz, int cnt);
-bool pinv(cudaStream_t s, const cx<float>* buf, long long M, const cx<float>* tw, const int* row_ptr, const int* cell,
-          cx<float>* out, long long o_stride, int n, int nz, int cnt);
+bool quadrant_supported(bool fp32, int nx, int ny);
+template <typename T>
+bool pfwd(cudaStream_t s, const cx<T>* rho, long long rho_stride, const int* row_ptr, const int* cell, cx<T>* buf,
+          long long M, const cx<T>* tw, int n, int nz, int cnt);
+template <typename T>
+bool pinv(cudaStream_t s, const cx<T>* buf, long long M, const cx<T>* tw, const int* row_ptr, const int* cell,
+          cx<T>* out, long long o_stride, int n, int nz, int cnt);
+template <typename T>
+bool pfwd_xy(cudaStream_t s, const cx<T>* rho, long long rho_stride, const int* row_ptr, const int* cell, cx<T>* buf,
+             long long M, const cx<T>* twx, const cx<T>* twy, int nx, int ny, int nz, int cnt);
+template <typename T>
+bool pinv_xy(cudaStream_t s, const cx<T>* buf, long long M, const cx<T>* twx, const cx<T>* twy, const int* row_ptr,
+             const int* cell, cx<T>* out, long long o_stride, int nx, int ny, int nz, int cnt);
 template <typename T>
 bool xyfwd(cudaStream_t s, const cx<T>* rho, long long rho_stride, const int* row_ptr, const int* cell, cx<T>* buf,
            long long M, const cx<T>* tw, const clk::RoundPhase& rp, int nx, int ny, int nz, int cnt);
@@ -110,14 +116,16 @@ template <typename T>
 bool zmix(cudaStream_t s, cx<T>* buf, long long stride, const cx<T>* tw, const cx<T>* H, const cx<T>* phxy,
           const cx<T>* phz, const clk::SlMix& mix, bool zb, long long nxy, int nz, int cnt);
 
-// The same for FP32 and the class sets that one thread mixes in registers (zmix_wht.cuh): the zinc-blende
-// classes and two-class sets, with their packed coefficient table (k_zw_table) and, for zinc-blende, the
-// column and z phases (k_zw_columns).  false: no compiled split of nz (nothing launched).
+// The same for the class sets that one thread mixes in registers (zmix_wht.cuh): the zinc-blende classes and
+// two-class sets, with their packed coefficient table (k_zw_table) and, for zinc-blende, the column and z
+// phases (k_zw_columns).  false: no compiled split of nz (nothing launched).
 bool zw_zb_supported(int nz);
 bool zw_pair_supported(int nz);
-bool zw_zb(cudaStream_t s, cx<float>* buf, long long stride, const cx<float>* tw, const float4* tab,
-           const cx<float>* col, const cx<float>* zph, long long nxy, int nz, int cnt);
-bool zw_pair(cudaStream_t s, cx<float>* buf, long long stride, const cx<float>* tw, const float4* tab, long long nxy,
+template <typename T>
+bool zw_zb(cudaStream_t s, cx<T>* buf, long long stride, const cx<T>* tw, const clk::Quad<T>* tab, const cx<T>* col,
+           const cx<T>* zph, long long nxy, int nz, int cnt);
+template <typename T>
+bool zw_pair(cudaStream_t s, cx<T>* buf, long long stride, const cx<T>* tw, const clk::Quad<T>* tab, long long nxy,
              int nz, int cnt);
 
 }  // namespace clp

@@ -1,4 +1,4 @@
-// Launchers of the quadrant plane passes for planes of two lengths (plane_xy.cuh), forward.
+// Launchers of the quadrant plane passes (plane_w.cuh, plane_xy.cuh) for planes of two lengths, forward, in FP32.
 #include <algorithm>
 
 #include "passes_impl.cuh"
@@ -6,11 +6,13 @@
 
 namespace clp {
 
-bool pfwd_xy(cudaStream_t s, const cx<float>* rho, long long rho_stride, const int* row_ptr, const int* cell,
-             cx<float>* buf, long long M, const cx<float>* twx, const cx<float>* twy, int nx, int ny, int nz, int cnt) {
+template <>
+bool pfwd_xy<float>(cudaStream_t s, const cx<float>* rho, long long rho_stride, const int* row_ptr, const int* cell,
+                    cx<float>* buf, long long M, const cx<float>* twx, const cx<float>* twy, int nx, int ny, int nz,
+                    int cnt) {
     return clk::pw::with_plane_w(nx, [&](auto tag) {
-        using P = clk::pw::PlaneXY<decltype(tag)::r1, decltype(tag)::r2, true>;
-        auto kern = clk::pw::k_pfwd_xy<decltype(tag)::r1, decltype(tag)::r2>;
+        using P = clk::pw::PlaneXY<float, decltype(tag)::r1, decltype(tag)::r2, true>;
+        auto kern = clk::pw::k_pfwd_xy<float, decltype(tag)::r1, decltype(tag)::r2>;
         set_smem(kern, 227 * 1024);
         kern<<<dim3((unsigned)nz, plane_groups(nz, cnt, P::resident(ny))), P::THREADS, P::smem(ny), s>>>(
             rho, rho_stride, row_ptr, cell, buf, M, twx, twy, ny, cnt);

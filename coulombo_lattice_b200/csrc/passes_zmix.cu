@@ -18,12 +18,9 @@ constexpr int zmix_lines() {
     return 2;
 }
 
-// FP32 zinc-blende lines of 12 to 128 points take the pass that mixes in registers (zmix_wht.cuh); every
+// Zinc-blende lines of 12 to 128 points take the pass that mixes in registers (zmix_wht.cuh); every
 // length of with_zmix_split in that range has a split there.
-template <typename T>
-constexpr bool mixed_in_registers(int n) {
-    return sizeof(T) == 4 && n >= 12 && n <= 128;
-}
+constexpr bool mixed_in_registers(int n) { return n >= 12 && n <= 128; }
 
 }  // namespace
 
@@ -43,7 +40,7 @@ bool zmix(cudaStream_t s, cx<T>* buf, long long stride, const cx<T>* tw, const c
         const long long blocks = (nxy + L - 1) / L;
         const unsigned groups = density_groups(blocks, cnt);
         if (zb) {
-            if constexpr (!mixed_in_registers<T>(R1 * R2)) {
+            if constexpr (!mixed_in_registers(R1 * R2)) {
                 auto kern = clk::k_zmix_rf<T, R1, R2, L, true>;
                 set_smem(kern, smem);
                 kern<<<dim3((unsigned)blocks, groups), NT, smem, s>>>(buf, stride, tw, H, phxy, phz, mix, nxy, cnt);

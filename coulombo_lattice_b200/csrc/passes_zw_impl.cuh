@@ -33,17 +33,17 @@ unsigned zw_density_groups(long long blocks, int cnt, int groups, int blocks_per
     return best;
 }
 
-template <int SET>
-bool zw_launch(cudaStream_t s, cx<float>* buf, long long stride, const cx<float>* tw, const float4* tab,
-               const cx<float>* col, const cx<float>* zph, long long nxy, int nz, int cnt) {
+template <int SET, typename T>
+bool zw_launch(cudaStream_t s, cx<T>* buf, long long stride, const cx<T>* tw, const clk::Quad<T>* tab,
+               const cx<T>* col, const cx<T>* zph, long long nxy, int nz, int cnt) {
     return clk::with_zw_split<SET>(nz, [&](auto tag) {
         using Tag = decltype(tag);
-        using Lay = clk::ZwLayout<SET, Tag::r1, Tag::r2>;
+        using Lay = clk::ZwLayout<T, SET, Tag::r1, Tag::r2>;
         const long long blocks = (nxy + Lay::L - 1) / Lay::L;
         constexpr int per_sm = Lay::resident(Lay::G) / (Lay::NT * Lay::G);
         const unsigned y = zw_density_groups(blocks, cnt, Lay::G, per_sm);
         const int groups = std::min<int>(Lay::G, (cnt + (int)y - 1) / (int)y);
-        auto kern = clk::k_zw<SET, Tag::r1, Tag::r2>;
+        auto kern = clk::k_zw<T, SET, Tag::r1, Tag::r2>;
         set_smem(kern, Lay::smem(Lay::G));
         kern<<<dim3((unsigned)blocks, y), Lay::NT * groups, Lay::smem(groups), s>>>(buf, stride, tw, tab, col, zph,
                                                                                    nxy, cnt);

@@ -1,4 +1,4 @@
-// Quadrant plane passes of the FP32 sub-lattice forms: the x and y transforms of a class plane in one
+// Quadrant plane passes of the sub-lattice forms: the x and y transforms of a class plane in one
 // kernel each way, for square planes of every length the class-mixing z pass serves (zmix_wht.cuh).
 //
 // A class plane of N x N points (N = 2n/m) holds atoms only in its [0, Q)^2 quadrant, Q = N / 2.  Forward,
@@ -12,16 +12,18 @@
 // inverse, the next RB rows' (or the next plane's first) points are loaded into registers while the
 // current ones are transformed.  The inverse writes its last stage's outputs straight to the atoms.
 //
-// Pitches: the x stage's lanes hold R2 adjacent columns of consecutive rows, so PQ = R2 mod 16 puts a
-// half-warp on consecutive words; a scratch row holds item t's outputs at t TP, TP = ceil(16 / R2) mod
-// 16 and SP = 1 mod 16, so that R2 x (16 / R2) lanes hit distinct banks when written and consecutive
-// lanes consecutive words when read.
+// Pitches, with W = 16 complex values (8 in FP64) a shared-memory wavefront: the x stage's lanes hold R2
+// adjacent columns of consecutive rows, so PQ = R2 mod W puts W lanes on consecutive words; a scratch row
+// holds item t's outputs at t TP, TP = ceil(W / R2) mod W and SP = 1 mod W, so that R2 x (W / R2) lanes hit
+// distinct banks when written and consecutive lanes consecutive words when read.
 //
 // Bound: shared-memory wavefronts and latency at 16 warps an SM; HBM at 64-point planes.  Measured on a B200
 // against the passes these replace (a whole plane in shared memory, one block an SM, and a quadrant forward
 // pass, at 128 points; separate x and y passes at lengths without a plane pass): 36 densities of 128 x 128
 // planes, 2.1M atoms, 0.889 -> 0.570 ms forward (5.3 TB/s) and 0.898 -> 0.746 inverse (4.1); 820 of 64 x
 // 64, 1.94 -> 1.35 (6.4 TB/s) and 1.89 -> 1.55; 78 of 48 x 48, 0.159 -> 0.085 and 0.165 -> 0.084.
+// In FP64: 78 densities of 48 x 48, 0.280 -> 0.138 ms and 0.281 -> 0.140; 36 of 128 x 128 (64 x 64 x 16
+// cells), both ways, 1.08 -> 0.83.
 #pragma once
 
 #include "fft.cuh"
@@ -31,25 +33,32 @@
 namespace clk {
 namespace pw {
 
-constexpr int up_to(int at_least, int rest) { return at_least + ((rest - at_least) % 16 + 16) % 16; }
+// The least number from at_least up that is rest modulo w.
+constexpr int up_to(int at_least, int rest, int w) { return at_least + ((rest - at_least) % w + w) % w; }
 
-template <int H, int R2, bool FWD>
+template <typename T, int H, int R2, bool FWD>
 struct PlaneW {
     static constexpr int R1 = 2 * H, N = R1 * R2, Q = N / 2;
-    static constexpr int PQ = up_to(Q, R2 % 16);
-    static constexpr int TP = up_to(R1, (16 + R2 - 1) / R2 % 16);
-    static constexpr int SP = up_to(R2 * TP, 1);
-    // Threads, and x-stage rows at a time.  Measured (a request's densities, ms): 128-point planes, 256
-    // threads with 32 rows 0.57 forward and 0.80 inverse, with 16 rows 0.60 and 0.74; 512 threads of 64
+    static constexpr int W = 128 / (int)sizeof(cx<T>);  // values a shared-memory wavefront serves
+    static constexpr int PQ = up_to(Q, R2 % W, W);
+    static constexpr int TP = up_to(R1, (W + R2 - 1) / R2 % W, W);
+    static constexpr int SP = up_to(R2 * TP, 1, W);
+    // Threads, and x-stage rows at a time.  Measured in FP32 (a request's densities, ms): 128-point planes,
+    // 256 threads with 32 rows 0.57 forward and 0.80 inverse, with 16 rows 0.60 and 0.74; 512 threads of 64
     // registers 0.63 and 0.76; 64-point planes, 128 threads with 32 rows 0.67 and 0.77, 256 threads 0.72
     // and 0.77, with all 64 rows 0.73 and 0.78; 48-point planes, all rows 0.082 and 0.081, half of them
-    // 0.079 and 0.087.
-    static constexpr int THREADS = N > 96 ? 256 : 128;
-    static constexpr int RB = N > 96 ? (FWD ? 32 : 16) : N > 48 ? (N + 1) / 2 : N;
-    static constexpr size_t smem = sizeof(cx<float>) * ((size_t)N * PQ + (size_t)RB * SP + N) + 3 * Q * sizeof(unsigned);
+    // 0.079 and 0.087.  FP64 planes are twice the size: half the rows, and 256 threads from 65 points on
+    // (64-point planes, 36 densities, 128 threads 0.143 and 0.174, 256 threads 0.158 and 0.187; at 168
+    // registers a thread, one block of 256 an SM, 0.158 and 0.297).
+    static constexpr bool F32 = sizeof(T) == 4;
+    static constexpr int THREADS = N > (F32 ? 96 : 64) ? 256 : 128;
+    static constexpr int RB = F32 ? (N > 96 ? (FWD ? 32 : 16) : N > 48 ? (N + 1) / 2 : N)
+                                  : (N > 96 ? 16 : N > 48 ? (N + 3) / 4 : (N + 1) / 2);
+    static constexpr size_t smem = sizeof(cx<T>) * ((size_t)N * PQ + (size_t)RB * SP + N) + 3 * Q * sizeof(unsigned);
+    static constexpr int kThreads = 512;  // resident at 128 registers
     static constexpr int fit = (int)(228 * 1024 / (smem + 1024));
-    static constexpr int BLOCKS = fit < 1024 / THREADS ? (fit < 1 ? 1 : fit) : 1024 / THREADS;
-    static constexpr int MIN = BLOCKS > 512 / THREADS ? 512 / THREADS : BLOCKS;  // <= 128 registers
+    static constexpr int MOST = kThreads / THREADS < 1 ? 1 : kThreads / THREADS;
+    static constexpr int MIN = fit < MOST ? (fit < 1 ? 1 : fit) : MOST;
 };
 
 // Which quadrant points of the plane hold atoms: 64 bits a row and the row's first atom.
@@ -81,40 +90,41 @@ __device__ __forceinline__ int atom_at(const Occupancy& o, int x, int y, int Q) 
     return (int)(o.base[y] + (x < 32 ? 0 : __popc(w0)) + __popc(w & ((1u << (x & 31)) - 1u)));
 }
 
-template <int H, int R2>
-__global__ void __launch_bounds__(PlaneW<H, R2, true>::THREADS, PlaneW<H, R2, true>::MIN)
-    k_pfwd(const cx<float>* __restrict__ rho, long long rho_stride, const int* __restrict__ row_ptr,
-           const int* __restrict__ cell, cx<float>* __restrict__ out, long long out_stride,
-           const cx<float>* __restrict__ tw_g, int np) {
-    using L = PlaneW<H, R2, true>;
+template <typename T, int H, int R2>
+__global__ void __launch_bounds__(PlaneW<T, H, R2, true>::THREADS, PlaneW<T, H, R2, true>::MIN)
+    k_pfwd(const cx<T>* __restrict__ rho, long long rho_stride, const int* __restrict__ row_ptr,
+           const int* __restrict__ cell, cx<T>* __restrict__ out, long long out_stride,
+           const cx<T>* __restrict__ tw_g, int np) {
+    using L = PlaneW<T, H, R2, true>;
     constexpr int R1 = L::R1, N = L::N, Q = L::Q, PQ = L::PQ, TP = L::TP, SP = L::SP, RB = L::RB, THREADS = L::THREADS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    cx<float>* I = reinterpret_cast<cx<float>*>(smem_raw);
-    cx<float>* S = I + N * PQ;
-    cx<float>* tw = S + RB * SP;
+    cx<T>* I = reinterpret_cast<cx<T>*>(smem_raw);
+    cx<T>* S = I + N * PQ;
+    cx<T>* tw = S + RB * SP;
     const int tid = threadIdx.x, z = blockIdx.x;
     for (int i = tid; i < N; i += THREADS) tw[i] = tw_g[(i / R1) * (i % R1)];  // [t][q]: W^(t q)
     const int a0 = row_ptr[z * N], a1 = row_ptr[z * N + N];
     const Occupancy occ = plane_occupancy(reinterpret_cast<unsigned*>(tw + N), row_ptr, cell, z, a0, a1, Q, Q, N, N);
     const int per = (np + gridDim.y - 1) / gridDim.y;
     const int p_begin = blockIdx.y * per, p_end = min(np, p_begin + per);
-    const bool pairs = occ.full && Q % 2 == 0 && PQ % 2 == 0 && rho_stride % 2 == 0 &&
+    constexpr int PER = 16 / (int)sizeof(cx<T>);  // values a 16-byte copy
+    const bool whole = occ.full && Q % PER == 0 && PQ % PER == 0 && rho_stride % PER == 0 &&
                        reinterpret_cast<uintptr_t>(rho + a0) % 16 == 0;
     const auto copy_in = [&](int p) {
-        const cx<float>* src = rho + (long long)p * rho_stride + a0;
-        if (pairs) {
-            for (int e = tid; e < Q * Q / 2; e += THREADS) {
-                const int y = e / (Q / 2), x = 2 * (e % (Q / 2));
-                pd_cp_async16(I + y * PQ + x, src + 2 * e);
+        const cx<T>* src = rho + (long long)p * rho_stride + a0;
+        if (whole) {
+            for (int e = tid; e < Q * Q / PER; e += THREADS) {
+                const int y = e / (Q / PER), x = PER * (e % (Q / PER));
+                pd_cp_async16(I + y * PQ + x, src + PER * e);
             }
         } else {
             for (int e = tid; e < Q * Q; e += THREADS) {
                 const int y = e / Q, x = e % Q;
                 const int i = atom_at(occ, x, y, Q);
                 if (i >= 0)
-                    cp_async<8>(I + y * PQ + x, src + i);
+                    cp_async<sizeof(cx<T>)>(I + y * PQ + x, src + i);
                 else
-                    I[y * PQ + x] = mk(0.f, 0.f);
+                    I[y * PQ + x] = mk(T(0), T(0));
             }
         }
     };
@@ -126,8 +136,8 @@ __global__ void __launch_bounds__(PlaneW<H, R2, true>::THREADS, PlaneW<H, R2, tr
 #pragma unroll 1
         for (int e = tid; e < Q * R2; e += THREADS) {
             const int x = e % Q, t = e / Q;
-            cx<float>* c = I + t * PQ + x;
-            cx<float> v[H], ev[H], od[H];
+            cx<T>* c = I + t * PQ + x;
+            cx<T> v[H], ev[H], od[H];
 #pragma unroll
             for (int j = 0; j < H; ++j) v[j] = c[(R2 * j) * PQ];
             dft_zero_padded<H>(v, ev, od);
@@ -142,8 +152,8 @@ __global__ void __launch_bounds__(PlaneW<H, R2, true>::THREADS, PlaneW<H, R2, tr
 #pragma unroll 2
         for (int e = tid; e < Q * R1; e += THREADS) {
             const int x = e % Q, q = e / Q;
-            cx<float>* c = I + (R2 * q) * PQ + x;
-            cx<float> u[R2];
+            cx<T>* c = I + (R2 * q) * PQ + x;
+            cx<T> u[R2];
 #pragma unroll
             for (int t = 0; t < R2; ++t) u[t] = t == 0 ? c[0] : cmul(c[t * PQ], tw[t * R1 + q]);
             dft<R2, -1>(u);
@@ -151,7 +161,7 @@ __global__ void __launch_bounds__(PlaneW<H, R2, true>::THREADS, PlaneW<H, R2, tr
             for (int s = 0; s < R2; ++s) c[s * PQ] = u[s];
         }
         __syncthreads();
-        cx<float>* o = out + (long long)p * out_stride + (long long)z * N * N;
+        cx<T>* o = out + (long long)p * out_stride + (long long)z * N * N;
         bool copied = false;
 #pragma unroll 1
         for (int r0 = 0; r0 < N; r0 += RB) {
@@ -160,12 +170,12 @@ __global__ void __launch_bounds__(PlaneW<H, R2, true>::THREADS, PlaneW<H, R2, tr
 #pragma unroll 1
             for (int e = tid; e < rows * R2; e += THREADS) {
                 const int t = e % R2, rr = e / R2;
-                const cx<float>* c = I + (r0 + rr) * PQ + t;
-                cx<float> v[H], ev[H], od[H];
+                const cx<T>* c = I + (r0 + rr) * PQ + t;
+                cx<T> v[H], ev[H], od[H];
 #pragma unroll
                 for (int j = 0; j < H; ++j) v[j] = c[R2 * j];
                 dft_zero_padded<H>(v, ev, od);
-                cx<float>* d = S + rr * SP + t * TP;
+                cx<T>* d = S + rr * SP + t * TP;
 #pragma unroll
                 for (int k = 0; k < H; ++k) {
                     d[2 * k] = ev[k];
@@ -181,12 +191,12 @@ __global__ void __launch_bounds__(PlaneW<H, R2, true>::THREADS, PlaneW<H, R2, tr
 #pragma unroll 2
             for (int e = tid; e < rows * R1; e += THREADS) {
                 const int q = e % R1, rr = e / R1, r = r0 + rr;
-                const cx<float>* d = S + rr * SP + q;
-                cx<float> u[R2];
+                const cx<T>* d = S + rr * SP + q;
+                cx<T> u[R2];
 #pragma unroll
                 for (int t = 0; t < R2; ++t) u[t] = t == 0 ? d[0] : cmul(d[t * TP], tw[t * R1 + q]);
                 dft<R2, -1>(u);
-                cx<float>* orow = o + (r / R2 + R1 * (r % R2)) * N + q;
+                cx<T>* orow = o + (r / R2 + R1 * (r % R2)) * N + q;
 #pragma unroll
                 for (int s = 0; s < R2; ++s) orow[R1 * s] = u[s];
             }
@@ -195,32 +205,32 @@ __global__ void __launch_bounds__(PlaneW<H, R2, true>::THREADS, PlaneW<H, R2, tr
     }
 }
 
-template <int H, int R2>
-__global__ void __launch_bounds__(PlaneW<H, R2, false>::THREADS, PlaneW<H, R2, false>::MIN)
-    k_pinv(const cx<float>* __restrict__ buf, long long stride, const cx<float>* __restrict__ tw_g,
-           const int* __restrict__ row_ptr, const int* __restrict__ cell, cx<float>* __restrict__ out,
+template <typename T, int H, int R2>
+__global__ void __launch_bounds__(PlaneW<T, H, R2, false>::THREADS, PlaneW<T, H, R2, false>::MIN)
+    k_pinv(const cx<T>* __restrict__ buf, long long stride, const cx<T>* __restrict__ tw_g,
+           const int* __restrict__ row_ptr, const int* __restrict__ cell, cx<T>* __restrict__ out,
            long long o_stride, int np) {
-    using L = PlaneW<H, R2, false>;
+    using L = PlaneW<T, H, R2, false>;
     constexpr int R1 = L::R1, N = L::N, Q = L::Q, PQ = L::PQ, TP = L::TP, SP = L::SP, RB = L::RB, THREADS = L::THREADS;
     constexpr int IX = (RB * R1 + THREADS - 1) / THREADS;  // first-stage items of a thread
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    cx<float>* I = reinterpret_cast<cx<float>*>(smem_raw);
-    cx<float>* S = I + N * PQ;
-    cx<float>* tw = S + RB * SP;
+    cx<T>* I = reinterpret_cast<cx<T>*>(smem_raw);
+    cx<T>* S = I + N * PQ;
+    cx<T>* tw = S + RB * SP;
     const int tid = threadIdx.x, z = blockIdx.x;
     for (int i = tid; i < N; i += THREADS) tw[i] = tw_g[(i / R1) * (i % R1)];  // [t][q]: W^(t q)
     const int a0 = row_ptr[z * N], a1 = row_ptr[z * N + N];
     const Occupancy occ = plane_occupancy(reinterpret_cast<unsigned*>(tw + N), row_ptr, cell, z, a0, a1, Q, Q, N, N);
     const int per = (np + gridDim.y - 1) / gridDim.y;
     const int p_begin = blockIdx.y * per, p_end = min(np, p_begin + per);
-    cx<float> v[IX][R2];
+    cx<T> v[IX][R2];
     const auto load = [&](int p, int r0) {  // rows r0.. of density p
-        const cx<float>* src = buf + (long long)p * stride + (long long)z * N * N;
+        const cx<T>* src = buf + (long long)p * stride + (long long)z * N * N;
 #pragma unroll
         for (int a = 0; a < IX; ++a) {
             const int e = tid + a * THREADS, q = e % R1, r = r0 + e / R1;
 #pragma unroll
-            for (int s = 0; s < R2; ++s) v[a][s] = (e < RB * R1 && r < N) ? src[r * N + q + R1 * s] : mk(0.f, 0.f);
+            for (int s = 0; s < R2; ++s) v[a][s] = (e < RB * R1 && r < N) ? src[r * N + q + R1 * s] : mk(T(0), T(0));
         }
     };
     if (p_begin < p_end) load(p_begin, 0);
@@ -234,7 +244,7 @@ __global__ void __launch_bounds__(PlaneW<H, R2, false>::THREADS, PlaneW<H, R2, f
                 const int e = tid + a * THREADS, q = e % R1, rr = e / R1;
                 if (rr < rows) {
                     dft<R2, +1>(v[a]);
-                    cx<float>* d = S + rr * SP + q;
+                    cx<T>* d = S + rr * SP + q;
 #pragma unroll
                     for (int t = 0; t < R2; ++t) d[t * TP] = t == 0 ? v[a][0] : cmulc(v[a][t], tw[t * R1 + q]);
                 }
@@ -248,15 +258,15 @@ __global__ void __launch_bounds__(PlaneW<H, R2, false>::THREADS, PlaneW<H, R2, f
 #pragma unroll 1
             for (int e = tid; e < rows * R2; e += THREADS) {
                 const int t = e % R2, rr = e / R2;
-                const cx<float>* d = S + rr * SP + t * TP;
-                cx<float> ev[H], od[H];
+                const cx<T>* d = S + rr * SP + t * TP;
+                cx<T> ev[H], od[H];
 #pragma unroll
                 for (int k = 0; k < H; ++k) {
                     ev[k] = d[2 * k];
                     od[k] = d[2 * k + 1];
                 }
                 idft_first_half<H>(ev, od);
-                cx<float>* c = I + (r0 + rr) * PQ + t;
+                cx<T>* c = I + (r0 + rr) * PQ + t;
 #pragma unroll
                 for (int n = 0; n < H; ++n) c[R2 * n] = ev[n];
             }
@@ -266,8 +276,8 @@ __global__ void __launch_bounds__(PlaneW<H, R2, false>::THREADS, PlaneW<H, R2, f
 #pragma unroll 2
         for (int e = tid; e < Q * R1; e += THREADS) {
             const int x = e % Q, q = e / Q;
-            cx<float>* c = I + q * PQ + x;
-            cx<float> u[R2];
+            cx<T>* c = I + q * PQ + x;
+            cx<T> u[R2];
 #pragma unroll
             for (int s = 0; s < R2; ++s) u[s] = c[(R1 * s) * PQ];
             dft<R2, +1>(u);
@@ -276,12 +286,12 @@ __global__ void __launch_bounds__(PlaneW<H, R2, false>::THREADS, PlaneW<H, R2, f
         }
         __syncthreads();
         // y, second stage: outputs y = t + R2 n < Q, to the atoms
-        cx<float>* op = out + (long long)p * o_stride + a0;
+        cx<T>* op = out + (long long)p * o_stride + a0;
 #pragma unroll 1
         for (int e = tid; e < Q * R2; e += THREADS) {
             const int x = e % Q, t = e / Q;
-            const cx<float>* c = I + (R1 * t) * PQ + x;
-            cx<float> ev[H], od[H];
+            const cx<T>* c = I + (R1 * t) * PQ + x;
+            cx<T> ev[H], od[H];
 #pragma unroll
             for (int k = 0; k < H; ++k) {
                 ev[k] = c[(2 * k) * PQ];

@@ -1,4 +1,4 @@
-// z pass of the FP32 sub-lattice forms for the two class sets that crystals on the a/4 grid give:
+// z pass of the sub-lattice forms for the two class sets that crystals on the a/4 grid give:
 // the 8 zinc-blende classes modulo 4 and a pair of classes modulo 2.
 //
 // One thread mixes all the classes of R2 frequencies in registers.  A class line of N = 2 H R2
@@ -37,6 +37,8 @@
 // lines, 820 densities, 6.93 -> 4.31 ms; 48-point, 78 densities, 0.309 -> 0.212 ms; two classes,
 // 54 x 72 x 80 grid, 36 densities, 0.587 -> 0.071 ms (k_zmix_rf keeps 8 classes' threads whatever the
 // set).  Without the staging: 1.88, 5.24 and 0.228 ms on the three zinc-blende shapes.
+// In FP64 (4 columns a block, 256 threads an SM at 255 registers): 48-point lines, 78 densities, 0.571 ->
+// 0.362 ms; 64-point, 36 densities, 0.679 -> 0.399; 54 x 72 x 80, two classes, 0.750 -> 0.111.
 #pragma once
 
 #include "fft.cuh"
@@ -334,30 +336,36 @@ __device__ __forceinline__ void idft_first_half(cx<T>* even, cx<T>* odd) {
 
 // Class sets: kZwZb 8 zinc-blende classes modulo 4; kZwPair two classes modulo 2.
 enum { kZwZb = 0, kZwPair = 1 };
-template <int SET>
+// Four values of a (column, frequency): 16-byte pieces of the coefficient table.
+template <typename T>
+struct alignas(16) Quad {
+    T x, y, z, w;
+};
+template <typename T, int SET>
 struct ZwSet {
     static constexpr int S = SET == kZwZb ? 8 : 2;      // classes
-    static constexpr int C = SET == kZwZb ? 3 : 1;      // float4 of coefficients a (column, frequency)
-    static constexpr int L = SET == kZwZb ? 8 : 16;     // columns per block
+    static constexpr int C = SET == kZwZb ? 3 : 1;      // quads of coefficients a (column, frequency)
+    // columns per block: 64 contiguous bytes a plane and class (zinc-blende), 128 (pair)
+    static constexpr int L = (SET == kZwZb ? 64 : 128) / (int)sizeof(cx<T>);
 };
 
-template <int SET, int H, int R2>
+template <typename T, int SET, int H, int R2>
 struct ZwLayout {
-    using Z = ZwSet<SET>;
+    using Z = ZwSet<T, SET>;
     static constexpr int R1 = 2 * H, N = R1 * R2, L = Z::L, LL = Z::S * L;
     static constexpr bool SYM = SET == kZwZb && R2 % 2 == 0;  // coefficients at kz <= N/2 only
     static constexpr int K = SYM ? N / 2 + 1 : N;
-    // Row pitch of one q: the lanes of phase B read 8 columns at consecutive q, so consecutive q start
-    // half a 128-byte row apart (16 columns fill a row by themselves).
-    static constexpr int QP = R2 * LL + (L == 8 ? 8 : 0);
+    // Row pitch of one q: the lanes of phase B read 64 bytes of columns at consecutive q, so consecutive q
+    // start half a 128-byte row apart (a pair's columns fill a row by themselves).
+    static constexpr int QP = R2 * LL + (SET == kZwZb ? L : 0);
     static constexpr int NT = (L * R1 + 31) / 32 * 32;  // threads of a group
     static constexpr int NCOL = SET == kZwZb ? 7 : 0;   // column phases
     static constexpr int NPH = SET == kZwZb ? 2 * N : 0;  // z phases of the two halves
-    static constexpr size_t table = sizeof(float4) * (size_t)Z::C * K * L;
-    static constexpr size_t shared = table + sizeof(cx<float>) * (size_t)(N + NPH + NCOL * L);
-    static constexpr size_t group = sizeof(cx<float>) * ((size_t)R1 * QP + (size_t)(N / 2) * LL);
+    static constexpr size_t table = sizeof(Quad<T>) * (size_t)Z::C * K * L;
+    static constexpr size_t shared = table + sizeof(cx<T>) * (size_t)(N + NPH + NCOL * L);
+    static constexpr size_t group = sizeof(cx<T>) * ((size_t)R1 * QP + (size_t)(N / 2) * LL);
     static constexpr size_t smem(int groups) { return shared + groups * group; }
-    static constexpr int kThreads = 512;  // resident threads at 128 registers
+    static constexpr int kThreads = sizeof(T) == 4 ? 512 : 256;  // resident threads at 128, 255 registers
     static constexpr int resident(int groups) {  // threads an SM holds with blocks of `groups`
         const int by_regs = kThreads / (NT * groups), by_smem = (int)(228 * 1024 / (smem(groups) + 1024));
         return smem(groups) > 227 * 1024 ? 0 : (by_regs < by_smem ? by_regs : by_smem) * NT * groups;
@@ -378,7 +386,7 @@ __device__ __forceinline__ void group_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }
 
-// The mixing coefficients, packed for the kernel: tab[c][kz][ky][kx] float4 with
+// The mixing coefficients, packed for the kernel: tab[c][kz][ky][kx] quads with
 //   zinc-blende   c = 0: alpha^_0..3 / 4;  c = 1, 2: beta'_0..1 / 4, beta'_2..3 / 4 (re, im)
 //   pair          alpha (H_0), beta' (re, im), 0
 // from the FP64 class kernels; beta' = beta e^{i pi k.delta/n}, delta = offset(class 0 of the second
@@ -389,8 +397,8 @@ struct ZwBuild {
     int p[3];             // transform lengths
     int sgn[2][3];        // +-1: half h's axis phase is e^{-+i pi k/P}
 };
-template <int SET>
-__global__ void k_zw_table(const cx<double>* __restrict__ raw, ZwBuild b, float4* __restrict__ tab) {
+template <typename T, int SET>
+__global__ void k_zw_table(const cx<double>* __restrict__ raw, ZwBuild b, Quad<T>* __restrict__ tab) {
     const long long nxy = (long long)b.p[0] * b.p[1], nq = nxy * b.p[2];
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nq;
          q += (long long)gridDim.x * blockDim.x) {
@@ -412,13 +420,12 @@ __global__ void k_zw_table(const cx<double>* __restrict__ raw, ZwBuild b, float4
             wht4(v + 4, be);
 #pragma unroll
             for (int c = 0; c < 4; ++c) be[c] = scale(cmul(be[c], g), 0.25);
-            tab[q] = make_float4((float)(0.25 * al[0].re), (float)(0.25 * al[1].re), (float)(0.25 * al[2].re),
-                                 (float)(0.25 * al[3].re));
-            tab[nq + q] = make_float4((float)be[0].re, (float)be[0].im, (float)be[1].re, (float)be[1].im);
-            tab[2 * nq + q] = make_float4((float)be[2].re, (float)be[2].im, (float)be[3].re, (float)be[3].im);
+            tab[q] = Quad<T>{T(0.25 * al[0].re), T(0.25 * al[1].re), T(0.25 * al[2].re), T(0.25 * al[3].re)};
+            tab[nq + q] = Quad<T>{T(be[0].re), T(be[0].im), T(be[1].re), T(be[1].im)};
+            tab[2 * nq + q] = Quad<T>{T(be[2].re), T(be[2].im), T(be[3].re), T(be[3].im)};
         } else {
             const cx<double> be = cmul(v[1], g);
-            tab[q] = make_float4((float)v[0].re, (float)be.re, (float)be.im, 0.0f);
+            tab[q] = Quad<T>{T(v[0].re), T(be.re), T(be.im), T(0)};
         }
     }
 }
@@ -426,12 +433,13 @@ __global__ void k_zw_table(const cx<double>* __restrict__ raw, ZwBuild b, float4
 // Phases of the zinc-blende mixing that depend on the column, col[i][ky][kx]: x, y, x y of the first
 // half; then with the halves' ratio e^{-i pi (kx dx/nx + ky dy/ny)} = r: r, r x, r y, r x y of the second.
 // zph[h][kz]: the z phase of half h.
-static __global__ void k_zw_columns(ZwBuild b, cx<float>* __restrict__ col, cx<float>* __restrict__ zph) {
+template <typename T>
+__global__ void k_zw_columns(ZwBuild b, cx<T>* __restrict__ col, cx<T>* __restrict__ zph) {
     const int nxy = b.p[0] * b.p[1];
-    const auto put = [](cx<float>* at, double turn) {
+    const auto put = [](cx<T>* at, double turn) {
         double s, c;
         sincospi(-turn, &s, &c);
-        *at = mk((float)c, (float)s);
+        *at = mk(T(c), T(s));
     };
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nxy; i += gridDim.x * blockDim.x) {
         const int kx = i % b.p[0], ky = i / b.p[0];
@@ -453,23 +461,23 @@ static __global__ void k_zw_columns(ZwBuild b, cx<float>* __restrict__ col, cx<f
 // Mixes the 8 zinc-blende classes u[0..7] of one frequency in place: phases (tf, to: those of classes
 // 1-3 and 5-7; t4: class 4), the Walsh-Hadamard transforms of the halves, the alpha/beta step, and back
 // (see sublattice.cuh).  UPPER: the coefficients are those of the mirrored frequency.
-template <bool UPPER>
-__device__ __forceinline__ void zw_mix_zb(cx<float>* const (&u)[8], const cx<float>* tf, const cx<float>* to,
-                                          cx<float> t4, float4 a, float4 b01, float4 b23) {
-    cx<float> f[4] = {*u[0], cmul(*u[1], tf[0]), cmul(*u[2], tf[1]), cmul(*u[3], tf[2])};
-    cx<float> o[4] = {cmul(*u[4], t4), cmul(*u[5], to[0]), cmul(*u[6], to[1]), cmul(*u[7], to[2])};
-    cx<float> xf[4], xo[4];
+template <bool UPPER, typename T>
+__device__ __forceinline__ void zw_mix_zb(cx<T>* const (&u)[8], const cx<T>* tf, const cx<T>* to,
+                                          cx<T> t4, Quad<T> a, Quad<T> b01, Quad<T> b23) {
+    cx<T> f[4] = {*u[0], cmul(*u[1], tf[0]), cmul(*u[2], tf[1]), cmul(*u[3], tf[2])};
+    cx<T> o[4] = {cmul(*u[4], t4), cmul(*u[5], to[0]), cmul(*u[6], to[1]), cmul(*u[7], to[2])};
+    cx<T> xf[4], xo[4];
     wht4(f, xf);
     wht4(o, xo);
-    float al[4] = {a.x, a.y, a.z, a.w};
-    cx<float> be[4] = {mk(b01.x, b01.y), mk(b01.z, b01.w), mk(b23.x, b23.y), mk(b23.z, b23.w)};
+    T al[4] = {a.x, a.y, a.z, a.w};
+    cx<T> be[4] = {mk(b01.x, b01.y), mk(b01.z, b01.w), mk(b23.x, b23.y), mk(b23.z, b23.w)};
     if (UPPER) {
-        const float t0 = al[0], t1 = al[1];
+        const T t0 = al[0], t1 = al[1];
         al[0] = al[3];
         al[3] = t0;
         al[1] = al[2];
         al[2] = t1;
-        const cx<float> s0 = be[0], s1 = be[1];
+        const cx<T> s0 = be[0], s1 = be[1];
         be[0] = mk(be[3].re, -be[3].im);
         be[3] = mk(s0.re, -s0.im);
         be[1] = mk(-be[2].re, be[2].im);
@@ -493,34 +501,35 @@ __device__ __forceinline__ void zw_mix_zb(cx<float>* const (&u)[8], const cx<flo
     }
 }
 
-template <int SET, int H, int R2>
-__global__ void __launch_bounds__(ZwLayout<SET, H, R2>::kThreads, 1)
-    k_zw(cx<float>* __restrict__ buf, long long stride, const cx<float>* __restrict__ tw_g,
-         const float4* __restrict__ tab, const cx<float>* __restrict__ col_g, const cx<float>* __restrict__ zph_g,
+template <typename T, int SET, int H, int R2>
+__global__ void __launch_bounds__(ZwLayout<T, SET, H, R2>::kThreads, 1)
+    k_zw(cx<T>* __restrict__ buf, long long stride, const cx<T>* __restrict__ tw_g,
+         const Quad<T>* __restrict__ tab, const cx<T>* __restrict__ col_g, const cx<T>* __restrict__ zph_g,
          long long nxy, int np) {
-    using Lay = ZwLayout<SET, H, R2>;
-    using Z = ZwSet<SET>;
+    using Lay = ZwLayout<T, SET, H, R2>;
+    using Z = ZwSet<T, SET>;
     constexpr int R1 = Lay::R1, N = Lay::N, L = Lay::L, LL = Lay::LL, QP = Lay::QP, NT = Lay::NT, S = Z::S,
                   K = Lay::K, NCOL = Lay::NCOL, NPH = Lay::NPH;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int g = threadIdx.x / NT, tid = threadIdx.x - g * NT, groups = blockDim.x / NT;
-    float4* tb = reinterpret_cast<float4*>(smem_raw);
-    cx<float>* ST = reinterpret_cast<cx<float>*>(smem_raw + Lay::table) + (size_t)g * (N / 2) * LL;
-    cx<float>* E = reinterpret_cast<cx<float>*>(smem_raw + Lay::table) + (size_t)groups * (N / 2) * LL +
+    Quad<T>* tb = reinterpret_cast<Quad<T>*>(smem_raw);
+    cx<T>* ST = reinterpret_cast<cx<T>*>(smem_raw + Lay::table) + (size_t)g * (N / 2) * LL;
+    cx<T>* E = reinterpret_cast<cx<T>*>(smem_raw + Lay::table) + (size_t)groups * (N / 2) * LL +
                    (size_t)g * R1 * QP;
-    cx<float>* tw = reinterpret_cast<cx<float>*>(smem_raw + Lay::table) +
+    cx<T>* tw = reinterpret_cast<cx<T>*>(smem_raw + Lay::table) +
                     (size_t)groups * ((N / 2) * LL + R1 * QP);
-    cx<float>* zph = tw + N;
-    cx<float>* colp = zph + NPH;
+    cx<T>* zph = tw + N;
+    cx<T>* colp = zph + NPH;
     const long long c0 = (long long)blockIdx.x * L;
     const int cols = (int)min((long long)L, nxy - c0);  // even: nxy is a multiple of 4
     const int per = (np + gridDim.y - 1) / gridDim.y;
     const int p_end = min(np, (int)(blockIdx.y + 1) * per);
-    // stored planes of density p to ST[z][class][column], two columns a copy
+    // stored planes of density p to ST[z][class][column], 16 bytes of columns a copy
+    constexpr int W = 16 / (int)sizeof(cx<T>);
     const auto stage_in = [&](int p) {
-        const cx<float>* src = buf + (long long)p * stride + c0;
-        for (int i = tid; i < (N / 2) * LL / 2; i += NT) {
-            const int col = 2 * (i % (L / 2)), r = i / (L / 2), cls = r % S, z = r / S;
+        const cx<T>* src = buf + (long long)p * stride + c0;
+        for (int i = tid; i < (N / 2) * LL / W; i += NT) {
+            const int col = W * (i % (L / W)), r = i / (L / W), cls = r % S, z = r / S;
             if (col < cols)
                 pd_cp_async16(ST + z * LL + cls * L + col, src + (long long)(cls * (N / 2) + z) * nxy + col);
         }
@@ -530,25 +539,25 @@ __global__ void __launch_bounds__(ZwLayout<SET, H, R2>::kThreads, 1)
     for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = tw_g[i];
     for (int i = threadIdx.x; i < NPH; i += blockDim.x) zph[i] = zph_g[i];
     for (int i = threadIdx.x; i < NCOL * L; i += blockDim.x)
-        colp[i] = i % L < cols ? col_g[(long long)(i / L) * nxy + c0 + i % L] : mk(0.f, 0.f);
+        colp[i] = i % L < cols ? col_g[(long long)(i / L) * nxy + c0 + i % L] : mk(T(0), T(0));
     for (int i = threadIdx.x; i < Z::C * K * L; i += blockDim.x) {
         const int l = i % L, r = i / L, c = r / K, k = r - c * K;
-        tb[i] = l < cols ? tab[((long long)c * N + k) * nxy + c0 + l] : make_float4(0.f, 0.f, 0.f, 0.f);
+        tb[i] = l < cols ? tab[((long long)c * N + k) * nxy + c0 + l] : Quad<T>{T(0), T(0), T(0), T(0)};
     }
     __syncthreads();
     for (; p < p_end; p += groups) {
-        cx<float>* base = buf + (long long)p * stride + c0;
+        cx<T>* base = buf + (long long)p * stride + c0;
         asm volatile("cp.async.wait_all;\n" ::: "memory");
         group_sync(1 + g, NT);  // ST has landed, and E is free (phase A' of the last density is over)
         // phase A
 #pragma unroll 1
         for (int it = tid; it < LL * R2; it += NT) {
             const int line = it % LL, t = it / LL;
-            cx<float> x[H], ev[H], od[H];
+            cx<T> x[H], ev[H], od[H];
 #pragma unroll
             for (int j = 0; j < H; ++j) x[j] = ST[(t + R2 * j) * LL + line];
             dft_zero_padded<H>(x, ev, od);
-            cx<float>* e = E + t * LL + line;
+            cx<T>* e = E + t * LL + line;
 #pragma unroll
             for (int k = 0; k < H; ++k) {
                 e[(2 * k) * QP] = ev[k];
@@ -560,16 +569,16 @@ __global__ void __launch_bounds__(ZwLayout<SET, H, R2>::kThreads, 1)
         // phase B
         if (tid < L * R1) {
             const int col = tid % L, q = tid / L;
-            cx<float>* e = E + q * QP + col;
-            cx<float> w[R2];
+            cx<T>* e = E + q * QP + col;
+            cx<T> w[R2];
 #pragma unroll
             for (int t = 1; t < R2; ++t) w[t] = tw[t * q];
-            cx<float> x[S][R2];
+            cx<T> x[S][R2];
 #pragma unroll
             for (int s = 0; s < S; ++s) {
 #pragma unroll
                 for (int t = 0; t < R2; ++t) {
-                    const cx<float> v = e[t * LL + s * L];
+                    const cx<T> v = e[t * LL + s * L];
                     x[s][t] = t == 0 ? v : cmul(v, w[t]);
                 }
                 dft<R2, -1>(x[s]);
@@ -580,12 +589,12 @@ __global__ void __launch_bounds__(ZwLayout<SET, H, R2>::kThreads, 1)
                     const int k = q + R1 * r;
                     const bool upper = Lay::SYM && r >= R2 / 2;  // compile time
                     const int kt = upper ? N - k : k;
-                    const cx<float> zf = zph[k], zo = zph[N + k];
-                    const cx<float> tf[3] = {cmul(colp[L + col], zf), cmul(colp[col], zf), colp[2 * L + col]};
-                    const cx<float> to[3] = {cmul(colp[5 * L + col], zo), cmul(colp[4 * L + col], zo), colp[6 * L + col]};
-                    cx<float>* const u[8] = {&x[0][r], &x[1][r], &x[2][r], &x[3][r],
+                    const cx<T> zf = zph[k], zo = zph[N + k];
+                    const cx<T> tf[3] = {cmul(colp[L + col], zf), cmul(colp[col], zf), colp[2 * L + col]};
+                    const cx<T> to[3] = {cmul(colp[5 * L + col], zo), cmul(colp[4 * L + col], zo), colp[6 * L + col]};
+                    cx<T>* const u[8] = {&x[0][r], &x[1][r], &x[2][r], &x[3][r],
                                              &x[4][r], &x[5][r], &x[6][r], &x[7][r]};
-                    const float4 a = tb[kt * L + col], b01 = tb[(K + kt) * L + col], b23 = tb[(2 * K + kt) * L + col];
+                    const Quad<T> a = tb[kt * L + col], b01 = tb[(K + kt) * L + col], b23 = tb[(2 * K + kt) * L + col];
                     if (upper)
                         zw_mix_zb<true>(u, tf, to, colp[3 * L + col], a, b01, b23);
                     else
@@ -594,8 +603,8 @@ __global__ void __launch_bounds__(ZwLayout<SET, H, R2>::kThreads, 1)
             } else {
 #pragma unroll
                 for (int r = 0; r < R2; ++r) {
-                    const float4 h = tb[(q + R1 * r) * L + col];
-                    const cx<float> a = x[0][r], b = x[1][r];
+                    const Quad<T> h = tb[(q + R1 * r) * L + col];
+                    const cx<T> a = x[0][r], b = x[1][r];
                     x[0][r] = mk(h.x * a.re + h.y * b.re + h.z * b.im, h.x * a.im + h.y * b.im - h.z * b.re);
                     x[1][r] = mk(h.x * b.re + h.y * a.re - h.z * a.im, h.x * b.im + h.y * a.im + h.z * a.re);
                 }
@@ -613,8 +622,8 @@ __global__ void __launch_bounds__(ZwLayout<SET, H, R2>::kThreads, 1)
         for (int it = tid; it < LL * R2; it += NT) {
             const int line = it % LL, t = it / LL;
             const int cls = line / L, col = line % L;
-            const cx<float>* e = E + t * LL + line;
-            cx<float> ev[H], od[H];
+            const cx<T>* e = E + t * LL + line;
+            cx<T> ev[H], od[H];
 #pragma unroll
             for (int k = 0; k < H; ++k) {
                 ev[k] = e[(2 * k) * QP];
@@ -622,7 +631,7 @@ __global__ void __launch_bounds__(ZwLayout<SET, H, R2>::kThreads, 1)
             }
             idft_first_half<H>(ev, od);
             if (col < cols) {
-                cx<float>* dst = base + (long long)(cls * (N / 2) + t) * nxy + col;
+                cx<T>* dst = base + (long long)(cls * (N / 2) + t) * nxy + col;
 #pragma unroll
                 for (int n = 0; n < H; ++n) dst[(long long)(R2 * n) * nxy] = ev[n];
             }
