@@ -1328,7 +1328,7 @@ enum class GramKind {
     kSplit,  // TF32x3 after the split pass (k_tf32_split, k_gram_tc)
 };
 // FP32 potentials and densities can take either TF32x3 Gram: the fused one splits the operands of its
-// tile (at most 64 x 40 densities) itself, once per tile, the other reads split operands that a pass of
+// tile (at most 64 x 48 densities) itself, once per tile, the other reads split operands that a pass of
 // their own writes.  Per k-tile of 32 atoms an SM takes 1.06 us for a fused tile and 1.10 us for a
 // 64 x 64 tile after the split, whose pass costs 0.019 us a density (36 densities a side over 2.1M
 // atoms: 0.47 ms in one fused tile; 820: 5.56 ms in 91 tiles, and 1.64 ms the split).  CL_TC_SPLIT=1
@@ -1487,15 +1487,19 @@ void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, const cx<f
         CL_CUDA(cudaFuncSetAttribute(k_gram_tc_fused<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         CL_CUDA(cudaFuncSetAttribute(k_gram_tc_fused<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         CL_CUDA(cudaFuncSetAttribute(k_gram_tc_fused<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        CL_CUDA(cudaFuncSetAttribute(k_gram_tc_ws<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        CL_CUDA(cudaFuncSetAttribute(k_gram_tc_ws<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        CL_CUDA(cudaFuncSetAttribute(k_gram_tc_ws<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     });
-    // the warp-specialised kernel takes up to 40 right densities a tile; CL_TC_NO_WS=1 keeps the kernel
-    // whose warps take every role in turn, up to 64
+    // the warp-specialised kernel takes up to 48 right densities a tile, with 8 drain warps up to 40 (96^3,
+    // blocks of 42 and 36 densities: 0.087 ms in three tiles, 0.070 in two wider ones); CL_TC_NO_WS=1 keeps
+    // the kernel whose warps take every role in turn, up to 64
     const bool ws = !std::getenv("CL_TC_NO_WS");
     FusedGram g{};
-    g.tiles = tc_tiles(plan, BM / 2, ws ? WS_MAX_NB / 2 : BN / 2);
+    g.tiles = tc_tiles(plan, BM / 2, ws ? WS_MAX_NB8 / 2 : BN / 2);
+    bool wide = false;
+    if (ws) {
+        const clk::GramTiles wider = tc_tiles(plan, BM / 2, WS_MAX_NB / 2);
+        wide = clk::gram_tile_count(wider) < clk::gram_tile_count(g.tiles);
+        if (wide) g.tiles = wider;
+    }
     int nA = 1, nB = 1;
     for (int b = 0; b < g.tiles.n; ++b) {
         nA = std::max(nA, std::min(g.tiles.wl[b], g.tiles.b[b].nl));
@@ -1529,12 +1533,22 @@ void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, const cx<f
     if (smem2 > 227 * 1024) cl::fail(CL_ERR_UNSUPPORTED, "fused Gram needs %zu bytes of shared memory", smem2);
     cudaEvent_t e = prof_begin(c);
     const dim3 grid(tiles, splits);
+    const auto launch_ws = [&](auto ahead, size_t smem) {
+        constexpr int AHEAD = decltype(ahead)::value;
+        if (wide) {
+            ensure_smem(k_gram_tc_ws<AHEAD, 12>, 227 * 1024);
+            k_gram_tc_ws<AHEAD, 12><<<grid, ws_threads(12), smem, c->stream>>>(g);
+        } else {
+            ensure_smem(k_gram_tc_ws<AHEAD, 8>, 227 * 1024);
+            k_gram_tc_ws<AHEAD, 8><<<grid, ws_threads(8), smem, c->stream>>>(g);
+        }
+    };
     if (ws && smem5 <= 227 * 1024)
-        k_gram_tc_ws<5><<<grid, WS_THREADS, smem5, c->stream>>>(g);
+        launch_ws(std::integral_constant<int, 5>{}, smem5);
     else if (ws && smem3 <= 227 * 1024)
-        k_gram_tc_ws<3><<<grid, WS_THREADS, smem3, c->stream>>>(g);
+        launch_ws(std::integral_constant<int, 3>{}, smem3);
     else if (ws)
-        k_gram_tc_ws<2><<<grid, WS_THREADS, smem2, c->stream>>>(g);
+        launch_ws(std::integral_constant<int, 2>{}, smem2);
     else if (smem5 <= 227 * 1024)
         k_gram_tc_fused<5><<<grid, FUSED_THREADS, smem5, c->stream>>>(g);
     else if (smem3 <= 227 * 1024)

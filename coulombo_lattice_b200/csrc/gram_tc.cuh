@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_gram_tc_fused(const FusedG
 }
 
 // ---------------------------------------------------------------------------------------
-// The fused Gram with its roles in separate warps (at most 40 right densities a block: N <= 80),
+// The fused Gram with its roles in separate warps (at most 48 right densities a block: N <= 96),
 // so that the conversion of k-tile t + 1, the MMAs of k-tile t and the drain of k-tile t - 1
 // run at the same time instead of one after another in every warp:
 //   warps 0-6    copy their items' raw values AHEAD k-tiles ahead with cp.async (16 bytes on
@@ -721,8 +721,9 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_gram_tc_fused(const FusedG
 //   warp 7       lane 0 issues the tile's 12 MMAs once the stage is full and its accumulator
 //                buffer drained (three main buffers in tensor memory, the correction in a
 //                fourth), and commits them to the stage's empty and the buffer's full barrier;
-//   warps 8-15   drain: warp w reads lane quarter w % 4, columns [h DC, h DC + DC) for h =
-//                (w - 8) / 4, DC = N / 2, two k-tiles at a time: the two FP32 values of a
+//   warps 8-     drain: 8 of them up to N = 80, 12 above (36 densities a side: 0.472 ms with 8, 0.483 with
+//                12); warp w reads lane quarter w % 4 and its share (a half, a third) of the column groups
+//                of 8, two k-tiles at a time: the two FP32 values of a
 //                column summed once (round to nearest, unbiased, at most 2^-24 of the pair
 //                against the TF32 parts' 2^-22 of each product) and added to FP64 registers;
 //                the correction accumulator once after the last k-tile.
@@ -732,12 +733,11 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_gram_tc_fused(const FusedG
 constexpr int WS_CONV_WARPS = 7;
 constexpr int WS_MMA_WARP = 7;
 constexpr int WS_DRAIN_WARP0 = 8;
-constexpr int WS_DRAIN_WARPS = 8;
-constexpr int WS_THREADS = 32 * (WS_DRAIN_WARP0 + WS_DRAIN_WARPS);
+constexpr int ws_threads(int drains) { return 32 * (WS_DRAIN_WARP0 + drains); }
 constexpr int WS_NACC = 3;         // main accumulator buffers (128 columns apart)
 constexpr int WS_STAGES = 2;       // MMA operand stages in shared memory
-constexpr int WS_MAX_NB = 80;      // MMA N: at most 40 right densities
-constexpr int WS_MAX_DC = WS_MAX_NB / 2;
+constexpr int WS_MAX_NB = 96;      // MMA N: at most 48 right densities
+constexpr int WS_MAX_NB8 = 80;     // with 8 drain warps: at most 40
 // items of 4 atoms a converter thread takes: 64 left + 40 right densities, 8 items each
 constexpr int WS_ITEMS = ((BM / 2 + WS_MAX_NB / 2) * (BK / 4) + 32 * WS_CONV_WARPS - 1) / (32 * WS_CONV_WARPS);
 
@@ -760,8 +760,8 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-template <int AHEAD>
-__global__ void __launch_bounds__(WS_THREADS, 1) k_gram_tc_ws(const FusedGram g) {
+template <int AHEAD, int DRAINS>
+__global__ void __launch_bounds__(ws_threads(DRAINS), 1) k_gram_tc_ws(const FusedGram g) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -797,7 +797,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_gram_tc_ws(const FusedGram g)
         }
         for (int b = 0; b < WS_NACC; ++b) {
             mbar_init(bar(ACCF + b), 1);
-            mbar_init(bar(ACCE + b), WS_DRAIN_WARPS);
+            mbar_init(bar(ACCE + b), DRAINS);
         }
         mbar_init(bar(DRAIN), 1);
         *abort_flag = 0;
@@ -809,6 +809,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_gram_tc_ws(const FusedGram g)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    constexpr int WS_THREADS = 32 * (WS_DRAIN_WARP0 + DRAINS);
     for (int i = threadIdx.x; i < nd; i += WS_THREADS) {
         if (i < nA) {
             src_tab[i] = g.V + (long long)(la0 + i) * g.v_stride;
@@ -963,8 +964,10 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_gram_tc_ws(const FusedGram g)
     } else {
         // ---- drain warps
         const int q = warp & 3;
-        const int dc = nb / 2;                                // columns a drain warp takes
-        const int col0 = ((warp - WS_DRAIN_WARP0) >> 2) * dc;
+        // columns of this warp: its share of the groups of 8
+        constexpr int PARTS = DRAINS / 4, WS_MAX_DC = (PARTS == 2 ? WS_MAX_NB8 : WS_MAX_NB) / PARTS;
+        const int h = (warp - WS_DRAIN_WARP0) >> 2;
+        const int col0 = nb / 8 * h / PARTS * 8, dc = nb / 8 * (h + 1) / PARTS * 8 - col0;
         const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
         double acc[WS_MAX_DC];
 #pragma unroll
