@@ -306,7 +306,7 @@ struct cl_ctx {
     DevBuf<unsigned char> rounds;  // per-round values at the atoms of a chunk of densities
     DevBuf<cx<double>> req_rho, req_V;
     DevBuf<double> req_o4;
-    DevBuf<int> req_ridx;
+    DevBuf<int> req_rows;
     DevBuf<float> tc_buf;  // TF32 hi/lo operands of the tensor-core Gram
     std::unique_ptr<PairSetup, void (*)(PairSetup*)> eager_pairs{nullptr, nullptr};  // lists of the last eager call
     DevBuf<int> slot_of_atom;      // input atom -> sorted slot (the potentials' gather)
@@ -1406,12 +1406,13 @@ DmmaShape dmma_shape(int ta, int tb) {
 // block's diagonal closer), in whole 8-row tiles of the MMA.
 template <typename SV, typename SR>
 void gram_dmma(cl_ctx* c, const cx<SV>* V, long long v_stride, const cx<SR>* rho, long long r_stride,
-               const int* ridx_dev, const GramPlan& plan, long long n_atoms, double* out4_dev) {
+               const int* rows_dev, const GramPlan& plan, long long n_atoms, double* out4_dev) {
     using namespace clk::dm;
     GramArgs<SV> g{};
     g.V = V;
     g.v_stride = v_stride;
-    g.ridx = ridx_dev;
+    g.lidx = rows_dev;
+    g.ridx = rows_dev ? rows_dev + plan.nl : nullptr;
     g.r_stride = r_stride;
     g.na = n_atoms;
     g.out4 = out4_dev;
@@ -1480,7 +1481,7 @@ void gram_dmma(cl_ctx* c, const cx<SV>* V, long long v_stride, const cx<SR>* rho
 
 // The fused Gram on FP32 operands over the whole atom range (see k_gram_tc_fused).
 void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, const cx<float>* rho, long long r_stride,
-                   const int* ridx_dev, const GramPlan& plan, long long n_atoms, double* out4_dev) {
+                   const int* rows_dev, const GramPlan& plan, long long n_atoms, double* out4_dev) {
     using namespace clk::tc;
     static std::once_flag once;
     std::call_once(once, [] {
@@ -1510,7 +1511,8 @@ void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, const cx<f
     g.v_stride = v_stride;
     g.rho = reinterpret_cast<const float2*>(rho);
     g.r_stride = r_stride;
-    g.ridx = ridx_dev;
+    g.lidx = rows_dev;
+    g.ridx = rows_dev ? rows_dev + plan.nl : nullptr;
     g.na = n_atoms;
     g.out4 = out4_dev;
     g.err = out4_dev + (size_t)4 * plan.nl * plan.nr;
@@ -1561,7 +1563,7 @@ void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, const cx<f
 
 // The split pass and the TF32x3 Gram on its operands, in chunks of the atom range.
 void gram_tc_split(cl_ctx* c, const void* V, bool v_f32, long long v_stride, const void* rho, bool rho_f32,
-                   long long r_stride, const int* ridx_dev, const GramPlan& plan, long long n_atoms, double* out4_dev) {
+                   long long r_stride, const int* rows_dev, const GramPlan& plan, long long n_atoms, double* out4_dev) {
     using namespace clk::tc;
     const int nl = plan.nl, nr = plan.nr;
     const TcShape sh = tc_shape(c, nl, nr, n_atoms);
@@ -1581,17 +1583,17 @@ void gram_tc_split(cl_ctx* c, const void* V, bool v_f32, long long v_stride, con
         const int xblocks = (int)std::min<long long>((kp + 255) / 256, 64);
         if (v_f32)
             clk::tc::k_tf32_split<float><<<dim3(xblocks, nl), 256, 0, c->stream>>>(
-                static_cast<const cx<float>*>(V), v_stride, nullptr, nl, a0, na, sh.k_pad, A);
+                static_cast<const cx<float>*>(V), v_stride, rows_dev, nl, a0, na, sh.k_pad, A);
         else
             clk::tc::k_tf32_split<double><<<dim3(xblocks, nl), 256, 0, c->stream>>>(
-                static_cast<const cx<double>*>(V), v_stride, nullptr, nl, a0, na, sh.k_pad, A);
+                static_cast<const cx<double>*>(V), v_stride, rows_dev, nl, a0, na, sh.k_pad, A);
         CL_LAUNCHED();
         if (rho_f32)
             clk::tc::k_tf32_split<float><<<dim3(xblocks, nr), 256, 0, c->stream>>>(
-                static_cast<const cx<float>*>(rho), r_stride, ridx_dev, nr, a0, na, sh.k_pad, B);
+                static_cast<const cx<float>*>(rho), r_stride, rows_dev ? rows_dev + nl : nullptr, nr, a0, na, sh.k_pad, B);
         else
             clk::tc::k_tf32_split<double><<<dim3(xblocks, nr), 256, 0, c->stream>>>(
-                static_cast<const cx<double>*>(rho), r_stride, ridx_dev, nr, a0, na, sh.k_pad, B);
+                static_cast<const cx<double>*>(rho), r_stride, rows_dev ? rows_dev + nl : nullptr, nr, a0, na, sh.k_pad, B);
         CL_LAUNCHED();
         prof_end(c, e0, CL_KCLASS_GRAM_SPLIT,
                  (double)na * (nl * (v_f32 ? 8.0 : 16.0) + nr * (rho_f32 ? 8.0 : 16.0)) +
@@ -1613,11 +1615,12 @@ void check_gram_slot(double slot) {
 }
 
 // out4[l][r] = {sum ac, bd, ad, bc} over atoms for the pairs of the plan's blocks; out4 holds
-// 4 * nl * nr + 1 doubles, the last one an error slot.  rho: the right densities, complex64 when rho_f32
+// 4 * nl * nr + 1 doubles, the last one an error slot.  rows_dev: the nl rows of V, then the nr rows of rho
+// (null: row l, row r).  rho: the right densities, complex64 when rho_f32
 // (the FP32 form's pair densities), else complex128 (the plain form's, and the grid API's caller-given
 // density).
 void gram(cl_ctx* c, const void* V_any, bool v_f32, long long v_stride, const void* rho_any, bool rho_f32,
-          long long r_stride, const int* ridx_dev, const GramPlan& plan, long long n_atoms, double* out4_dev) {
+          long long r_stride, const int* rows_dev, const GramPlan& plan, long long n_atoms, double* out4_dev) {
     CL_CUDA(cudaMemsetAsync(out4_dev, 0, sizeof(double) * (4 * (size_t)plan.nl * plan.nr + 1), c->stream));
     const auto* v32 = static_cast<const cx<float>*>(V_any);
     const auto* v64 = static_cast<const cx<double>*>(V_any);
@@ -1626,20 +1629,20 @@ void gram(cl_ctx* c, const void* V_any, bool v_f32, long long v_stride, const vo
     switch (gram_kind(c, plan, v_f32, rho_f32, n_atoms)) {
         case GramKind::kFused:
             if (!v_f32 || !rho_f32) cl::fail(CL_ERR_STATE, "the fused Gram needs FP32 operands");
-            gram_tc_fused(c, v32, v_stride, r32, r_stride, ridx_dev, plan, n_atoms, out4_dev);
+            gram_tc_fused(c, v32, v_stride, r32, r_stride, rows_dev, plan, n_atoms, out4_dev);
             break;
         case GramKind::kSplit:
-            gram_tc_split(c, V_any, v_f32, v_stride, rho_any, rho_f32, r_stride, ridx_dev, plan, n_atoms, out4_dev);
+            gram_tc_split(c, V_any, v_f32, v_stride, rho_any, rho_f32, r_stride, rows_dev, plan, n_atoms, out4_dev);
             break;
         case GramKind::kFp64:
             if (v_f32 && rho_f32)
-                gram_dmma(c, v32, v_stride, r32, r_stride, ridx_dev, plan, n_atoms, out4_dev);
+                gram_dmma(c, v32, v_stride, r32, r_stride, rows_dev, plan, n_atoms, out4_dev);
             else if (v_f32)
                 cl::fail(CL_ERR_STATE, "FP32 potentials go with FP32 densities");
             else if (rho_f32)
-                gram_dmma(c, v64, v_stride, r32, r_stride, ridx_dev, plan, n_atoms, out4_dev);
+                gram_dmma(c, v64, v_stride, r32, r_stride, rows_dev, plan, n_atoms, out4_dev);
             else
-                gram_dmma(c, v64, v_stride, r64, r_stride, ridx_dev, plan, n_atoms, out4_dev);
+                gram_dmma(c, v64, v_stride, r64, r_stride, rows_dev, plan, n_atoms, out4_dev);
             break;
     }
 }
@@ -2075,12 +2078,9 @@ int cl_calculate_grid(cl_ctx* c, const double* rho2, double out[2]) {
         c->grid_rho2.upload(reinterpret_cast<const cx<double>*>(rho2), c->M, c->stream);
         DevBuf<double> o4;
         o4.alloc(5);
-        DevBuf<int> ridx;
-        int zero = 0;
-        ridx.upload(&zero, 1, c->stream);
         const GramPlan dot = whole_gram(1, 1, false);
         tc_reserve(c, dot, c->M, false, false);
-        gram(c, c->grid_V.p, false, c->M, c->grid_rho2.p, false, c->M, ridx.p, dot, c->M, o4.p);
+        gram(c, c->grid_V.p, false, c->M, c->grid_rho2.p, false, c->M, nullptr, dot, c->M, o4.p);
         double h[5];
         CL_CUDA(cudaMemcpyAsync(h, o4.p, sizeof h, cudaMemcpyDeviceToHost, c->stream));
         CL_CUDA(cudaStreamSynchronize(c->stream));
@@ -2308,11 +2308,13 @@ int cl_set_states(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, int n_o
 
 namespace {
 
-// The densities of a request: rows (left densities first), right columns, and the blocks of the Gram
-// that its steps read (gram_blocks.hpp).
+// The densities of a request: rows (the left densities, then those only on the right, in ascending product
+// order: ascending higher states), the Gram's columns block by block, and the blocks that its steps read
+// (gram_blocks.hpp).
 struct DensityLayout {
-    std::vector<int> prods, slot;   // product of each row; row of each product, -1: none
-    std::vector<int> rights, rcol;  // row of each right column; column of each product
+    std::vector<int> prods;       // product of each row
+    std::vector<int> columns;     // row of each left, then of each right column of the Gram
+    std::vector<int> lcol, rcol;  // left and right column of each product, -1: none
     std::vector<char> sym;          // per product: pairs with it are read with the larger product on the left
     GramPlan gram;
     // (state, state) of every row, 0-based, the higher first
@@ -2334,10 +2336,9 @@ int symmetric_blocks(const cl_ctx* c, int round_mask = 0xFF) {
     return (round_mask & 0xFF) != 0xFF ? 0 : fp64_form(c) ? 2 : 1;
 }
 
-// Rows and columns go block by block, in ascending product order within a block; with `by_state` (the
-// overlapped upload) all left densities in one block, ordered by their higher state.  `symmetric`: which
-// blocks are treated as symmetric (symmetric_blocks).
-DensityLayout layout_densities(const std::vector<cl::PlanStep>& plan, int n_states, int symmetric, bool by_state) {
+// Columns go in ascending product order within a block.  `symmetric`: which blocks are treated as symmetric
+// (symmetric_blocks).
+DensityLayout layout_densities(const std::vector<cl::PlanStep>& plan, int n_states, int symmetric) {
     const int P = n_states * (n_states + 1) / 2;
     std::vector<char> is_left(P, 0), is_right(P, 0);
     for (const auto& st : plan) {
@@ -2388,7 +2389,15 @@ DensityLayout layout_densities(const std::vector<cl::PlanStep>& plan, int n_stat
         into.rights.insert(into.rights.end(), last.rights.begin(), last.rights.end());
     }
     DensityLayout d;
-    d.slot.assign(P, -1);
+    std::vector<int> row(P, -1);
+    for (const auto* side : {&is_left, &is_right}) {
+        for (int p = 0; p < P; ++p) {
+            if (!(*side)[p] || row[p] >= 0) continue;
+            row[p] = (int)d.prods.size();
+            d.prods.push_back(p);
+        }
+    }
+    d.lcol.assign(P, -1);
     d.rcol.assign(P, -1);
     d.sym.assign(P, 0);
     std::vector<char> part_sym;
@@ -2401,37 +2410,24 @@ DensityLayout layout_densities(const std::vector<cl::PlanStep>& plan, int n_stat
             for (int p : q.lefts) d.sym[p] = 1;
     }
     const bool all_sym = std::find(part_sym.begin(), part_sym.end(), 0) == part_sym.end();
-    if (by_state) {
-        Part all;
-        for (int p = 0; p < P; ++p) {
-            if (is_left[p]) all.lefts.push_back(p);  // ascending products: ascending higher states
-            if (is_right[p]) all.rights.push_back(p);
-        }
-        found.assign(1, std::move(all));
-        part_sym.assign(1, all_sym);
-    }
+    std::vector<int> right_rows;
     for (size_t k = 0; k < found.size(); ++k) {
         const Part& q = found[k];
-        d.gram.blocks.push_back(clk::GramBlock{(int)d.prods.size(), (int)q.lefts.size(), (int)d.rights.size(),
+        d.gram.blocks.push_back(clk::GramBlock{(int)d.columns.size(), (int)q.lefts.size(), (int)right_rows.size(),
                                                (int)q.rights.size(), part_sym[k]});
         for (int p : q.lefts) {
-            d.slot[p] = (int)d.prods.size();
-            d.prods.push_back(p);
+            d.lcol[p] = (int)d.columns.size();
+            d.columns.push_back(row[p]);
         }
         for (int p : q.rights) {
-            d.rcol[p] = (int)d.rights.size();
-            d.rights.push_back(p);  // the product; its row below
+            d.rcol[p] = (int)right_rows.size();
+            right_rows.push_back(row[p]);
         }
     }
-    d.gram.nl = (int)d.prods.size();
-    d.gram.nr = (int)d.rights.size();
+    d.gram.nl = (int)d.columns.size();
+    d.gram.nr = (int)right_rows.size();
     d.gram.whole = clk::GramBlock{0, d.gram.nl, 0, d.gram.nr, all_sym};
-    for (int p : d.rights)
-        if (d.slot[p] < 0) {
-            d.slot[p] = (int)d.prods.size();
-            d.prods.push_back(p);
-        }
-    for (int& r : d.rights) r = d.slot[r];
+    d.columns.insert(d.columns.end(), right_rows.begin(), right_rows.end());
     return d;
 }
 
@@ -2461,7 +2457,7 @@ std::vector<StepValue> step_values(const std::vector<cl::PlanStep>& plan, const 
             const auto& st = plan[i];
             // a symmetric block holds the pairs with the larger product on the left
             const bool turned = d.sym[st.left.product] && st.left.product < st.right.product;
-            const int l = d.slot[turned ? st.right.product : st.left.product];
+            const int l = d.lcol[turned ? st.right.product : st.left.product];
             const int r = d.rcol[turned ? st.left.product : st.right.product];
             v[i] = StepValue{(uint64_t)l * d.gram.nr + r, turned, st.left.conjugate != st.right.conjugate,
                              st.left.conjugate != 0};
@@ -2518,14 +2514,14 @@ void compute_impl(cl_ctx* c, int64_t n_int, const int16_t* spec, double* out, in
         const auto plan = shard_steps(cl::orient_steps(c->n_states, specs), c->n_states, shard, n_shards);
         if (n_shards > 1) std::memset(out, 0, sizeof(double) * 2 * (size_t)n_int);
         if (plan.empty()) return;
-        const DensityLayout lay = layout_densities(plan, c->n_states, symmetric_blocks(c, round_mask), false);
-        const std::vector<int>& rights = lay.rights;
+        const DensityLayout lay = layout_densities(plan, c->n_states, symmetric_blocks(c, round_mask));
+        const std::vector<int>& columns = lay.columns;
         const std::vector<int2> fl = lay.states();
         const int nu = (int)lay.prods.size(), nl = lay.gram.nl, nr = lay.gram.nr;
         const long long As = c->n_sorted;
-        DevBuf<int>& dr = c->req_ridx;
-        grow(dr, rights.size());
-        CL_CUDA(cudaMemcpyAsync(dr.p, rights.data(), rights.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+        DevBuf<int>& dr = c->req_rows;
+        grow(dr, columns.size());
+        CL_CUDA(cudaMemcpyAsync(dr.p, columns.data(), columns.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
         DevBuf<cx<double>>& rho = c->req_rho;
         DevBuf<cx<double>>& V = c->req_V;
         grow(rho, (size_t)nu * As);
@@ -2623,9 +2619,8 @@ void compute_states_impl(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, 
             upload_through(n_states - 1);
         cudaGetLastError();  // pageable memory is not an error
     }
-    // left densities ordered by their higher state, then right-only densities
-    const DensityLayout lay = layout_densities(plan, n_states, symmetric_blocks(c), true);
-    const std::vector<int>& rights = lay.rights;
+    const DensityLayout lay = layout_densities(plan, n_states, symmetric_blocks(c));
+    const std::vector<int>& columns = lay.columns;
     const std::vector<int2> rows = lay.states();
     const int nu = (int)lay.prods.size(), nl = lay.gram.nl, nr = lay.gram.nr;
     // groups of left densities: cut at a state boundary once a group holds nl/6 densities
@@ -2655,9 +2650,9 @@ void compute_states_impl(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, 
     if (nu > nl) pair_setup(c, pairs_of(nl, nu), ps_right);
     const long long As = c->n_sorted;
     const bool v32 = v_fp32(c);
-    DevBuf<int>& dr = c->req_ridx;
-    grow(dr, rights.size());
-    CL_CUDA(cudaMemcpyAsync(dr.p, rights.data(), rights.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    DevBuf<int>& dr = c->req_rows;
+    grow(dr, columns.size());
+    CL_CUDA(cudaMemcpyAsync(dr.p, columns.data(), columns.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
     DevBuf<cx<double>>& rho = c->req_rho;
     DevBuf<cx<double>>& V = c->req_V;
     grow(rho, (size_t)nu * As);
@@ -2804,7 +2799,7 @@ struct cl_request {
     std::vector<StepValue> values;
     int nl = 0, nr = 0;
     PairSetup ps;
-    DevBuf<int> ridx;
+    DevBuf<int> rows;
     DevBuf<cx<double>> rho, V;
     DevBuf<double> o4;
     double* o4_host = nullptr;  // pinned
@@ -2849,7 +2844,7 @@ void request_enqueue(cl_request* r) {
     pair_launch(c, r->ps, r->rho.p);
     const bool v32 = v_fp32(c);
     run_transforms(c, r->rho.p, As, r->nl, r->V.p, As, v32);
-    gram(c, r->V.p, v32, As, r->rho.p, rho_bytes(c) == sizeof(cx<float>), As, r->ridx.p, r->lay.gram, As, r->o4.p);
+    gram(c, r->V.p, v32, As, r->rho.p, rho_bytes(c) == sizeof(cx<float>), As, r->rows.p, r->lay.gram, As, r->o4.p);
     CL_CUDA(cudaMemcpyAsync(r->o4_host, r->o4.p, sizeof(double) * (4 * (size_t)r->nl * r->nr + 1),
                             cudaMemcpyDeviceToHost, c->stream));
 }
@@ -2891,15 +2886,15 @@ int cl_request_create_shard(cl_ctx* c, int64_t n_int, const int16_t* spec, int s
             *out = r;
             return;
         }
-        r->lay = layout_densities(r->plan, c->n_states, symmetric_blocks(c), false);
+        r->lay = layout_densities(r->plan, c->n_states, symmetric_blocks(c));
         r->nl = r->lay.gram.nl;
         r->nr = r->lay.gram.nr;
         r->values = step_values(r->plan, r->lay);
-        const std::vector<int>& rights = r->lay.rights;
+        const std::vector<int>& columns = r->lay.columns;
         const std::vector<int2> fl = r->lay.states();
         const long long As = c->n_sorted;
         pair_setup(c, fl, r->ps);
-        r->ridx.upload(rights.data(), rights.size(), c->stream);
+        r->rows.upload(columns.data(), columns.size(), c->stream);
         r->rho.alloc(fl.size() * As);
         r->V.alloc((size_t)r->nl * As);
         r->o4.alloc((size_t)4 * r->nl * r->nr + 1);

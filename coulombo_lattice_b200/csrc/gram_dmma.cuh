@@ -46,7 +46,8 @@ constexpr int WIDTH = 64;      // densities a tile side, at most
 
 template <typename S>
 struct GramArgs {
-    const cx<S>* V;       // left densities: V[l * v_stride + atom]
+    const cx<S>* V;       // left densities: V[(lidx ? lidx[l] : l) * v_stride + atom]
+    const int* lidx;
     long long v_stride;
     const int* ridx;      // right densities: rho[(ridx ? ridx[r] : r) * r_stride + atom]
     int nl, nr;
@@ -112,7 +113,7 @@ template <typename SV, typename SR, int KC, int A, int B>
 __global__ void __launch_bounds__(THREADS, 1) k_gram_dmma(const cx<SR>* __restrict__ rho, const GramArgs<SV> g) {
     constexpr int PITCH = pitch(KC);
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int right_row[WIDTH];
+    __shared__ int left_row[WIDTH], right_row[WIDTH];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     GramTile tile;
     gram_tile(g.tiles, blockIdx.x, &tile);
@@ -125,12 +126,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_gram_dmma(const cx<SR>* __restri
     const size_t b_off = (size_t)PITCH * g.nd_a * sizeof(cx<SV>);
     for (int r = threadIdx.x; r < tile.nr; r += THREADS)
         right_row[r] = g.ridx ? g.ridx[tile.r0 + r] : tile.r0 + r;
+    for (int l = threadIdx.x; l < tile.nl; l += THREADS)
+        left_row[l] = g.lidx ? g.lidx[tile.l0 + l] : tile.l0 + l;
     __syncthreads();
     const auto issue = [&](int c) {
         unsigned char* st = smem_raw + (size_t)(c % g.stages) * stage;
         const long long k0 = k_begin + (long long)c * KC;
         copy_chunk<KC, SV>(reinterpret_cast<cx<SV>*>(st), tile.nl, nA4, k0, k_end, g.align_v, g.V,
-                       [&](int i) { return g.V + (long long)(tile.l0 + i) * g.v_stride; });
+                       [&](int i) { return g.V + (long long)left_row[i] * g.v_stride; });
         copy_chunk<KC, SR>(reinterpret_cast<cx<SR>*>(st + b_off), tile.nr, nB4, k0, k_end, g.align_r, rho,
                        [&](int i) { return rho + (long long)right_row[i] * g.r_stride; });
     };

@@ -423,7 +423,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 // ordering the raw ring needs.
 // ---------------------------------------------------------------------------------------
 struct FusedGram {
-    const float2* V;      // left densities: V[l * v_stride + atom]
+    const float2* V;      // left densities: V[(lidx ? lidx[l] : l) * v_stride + atom]
+    const int* lidx;
     long long v_stride;
     const float2* rho;    // right densities: rho[(ridx ? ridx[r] : r) * r_stride + atom]
     long long r_stride;
@@ -529,7 +530,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_gram_tc_fused(const FusedG
     }
     for (int i = threadIdx.x; i < nd; i += FUSED_THREADS) {
         if (i < nA) {
-            src_tab[i] = g.V + (long long)(la0 + i) * g.v_stride;
+            src_tab[i] = g.V + (long long)(g.lidx ? g.lidx[la0 + i] : la0 + i) * g.v_stride;
         } else {
             const int r = rb0 + (i - nA);
             src_tab[i] = g.rho + (long long)(g.ridx ? g.ridx[r] : r) * g.r_stride;
@@ -812,7 +813,7 @@ __global__ void __launch_bounds__(ws_threads(DRAINS), 1) k_gram_tc_ws(const Fuse
     constexpr int WS_THREADS = 32 * (WS_DRAIN_WARP0 + DRAINS);
     for (int i = threadIdx.x; i < nd; i += WS_THREADS) {
         if (i < nA) {
-            src_tab[i] = g.V + (long long)(la0 + i) * g.v_stride;
+            src_tab[i] = g.V + (long long)(g.lidx ? g.lidx[la0 + i] : la0 + i) * g.v_stride;
         } else {
             const int r = rb0 + (i - nA);
             src_tab[i] = g.rho + (long long)(g.ridx ? g.ridx[r] : r) * g.r_stride;

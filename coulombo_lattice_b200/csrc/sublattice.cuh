@@ -22,9 +22,11 @@
 // (S = 8, m = 4) one eighth -- and the padded halves of each axis are neither loaded nor stored.
 //
 // On the GPU the classes are stacked along z into a virtual grid (P, P, S*s): class b's plane cz
-// is virtual plane b*s + cz, and its atoms sit at x, y < s.  The forward and inverse x and y
-// passes of the 8-round forms run unchanged on that grid (rows without atoms are neither stored
-// nor read); k_zmix_rf below does the z transforms and the class mixing in one pass.
+// is virtual plane b*s + cz, and its atoms sit at x, y < s.  The quadrant plane passes (plane_w.cuh,
+// plane_xy.cuh) transform its planes; where none is built, the x and y passes of the 8-round forms
+// run on that grid (rows without atoms are neither stored nor read).  k_zw (zmix_wht.cuh) does the z
+// transforms and the class mixing in one pass, k_zmix_rf below for the class sets and lengths that
+// it is not built for.
 #pragma once
 
 #include "fft.cuh"

@@ -153,8 +153,9 @@ int cl_form_info(cl_ctx* ctx, int info[8]);
 /* Same as cl_compute for one shard of the request: the prepared (left) densities of the plan, in
  * ascending product order, are dealt round-robin to n_shards shards, and out[i] holds integral i
  * when its left density belongs to shard `shard`, zero otherwise.  The shards' outputs add up to
- * cl_compute's, so n_shards GPUs (one process each) run one shard each and combine them with one
- * all-reduce (sum) of out: the multi-GPU unit of both forms (the sub-lattice forms have no
+ * cl_compute's (in the FP32 forms with more than 64 densities to the rounding of the transforms),
+ * so n_shards GPUs (one process each) run one shard each and combine them with one all-reduce
+ * (sum) of out: the multi-GPU unit of both forms (the sub-lattice forms have no
  * rounds).  Right densities are formed on every shard.  No reference counterpart: the reference
  * splits each grid over MPI ranks and reduces every calculate() (CoulombCalculator.cpp:165-172). */
 int cl_compute_shard(cl_ctx* ctx, int64_t n_int, const int16_t* spec, int shard, int n_shards, double* out);

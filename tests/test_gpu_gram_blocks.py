@@ -110,3 +110,24 @@ def test_odd_atom_count_rows_off_16_bytes():
             cc.initialize(dielectric=10.89, onsite=2.0)
             cc.set_states(st, cells, HOLES)
             _close(cc.compute(specs), want, mode)
+
+
+@pytest.mark.parametrize("text", ["eeee,hhhh,ehhe,eheh", "eheh,1111", "****/29"])
+@pytest.mark.parametrize("mode", cl.ALL_MODES)
+def test_overlapped_upload_sums_alike(text, mode, monkeypatch):
+    """compute_states transforms its densities in other groups than a request but reduces them in the same
+    tiles: only the order of the FP64 additions of the atom splits differs (1e-12 of the largest value)."""
+    monkeypatch.setenv("CL_TC_MIN_ATOMS", "0")
+    dims, st, cells = _system((4, 5, 4))
+    specs = _specs(text)
+    with cl.CoulombCalculator(dims, STEP, mode) as cc:
+        cc.initialize(dielectric=10.89, onsite=2.0)
+        cc.set_states(st, cells, HOLES)
+        want = cc.compute(specs)
+        req = cc.request(specs)
+        got = req.run().copy()
+        req.close()
+        over = cc.compute_states(st, cells, HOLES, specs)
+    tol = 1e-12 * np.abs(want).max()
+    assert np.abs(got - want).max() <= tol
+    assert np.abs(over - want).max() <= tol
