@@ -733,15 +733,16 @@ def run_ours(args):
     M = int(np.prod(d["dims"]))
     plan_steps = cl.plan(n, specs)
     n_prepared = len({int(s[1]) for s in plan_steps})
-    n_right = len({int(s[3]) for s in plan_steps})
     n_cells = int(np.unique(d["cells_idx"]).size)
     gram_tc = None
     if "gram" in prof and n_cells >= 65536:
-        # split-precision Gram (fused, or after the split pass): 3 TF32 products of a
-        # (2 n_left) x (2 n_right) x atoms real GEMM; the TF32 tensor rate is half the measured
-        # BF16 rate
+        # split-precision Gram (fused, or after the split pass): 3 TF32 products of the 2 x 2 real sums
+        # over the atoms of every pair of densities that the steps name, once for both orders (the
+        # Gram is symmetric); the TF32 tensor rate is half the measured BF16 rate
         g_ms, g_launches, _ = prof["gram"]
-        flops = 3 * 2.0 * (2 * n_prepared) * (2 * n_right) * n_cells * args.steps
+        lr = np.asarray(plan_steps)[:, [1, 3]].astype(np.int64)
+        n_pairs = np.unique(lr.min(axis=1) << 32 | lr.max(axis=1)).size
+        flops = 3 * 2.0 * 4 * n_pairs * n_cells * args.steps
         tf32_peak = peak_tflops_bf16() / 2
         gram_tc = {"bound": "tensor", "kernel": "gram", "achieved": flops / (g_ms / 1e3) / 1e12,
                    "peak": tf32_peak, "unit": "TFLOP/s", "frac": flops / (g_ms / 1e3) / 1e12 / tf32_peak,
