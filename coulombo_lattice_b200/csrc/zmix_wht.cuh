@@ -345,7 +345,8 @@ template <typename T, int SET>
 struct ZwSet {
     static constexpr int S = SET == kZwZb ? 8 : 2;      // classes
     static constexpr int C = SET == kZwZb ? 3 : 1;      // quads of coefficients a (column, frequency)
-    // columns per block: 64 contiguous bytes a plane and class (zinc-blende), 128 (pair)
+    // columns per block: 64 contiguous bytes a plane and class (zinc-blende; with 32 bytes and twice the
+    // groups a block, 36 densities of 128-point lines take 2.03 ms instead of 1.86), 128 (pair)
     static constexpr int L = (SET == kZwZb ? 64 : 128) / (int)sizeof(cx<T>);
 };
 
