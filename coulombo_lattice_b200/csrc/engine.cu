@@ -52,6 +52,7 @@ template <typename T>
 struct DevBuf {
     T* p = nullptr;
     size_t n = 0;
+    unsigned moves = 0;  // how often the storage changed
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
@@ -64,6 +65,7 @@ struct DevBuf {
     void alloc(size_t count) {
         if (count == n && p) return;
         release();
+        ++moves;
         if (count == 0) return;
         CL_CUDA(cudaMalloc(&p, count * sizeof(T)));
         n = count;
@@ -290,6 +292,7 @@ struct cl_ctx {
     bool grid_prepared = false;
 
     // states
+    long long layout_version = 0;  // bumped when the atoms, the states' number or the orbitals change
     int n_states = 0, n_holes = 0, n_orb = 0;
     long long n_atoms = 0, n_sorted = 0;
     DevBuf<cx<double>> coeff;
@@ -312,6 +315,17 @@ struct cl_ctx {
     DevBuf<int> slot_of_atom;      // input atom -> sorted slot (the potentials' gather)
     DevBuf<double> pot;            // potentials in input atom order
     double timings[4] = {0, 0, 0, 0};
+
+    // Changes whenever a buffer that a request's launches name gets other storage.
+    unsigned long long buffer_moves() const {
+        unsigned long long m = khat64.moves + khat32.moves + coeff.moves + cell_sorted.moves + row_ptr.moves;
+        m += (unsigned long long)work.moves + rounds.moves + tc_buf.moves;
+        m += (unsigned long long)sl.H64.moves + sl.phxy64.moves + sl.phz64.moves + sl.H32.moves + sl.phxy32.moves +
+             sl.phz32.moves + sl.zw_tab.moves + sl.zw_col.moves + sl.zw_zph.moves;
+        for (const Axis* a : {ax, sl.ax})
+            for (int d = 0; d < 3; ++d) m += (unsigned long long)a[d].tw64.moves + a[d].tw32.moves + a[d].phase.moves;
+        return m;
+    }
 
     // per-kernel profiling (events recorded around launches on `stream`)
     struct ProfEntry {
@@ -2199,6 +2213,7 @@ void load_cells(cl_ctx* c, int64_t n_atoms, const int64_t* cells) {
         std::memcmp(c->cells_seen.data(), cells, sizeof(int64_t) * (size_t)n_atoms) == 0)
         return;
     c->cells_seen.clear();
+    ++c->layout_version;
     std::vector<int> order((size_t)n_atoms);
     std::iota(order.begin(), order.end(), 0);
     for (int64_t a = 0; a < n_atoms; ++a)
@@ -2279,9 +2294,16 @@ void upload_state_sorted(cl_ctx* c, int s, const double* coeff, cudaStream_t str
                                                     c->coeff.p + (size_t)s * per_s);
     CL_LAUNCHED();
 }
-void reserve_coeff(cl_ctx* c, int n_states) {
-    grow(c->coeff, (size_t)n_states * c->n_sorted * c->n_orb);
-    grow(c->coeff_stage, 2 * (size_t)c->n_atoms * c->n_orb);
+// Makes room for the states' coefficients on the loaded cells; no states are loaded when that fails.
+void reserve_states(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, int n_orb) {
+    if (n_states != c->n_states || n_orb != c->n_orb) ++c->layout_version;
+    c->n_states = 0;
+    c->n_atoms = n_atoms;
+    grow(c->coeff, (size_t)n_states * c->n_sorted * n_orb);
+    grow(c->coeff_stage, 2 * (size_t)n_atoms * n_orb);
+    c->n_states = n_states;
+    c->n_holes = n_holes;
+    c->n_orb = n_orb;
 }
 
 }  // namespace
@@ -2294,11 +2316,7 @@ int cl_set_states(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, int n_o
         check_ctx(c);
         check_states_args(n_states, n_holes, n_atoms, n_orb, coeff, cells);
         load_cells(c, n_atoms, cells);
-        c->n_states = n_states;
-        c->n_holes = n_holes;
-        c->n_orb = n_orb;
-        c->n_atoms = n_atoms;
-        reserve_coeff(c, n_states);
+        reserve_states(c, n_states, n_holes, n_atoms, n_orb);
         for (int s = 0; s < n_states; ++s) upload_state_sorted(c, s, coeff, c->stream);
         CL_CUDA(cudaStreamSynchronize(c->stream));
     });
@@ -2565,11 +2583,7 @@ void compute_states_impl(cl_ctx* c, int n_states, int n_holes, int64_t n_atoms, 
     check_states_args(n_states, n_holes, n_atoms, n_orb, coeff, cells);
     if (n_int < 0 || (n_int && (!spec || !out))) cl::fail(CL_ERR_ARGUMENT, "invalid integral list");
     load_cells(c, n_atoms, cells);
-    c->n_states = n_states;
-    c->n_holes = n_holes;
-    c->n_orb = n_orb;
-    c->n_atoms = n_atoms;
-    reserve_coeff(c, n_states);
+    reserve_states(c, n_states, n_holes, n_atoms, n_orb);
     std::memset(c->timings, 0, sizeof c->timings);
     if (!c->copy_stream) CL_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
     while ((int)c->state_ev.size() < n_states) {
@@ -2791,6 +2805,16 @@ int cl_potentials(cl_ctx* c, double* out) {
 // ---------------------------------------------------------------------------------------
 // Prepared requests and graph-captured batches
 // ---------------------------------------------------------------------------------------
+// What a request's launches depend on besides its own lists: a graph names the buffers, sizes and tables of its
+// capture, and an eager run has sized them.
+struct LaunchState {
+    long long layout_version = -1, kernel_version = -1;
+    unsigned long long moves = 0;
+    bool operator==(const LaunchState& o) const {
+        return layout_version == o.layout_version && kernel_version == o.kernel_version && moves == o.moves;
+    }
+};
+
 struct cl_request {
     cl_ctx* ctx = nullptr;
     int64_t n_int = 0;
@@ -2803,8 +2827,10 @@ struct cl_request {
     DevBuf<cx<double>> rho, V;
     DevBuf<double> o4;
     double* o4_host = nullptr;  // pinned
-    bool warm = false;
+    LaunchState warm;  // at the last eager run
     int n_shards = 1;  // out entries of other shards' steps are zero
+    int top_state = 0;              // the highest state that the request names, from 1
+    long long layout_version = -1;  // the context's, at the last request_layout
     ~cl_request() {
         if (o4_host) cudaFreeHost(o4_host);
     }
@@ -2812,6 +2838,7 @@ struct cl_request {
 
 struct cl_batch {
     std::vector<cl_request*> reqs;
+    std::vector<LaunchState> captured;  // per request
     cudaStream_t master = nullptr;
     cudaEvent_t fork = nullptr, t0 = nullptr, t1 = nullptr;
     std::vector<cudaEvent_t> joins;
@@ -2821,10 +2848,16 @@ struct cl_batch {
     // per-launch event pairs captured into the graph for requests whose context profiles
     std::vector<std::vector<cl_ctx::ProfEntry>> prof;
     std::vector<cudaEvent_t> prof_events;
-    ~cl_batch() {
+    void drop_graph() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
+        exec = nullptr;
+        graph = nullptr;
         for (auto e : prof_events) cudaEventDestroy(e);
+        prof_events.clear();
+    }
+    ~cl_batch() {
+        drop_graph();
         for (auto e : joins) cudaEventDestroy(e);
         if (fork) cudaEventDestroy(fork);
         if (t0) cudaEventDestroy(t0);
@@ -2834,6 +2867,30 @@ struct cl_batch {
 };
 
 namespace {
+
+// Lists, launch shapes and buffers of a request for the states that its context holds now: made when the
+// request is created, and again when cl_set_states or cl_compute_states has loaded other atoms, another number of
+// states or of orbitals since (the stored shapes would read and write past the new buffers).
+void request_layout(cl_request* r) {
+    cl_ctx* c = r->ctx;
+    if (r->nl == 0 || r->layout_version == c->layout_version) return;
+    if (c->n_states < r->top_state)
+        cl::fail(CL_ERR_STATE, "the request names state %d of %d loaded", r->top_state, c->n_states);
+    const std::vector<int2> fl = r->lay.states();
+    const long long As = c->n_sorted;
+    r->ps.mma_ok = r->ps.tile_ok = false;
+    pair_setup(c, fl, r->ps);
+    grow(r->rho, fl.size() * As);
+    grow(r->V, (size_t)r->nl * As);
+    tc_reserve(c, r->lay.gram, As, v_fp32(c), rho_bytes(c) == sizeof(cx<float>));
+    CL_CUDA(cudaStreamSynchronize(c->stream));
+    r->layout_version = c->layout_version;
+}
+
+LaunchState launch_state(const cl_request* r) {
+    const cl_ctx* c = r->ctx;
+    return {c->layout_version, c->kernel_version, c->buffer_moves() + r->rho.moves + r->V.moves};
+}
 
 // Stream-ordered work of a prepared request: no allocation, no host synchronisation, no
 // pageable copies -- it can be captured.
@@ -2890,17 +2947,12 @@ int cl_request_create_shard(cl_ctx* c, int64_t n_int, const int16_t* spec, int s
         r->nl = r->lay.gram.nl;
         r->nr = r->lay.gram.nr;
         r->values = step_values(r->plan, r->lay);
+        for (const int2& p : r->lay.states()) r->top_state = std::max({r->top_state, p.x + 1, p.y + 1});
         const std::vector<int>& columns = r->lay.columns;
-        const std::vector<int2> fl = r->lay.states();
-        const long long As = c->n_sorted;
-        pair_setup(c, fl, r->ps);
         r->rows.upload(columns.data(), columns.size(), c->stream);
-        r->rho.alloc(fl.size() * As);
-        r->V.alloc((size_t)r->nl * As);
         r->o4.alloc((size_t)4 * r->nl * r->nr + 1);
         CL_CUDA(cudaMallocHost(&r->o4_host, sizeof(double) * (4 * (size_t)r->nl * r->nr + 1)));
-        tc_reserve(c, r->lay.gram, As, v_fp32(c), rho_bytes(c) == sizeof(cx<float>));
-        CL_CUDA(cudaStreamSynchronize(c->stream));
+        request_layout(r);
         *out = r;
     });
     if (st != CL_OK) delete r;
@@ -2917,10 +2969,11 @@ int cl_request_run(cl_request* r, double* out) {
     return cl::guarded([&] {
         if (!r || !out) cl::fail(CL_ERR_ARGUMENT, "null argument");
         check_ctx(r->ctx);
+        request_layout(r);
         request_enqueue(r);
         CL_CUDA(cudaStreamSynchronize(r->ctx->stream));
         prof_collect(r->ctx);
-        r->warm = true;
+        r->warm = launch_state(r);
         request_finish(r, out);
     });
 }
@@ -2963,15 +3016,22 @@ int cl_batch_run(cl_batch* b, double** outs) {
     return cl::guarded([&] {
         if (!b || !outs) cl::fail(CL_ERR_ARGUMENT, "null argument");
         CL_CUDA(cudaSetDevice(b->reqs[0]->ctx->device));
-        if (!b->exec) {
+        for (cl_request* r : b->reqs) request_layout(r);
+        // captured anew when a later call of one of the contexts has moved a buffer, loaded another layout or
+        // set another kernel
+        bool current = b->exec != nullptr;
+        for (size_t i = 0; current && i < b->reqs.size(); ++i) current = b->captured[i] == launch_state(b->reqs[i]);
+        if (!current) {
+            b->drop_graph();
+            b->captured.clear();
             // one eager run of every request sizes every buffer and sets every kernel
             // attribute; then the whole batch is captured once as parallel branches
             for (cl_request* r : b->reqs)
-                if (!r->warm) {
+                if (!(r->warm == launch_state(r))) {
                     request_enqueue(r);
                     CL_CUDA(cudaStreamSynchronize(r->ctx->stream));
                     prof_collect(r->ctx);
-                    r->warm = true;
+                    r->warm = launch_state(r);
                 }
             // contexts that profile record their launch events inside the graph
             b->prof.assign(b->reqs.size(), {});
@@ -2997,6 +3057,7 @@ int cl_batch_run(cl_batch* b, double** outs) {
                 r->ctx->prof_owned = nullptr;
             }
             CL_CUDA(cudaGraphInstantiate(&b->exec, b->graph, 0));
+            for (const cl_request* r : b->reqs) b->captured.push_back(launch_state(r));
         }
         CL_CUDA(cudaEventRecord(b->t0, b->master));
         CL_CUDA(cudaGraphLaunch(b->exec, b->master));

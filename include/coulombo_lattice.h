@@ -202,7 +202,9 @@ typedef struct cl_batch cl_batch;
 /* A request prepared once: the plan of n_int integrals (as for cl_compute), its device
  * buffers and its pinned result buffer.  Running it only enqueues kernels and copies, which
  * is what lets batches be captured in a CUDA graph.  Replaces, for repeated requests over the
- * same states, the per-call planning of coulombo.cpp:121-151. */
+ * same states, the per-call planning of coulombo.cpp:121-151.  A request follows its context: after
+ * cl_set_states or cl_compute_states with other atoms, states or orbitals its next run lays its buffers
+ * out again, and fails with CL_ERR_STATE when it names a state that is no longer loaded. */
 int cl_request_create(cl_ctx* ctx, int64_t n_int, const int16_t* spec, cl_request** out);
 /* A prepared request of one shard (see cl_compute_shard): runs write zeros for the other shards'
  * integrals; cl_request_create is shard 0 of 1. */
@@ -214,7 +216,8 @@ void cl_request_destroy(cl_request* req);
 /* A batch of requests on distinct contexts of one GPU (e.g. nanostructures of uneven grid
  * sizes).  The first cl_batch_run runs each request once, then captures all of them as
  * parallel branches of one CUDA graph (each on its own context's stream); every run launches
- * that graph once.  outs[i] receives request i's values.  No reference counterpart (the
+ * that graph once, captured again when a call in between has given one of the contexts another
+ * layout, kernel or buffer.  outs[i] receives request i's values.  No reference counterpart (the
  * reference runs one structure per process). */
 int cl_batch_create(cl_request** reqs, int n, cl_batch** out);
 int cl_batch_run(cl_batch* batch, double** outs);
