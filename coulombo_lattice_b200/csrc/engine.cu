@@ -2817,6 +2817,7 @@ struct LaunchState {
 
 struct cl_request {
     cl_ctx* ctx = nullptr;
+    int device = 0;  // the context's: a request may be destroyed after its context
     int64_t n_int = 0;
     std::vector<cl::PlanStep> plan;
     DensityLayout lay;
@@ -2837,6 +2838,7 @@ struct cl_request {
 };
 
 struct cl_batch {
+    int device = 0;
     std::vector<cl_request*> reqs;
     std::vector<LaunchState> captured;  // per request
     cudaStream_t master = nullptr;
@@ -2933,6 +2935,7 @@ int cl_request_create_shard(cl_ctx* c, int64_t n_int, const int16_t* spec, int s
         if (n_int <= 0 || !spec) cl::fail(CL_ERR_ARGUMENT, "invalid integral list");
         r = new cl_request();
         r->ctx = c;
+        r->device = c->device;
         r->n_int = n_int;
         std::vector<std::array<int16_t, 4>> specs((size_t)n_int);
         for (int64_t i = 0; i < n_int; ++i)
@@ -2961,7 +2964,7 @@ int cl_request_create_shard(cl_ctx* c, int64_t n_int, const int16_t* spec, int s
 
 void cl_request_destroy(cl_request* r) {
     if (!r) return;
-    cudaSetDevice(r->ctx->device);
+    cudaSetDevice(r->device);
     delete r;
 }
 
@@ -2993,6 +2996,7 @@ int cl_batch_create(cl_request** reqs, int n, cl_batch** out) {
         }
         CL_CUDA(cudaSetDevice(dev));
         b = new cl_batch();
+        b->device = dev;
         b->reqs.assign(reqs, reqs + n);
         CL_CUDA(cudaStreamCreateWithFlags(&b->master, cudaStreamNonBlocking));
         CL_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
@@ -3008,14 +3012,14 @@ int cl_batch_create(cl_request** reqs, int n, cl_batch** out) {
 
 void cl_batch_destroy(cl_batch* b) {
     if (!b) return;
-    if (!b->reqs.empty()) cudaSetDevice(b->reqs[0]->ctx->device);
+    cudaSetDevice(b->device);
     delete b;
 }
 
 int cl_batch_run(cl_batch* b, double** outs) {
     return cl::guarded([&] {
         if (!b || !outs) cl::fail(CL_ERR_ARGUMENT, "null argument");
-        CL_CUDA(cudaSetDevice(b->reqs[0]->ctx->device));
+        CL_CUDA(cudaSetDevice(b->device));
         for (cl_request* r : b->reqs) request_layout(r);
         // captured anew when a later call of one of the contexts has moved a buffer, loaded another layout or
         // set another kernel

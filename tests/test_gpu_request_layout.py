@@ -130,3 +130,18 @@ def test_states_no_longer_loaded(mode):
         _close(batch.run()[0], want)
         batch.close()
         req.close()
+
+
+def test_destroyed_after_their_context():
+    first = _contents("first")
+    for _ in range(4):
+        cc = cl.CoulombCalculator(DIMS, STEP, cl.MODE_FP32_SUBLATTICE)
+        cc.initialize(dielectric=10.0)
+        cc.set_states(*first, 0)
+        req = cc.request(SPECS)
+        batch = cl.Batch([req])
+        want = batch.run()[0]
+        cc.close()
+        req.close()
+        batch.close()
+        _close(_fresh(cl.MODE_FP32_SUBLATTICE, first, SPECS), want)
