@@ -59,6 +59,10 @@ __device__ __forceinline__ cx<T> mul_is(cx<T> a) {
 #define CLK_S2_5 0.58778525229247312916870595463907276860       // sin(4 pi/5)
 
 // R-point DFTs in registers: v[k] <- sum_j v[j] exp(S * 2 pi i j k / R).
+//
+// FINE: an FP32 constant is off by up to 3e-8, the same in every line, so it does not average out over a
+// smooth density as the rounding of the data does.  sin 60 and sin 72, whose errors weigh most, are then
+// multiplied as x + (c - 1) x, which costs a DFT of 5 nothing and one of 3 two operations of 12.
 template <int S, typename T>
 __device__ __forceinline__ void dft2(cx<T>* v) {
     cx<T> a = v[0], b = v[1];
@@ -66,12 +70,13 @@ __device__ __forceinline__ void dft2(cx<T>* v) {
     v[1] = a - b;
 }
 
-template <int S, typename T>
+template <int S, bool FINE = false, typename T>
 __device__ __forceinline__ void dft3(cx<T>* v) {
     const T h = T(0.5), s60 = T(CLK_SIN60);
     cx<T> t1 = v[1] + v[2];
     cx<T> t2 = v[0] - scale(t1, h);
-    cx<T> t3 = mul_is<S>(scale(v[1] - v[2], s60));
+    const cx<T> d = v[1] - v[2];
+    cx<T> t3 = mul_is<S>(FINE && sizeof(T) == 4 ? d + scale(d, T(CLK_SIN60 - 1.0)) : scale(d, s60));
     v[0] = v[0] + t1;
     v[1] = t2 + t3;
     v[2] = t2 - t3;
@@ -87,7 +92,7 @@ __device__ __forceinline__ void dft4(cx<T>* v) {
     v[3] = b - d;
 }
 
-template <int S, typename T>
+template <int S, bool FINE = false, typename T>
 __device__ __forceinline__ void dft5(cx<T>* v) {
     const T c1 = T(CLK_C1_5), c2 = T(CLK_C2_5), s1 = T(CLK_S1_5), s2 = T(CLK_S2_5);
     cx<T> a1 = v[1] + v[4], a2 = v[2] + v[3];
@@ -95,8 +100,10 @@ __device__ __forceinline__ void dft5(cx<T>* v) {
     cx<T> x0 = v[0];
     cx<T> p1 = x0 + scale(a1, c1) + scale(a2, c2);
     cx<T> p2 = x0 + scale(a1, c2) + scale(a2, c1);
-    cx<T> q1 = mul_is<S>(scale(b1, s1) + scale(b2, s2));
-    cx<T> q2 = mul_is<S>(scale(b1, s2) - scale(b2, s1));
+    constexpr bool fine = FINE && sizeof(T) == 4;
+    const T s1m = T(CLK_S1_5 - 1.0);
+    cx<T> q1 = mul_is<S>((fine ? b1 + scale(b1, s1m) : scale(b1, s1)) + scale(b2, s2));
+    cx<T> q2 = mul_is<S>(scale(b1, s2) - (fine ? b2 + scale(b2, s1m) : scale(b2, s1)));
     v[0] = x0 + a1 + a2;
     v[1] = p1 + q1;
     v[4] = p1 - q1;
@@ -377,12 +384,12 @@ template <> struct WConst<15> {
         return 0.0;
     }
 };
-template <int R, int S, typename T>
+template <int R, int S, bool FINE = false, typename T>
 __device__ __forceinline__ void dft(cx<T>* v);
 
 // Composite N = N1*N2 codelet in registers (decimation in time):
 //   X[k1 + N1 k2] = sum_t W_N2^(t k2) [ W_N^(t k1) sum_j1 x[t + N2 j1] W_N1^(j1 k1) ].
-template <int N1, int N2, int S, typename T>
+template <int N1, int N2, int S, bool FINE = false, typename T>
 __device__ __forceinline__ void dft_2f(cx<T>* v) {
     constexpr int N = N1 * N2;
     cx<T> y[N];
@@ -391,7 +398,7 @@ __device__ __forceinline__ void dft_2f(cx<T>* v) {
         cx<T> u[N1];
 #pragma unroll
         for (int j = 0; j < N1; ++j) u[j] = v[t + N2 * j];
-        dft<N1, S>(u);
+        dft<N1, S, FINE>(u);
 #pragma unroll
         for (int k = 0; k < N1; ++k) {
             const int m = (t * k) % N;
@@ -408,25 +415,58 @@ __device__ __forceinline__ void dft_2f(cx<T>* v) {
         cx<T> w2[N2];
 #pragma unroll
         for (int t = 0; t < N2; ++t) w2[t] = y[k * N2 + t];
-        dft<N2, S>(w2);
+        dft<N2, S, FINE>(w2);
 #pragma unroll
         for (int q = 0; q < N2; ++q) v[k + N1 * q] = w2[q];
     }
 }
 
-template <int R, int S, typename T>
+// The multiple of m below m n that is 1 modulo n.
+__host__ __device__ constexpr int unit_multiple(int m, int n) {
+    int e = m;
+    while (e % n != 1) e += m;
+    return e;
+}
+// Coprime N1, N2 without twiddles (Good 1958, Thomas 1963): inputs N2 n1 + N1 n2, outputs E1 k1 + E2 k2 modulo N,
+// E1 = 1 modulo N1 and 0 modulo N2, E2 the other way round.
+template <int N1, int N2, int S, bool FINE = false, typename T>
+__device__ __forceinline__ void dft_coprime(cx<T>* v) {
+    constexpr int N = N1 * N2, E1 = unit_multiple(N2, N1), E2 = unit_multiple(N1, N2);
+    cx<T> y[N];
+#pragma unroll
+    for (int n2 = 0; n2 < N2; ++n2) {
+        cx<T> u[N1];
+#pragma unroll
+        for (int n1 = 0; n1 < N1; ++n1) u[n1] = v[(N2 * n1 + N1 * n2) % N];
+        dft<N1, S, FINE>(u);
+#pragma unroll
+        for (int k1 = 0; k1 < N1; ++k1) y[k1 * N2 + n2] = u[k1];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) {
+        dft<N2, S, FINE>(y + k1 * N2);
+#pragma unroll
+        for (int k2 = 0; k2 < N2; ++k2) v[(E1 * k1 + E2 * k2) % N] = y[k1 * N2 + k2];
+    }
+}
+
+template <int R, int S, bool FINE, typename T>
 __device__ __forceinline__ void dft(cx<T>* v) {
     if constexpr (R == 1) return;  // a one-point DFT is the identity
     else if constexpr (R == 2) dft2<S>(v);
-    else if constexpr (R == 3) dft3<S>(v);
+    else if constexpr (R == 3) dft3<S, FINE>(v);
     else if constexpr (R == 4) dft4<S>(v);
-    else if constexpr (R == 5) dft5<S>(v);
-    else if constexpr (R == 6) dft_2f<2, 3, S>(v);
-    else if constexpr (R == 9) dft_2f<3, 3, S>(v);
-    else if constexpr (R == 15) dft_2f<3, 5, S>(v);
-    else if constexpr (R == 10) dft_2f<2, 5, S>(v);
-    else if constexpr (R == 12) dft_2f<4, 3, S>(v);
-    else if constexpr (R == 16) dft_2f<4, 4, S>(v);
+    else if constexpr (R == 5) dft5<S, FINE>(v);
+    else if constexpr (FINE && R == 6) dft_coprime<2, 3, S, FINE>(v);
+    else if constexpr (FINE && R == 10) dft_coprime<2, 5, S, FINE>(v);
+    else if constexpr (FINE && R == 12) dft_coprime<4, 3, S, FINE>(v);
+    else if constexpr (FINE && R == 15) dft_coprime<3, 5, S, FINE>(v);
+    else if constexpr (R == 6) dft_2f<2, 3, S, FINE>(v);
+    else if constexpr (R == 9) dft_2f<3, 3, S, FINE>(v);
+    else if constexpr (R == 15) dft_2f<3, 5, S, FINE>(v);
+    else if constexpr (R == 10) dft_2f<2, 5, S, FINE>(v);
+    else if constexpr (R == 12) dft_2f<4, 3, S, FINE>(v);
+    else if constexpr (R == 16) dft_2f<4, 4, S, FINE>(v);
     else dft8<S>(v);
 }
 

@@ -21,7 +21,7 @@
 // against the passes these replace (a whole plane in shared memory, one block an SM, and a quadrant forward
 // pass, at 128 points; separate x and y passes at lengths without a plane pass): 36 densities of 128 x 128
 // planes, 2.1M atoms, 0.889 -> 0.570 ms forward (5.3 TB/s) and 0.898 -> 0.746 inverse (4.1); 820 of 64 x
-// 64, 1.94 -> 1.35 (6.4 TB/s) and 1.89 -> 1.55; 78 of 48 x 48, 0.159 -> 0.085 and 0.165 -> 0.084.
+// 64, 1.94 -> 1.35 (6.4 TB/s) and 1.89 -> 1.57; 78 of 48 x 48, 0.159 -> 0.086 and 0.165 -> 0.087.
 // In FP64: 78 densities of 48 x 48, 0.280 -> 0.138 ms and 0.281 -> 0.140; 36 of 128 x 128 (64 x 64 x 16
 // cells), both ways, 1.08 -> 0.83.
 #pragma once
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(PlaneW<T, H, R2, true>::THREADS, PlaneW<T, H, 
             cx<T> u[R2];
 #pragma unroll
             for (int t = 0; t < R2; ++t) u[t] = t == 0 ? c[0] : cmul(c[t * PQ], tw[t * R1 + q]);
-            dft<R2, -1>(u);
+            dft<R2, -1, true>(u);
 #pragma unroll
             for (int s = 0; s < R2; ++s) c[s * PQ] = u[s];
         }
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(PlaneW<T, H, R2, true>::THREADS, PlaneW<T, H, 
                 cx<T> u[R2];
 #pragma unroll
                 for (int t = 0; t < R2; ++t) u[t] = t == 0 ? d[0] : cmul(d[t * TP], tw[t * R1 + q]);
-                dft<R2, -1>(u);
+                dft<R2, -1, true>(u);
                 cx<T>* orow = o + (r / R2 + R1 * (r % R2)) * N + q;
 #pragma unroll
                 for (int s = 0; s < R2; ++s) orow[R1 * s] = u[s];
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(PlaneW<T, H, R2, false>::THREADS, PlaneW<T, H,
             for (int a = 0; a < IX; ++a) {
                 const int e = tid + a * THREADS, q = e % R1, rr = e / R1;
                 if (rr < rows) {
-                    dft<R2, +1>(v[a]);
+                    dft<R2, +1, true>(v[a]);
                     cx<T>* d = S + rr * SP + q;
 #pragma unroll
                     for (int t = 0; t < R2; ++t) d[t * TP] = t == 0 ? v[a][0] : cmulc(v[a][t], tw[t * R1 + q]);
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(PlaneW<T, H, R2, false>::THREADS, PlaneW<T, H,
             cx<T> u[R2];
 #pragma unroll
             for (int s = 0; s < R2; ++s) u[s] = c[(R1 * s) * PQ];
-            dft<R2, +1>(u);
+            dft<R2, +1, true>(u);
 #pragma unroll
             for (int t = 0; t < R2; ++t) c[(R1 * t) * PQ] = t == 0 ? u[0] : cmulc(u[t], tw[t * R1 + q]);
         }

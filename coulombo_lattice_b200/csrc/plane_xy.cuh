@@ -57,7 +57,7 @@ __device__ __noinline__ void y_forward(cx<T>* I, int pitch, int Q, const cx<T>* 
         cx<T> u[R2];
 #pragma unroll
         for (int t = 0; t < R2; ++t) u[t] = t == 0 ? c[0] : cmul(c[t * pitch], tw[t * R1 + i.k]);
-        dft<R2, -1>(u);
+        dft<R2, -1, true>(u);
 #pragma unroll
         for (int s = 0; s < R2; ++s) c[s * pitch] = u[s];
     }
@@ -77,7 +77,7 @@ __device__ __noinline__ void y_inverse(cx<T>* I, int pitch, int Q, const cx<T>* 
         cx<T> u[R2];
 #pragma unroll
         for (int s = 0; s < R2; ++s) u[s] = c[s * step];
-        dft<R2, +1>(u);
+        dft<R2, +1, true>(u);
 #pragma unroll
         for (int t = 0; t < R2; ++t) c[t * step] = t == 0 ? u[0] : cmulc(u[t], tw[t * R1 + i.k]);
     }
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(PlaneXY<T, H, R2, true>::THREADS, PlaneXY<T, H
                 cx<T> u[R2];
 #pragma unroll
                 for (int t = 0; t < R2; ++t) u[t] = t == 0 ? d[0] : cmul(d[t * TP], tw[t * R1 + q]);
-                dft<R2, -1>(u);
+                dft<R2, -1, true>(u);
                 cx<T>* orow = o + (r / ry2 + ry1 * (r % ry2)) * N + q;
 #pragma unroll
                 for (int s = 0; s < R2; ++s) orow[R1 * s] = u[s];
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(PlaneXY<T, H, R2, false>::THREADS, PlaneXY<T, 
             for (int a = 0; a < IX; ++a) {
                 const int e = tid + a * THREADS, q = e % R1, rr = e / R1;
                 if (rr < rows) {
-                    dft<R2, +1>(v[a]);
+                    dft<R2, +1, true>(v[a]);
                     cx<T>* d = S + rr * SP + q;
 #pragma unroll
                     for (int t = 0; t < R2; ++t) d[t * TP] = t == 0 ? v[a][0] : cmulc(v[a][t], tw[t * R1 + q]);

@@ -33,10 +33,16 @@
 //
 // Bound: instruction issue (78 warp instructions a class point, 60 of them FP32, against 94 for
 // k_zmix_rf) at the 16 warps an SM that 128 registers allow.  Measured on a B200, k_zmix_rf -> this
-// pass: 128-point lines of the 2,097,152-atom box, 36 densities, 2.47 -> 1.86 ms (2.66 TB/s); 64-point
-// lines, 820 densities, 6.93 -> 4.31 ms; 48-point, 78 densities, 0.309 -> 0.212 ms; two classes,
-// 54 x 72 x 80 grid, 36 densities, 0.587 -> 0.071 ms (k_zmix_rf keeps 8 classes' threads whatever the
-// set).  Without the staging: 1.88, 5.24 and 0.228 ms on the three zinc-blende shapes.
+// pass: 128-point lines of the 2,097,152-atom box, 36 densities, 2.47 -> 1.83 ms (2.70 TB/s); 64-point
+// lines, 820 densities, 6.93 -> 4.39 ms; 48-point, 78 densities, 0.309 -> 0.217 ms; two classes,
+// 54 x 72 x 80 grid, 36 densities, 0.587 -> 0.070 ms (k_zmix_rf keeps 8 classes' threads whatever the
+// set).  Without the staging (and with plain constants) 1.88, 5.24 and 0.228 ms on the three zinc-blende shapes.
+//
+// Error.  The rounding of an FP32 constant is the same in every line, so on smooth densities it adds up
+// over the lines and axes: with every constant rounded as it is, integrals of Gaussians over 32 boxes of 12-
+// to 128-point axes were off by 5.1e-8 (geometric mean of the root-mean-square error against FP64; k_zmix_rf and
+// the whole-plane passes 3.7e-8).  Odd H without twiddles, coprime codelets without twiddles, and the constants of
+// turn, dft3 and dft5 as +-1 plus a small part bring it to 2.3e-8, for 0.97 to 1.03 of the pass's time.
 // In FP64 (4 columns a block, 256 threads an SM at 255 registers): 48-point lines, 78 densities, 0.571 ->
 // 0.362 ms; 64-point, 36 densities, 0.679 -> 0.399; 54 x 72 x 80, two classes, 0.750 -> 0.111.
 #pragma once
@@ -63,36 +69,6 @@ template <> struct WConst<8> {
             case 1: return 0.7071067811865475244008443621048490392848;
             case 2: return 1.0000000000000000000000000000000000000000;
             case 3: return 0.7071067811865475244008443621048490392848;
-        }
-        return 0.0;
-    }
-};
-template <> struct WConst<18> {
-    static __device__ __forceinline__ double c(int m) {
-        switch (m) {
-            case 0: return 1.0000000000000000000000000000000000000000;
-            case 1: return 0.9396926207859083840541092773247314699362;
-            case 2: return 0.7660444431189780352023926505554166739358;
-            case 3: return 0.5000000000000000000000000000000000000000;
-            case 4: return 0.1736481776669303488517166267693147960004;
-            case 5: return -0.1736481776669303488517166267693147960004;
-            case 6: return -0.5000000000000000000000000000000000000000;
-            case 7: return -0.7660444431189780352023926505554166739358;
-            case 8: return -0.9396926207859083840541092773247314699362;
-        }
-        return 0.0;
-    }
-    static __device__ __forceinline__ double s(int m) {
-        switch (m) {
-            case 0: return 0.0000000000000000000000000000000000000000;
-            case 1: return 0.3420201433256687330440996146822595807631;
-            case 2: return 0.6427876096865393263226434099072634329076;
-            case 3: return 0.8660254037844386467637231707529361834714;
-            case 4: return 0.9848077530122080593667430245895230136706;
-            case 5: return 0.9848077530122080593667430245895230136706;
-            case 6: return 0.8660254037844386467637231707529361834714;
-            case 7: return 0.6427876096865393263226434099072634329076;
-            case 8: return 0.3420201433256687330440996146822595807631;
         }
         return 0.0;
     }
@@ -161,48 +137,6 @@ template <> struct WConst<24> {
             case 9: return 0.7071067811865475244008443621048490392848;
             case 10: return 0.5000000000000000000000000000000000000000;
             case 11: return 0.2588190451025207623488988376240483283491;
-        }
-        return 0.0;
-    }
-};
-template <> struct WConst<30> {
-    static __device__ __forceinline__ double c(int m) {
-        switch (m) {
-            case 0: return 1.0000000000000000000000000000000000000000;
-            case 1: return 0.9781476007338056379285667478695995324597;
-            case 2: return 0.9135454576426008955021275719853171779408;
-            case 3: return 0.8090169943749474241022934171828190588602;
-            case 4: return 0.6691306063588582138262733306867804735996;
-            case 5: return 0.5000000000000000000000000000000000000000;
-            case 6: return 0.3090169943749474241022934171828190588602;
-            case 7: return 0.1045284632676534713998341548024981190807;
-            case 8: return -0.1045284632676534713998341548024981190807;
-            case 9: return -0.3090169943749474241022934171828190588602;
-            case 10: return -0.5000000000000000000000000000000000000000;
-            case 11: return -0.6691306063588582138262733306867804735996;
-            case 12: return -0.8090169943749474241022934171828190588602;
-            case 13: return -0.9135454576426008955021275719853171779408;
-            case 14: return -0.9781476007338056379285667478695995324597;
-        }
-        return 0.0;
-    }
-    static __device__ __forceinline__ double s(int m) {
-        switch (m) {
-            case 0: return 0.0000000000000000000000000000000000000000;
-            case 1: return 0.2079116908177593371017422844051251662166;
-            case 2: return 0.4067366430758002077539859903414976129231;
-            case 3: return 0.5877852522924731291687059546390727685977;
-            case 4: return 0.7431448254773942350146970489742569771891;
-            case 5: return 0.8660254037844386467637231707529361834714;
-            case 6: return 0.9510565162951535721164393333793821434057;
-            case 7: return 0.9945218953682733369226919449805703815208;
-            case 8: return 0.9945218953682733369226919449805703815208;
-            case 9: return 0.9510565162951535721164393333793821434057;
-            case 10: return 0.8660254037844386467637231707529361834714;
-            case 11: return 0.7431448254773942350146970489742569771891;
-            case 12: return 0.5877852522924731291687059546390727685977;
-            case 13: return 0.4067366430758002077539859903414976129231;
-            case 14: return 0.2079116908177593371017422844051251662166;
         }
         return 0.0;
     }
@@ -303,34 +237,80 @@ template <> struct WConst<36> {
 template <int R, int S, typename T>
 __device__ __forceinline__ void dft_h(cx<T>* v) {
     if constexpr (R == 18)
-        dft_2f<2, 9, S>(v);
+        dft_coprime<2, 9, S, true>(v);
     else
-        dft<R, S>(v);
+        dft<R, S, true>(v);
 }
 
-// 2H-point DFT of x[0..H) followed by H zeros: X[2k] = DFT_H(x)[k], X[2k+1] = DFT_H(x w_2H^j)[k].
+// e + x (c + i S s), c and s compile-time constants of a unit root; ADD false: without e.  In FP32 the larger of
+// the two is multiplied as +-x + (c -+ 1) x, whose constant is rounded to a fraction of c's error, and
+// sqrt(1/2) as 3/4 x - 0.0429 x (see FINE in fft.cuh).
+template <int S, bool ADD, typename T>
+__device__ __forceinline__ cx<T> turn(cx<T> e, cx<T> x, double c, double s) {
+    const T zero = T(0);
+    if (!ADD) e = mk(zero, zero);
+    if (c == 0.0) return ADD ? e + mul_is<S>(x) : mul_is<S>(x);  // s = 1
+    if (sizeof(T) == 8) {
+        const cx<T> w = mk(T(c), T(S * s));
+        return ADD ? mk(e.re + w.re * x.re - w.im * x.im, e.im + w.re * x.im + w.im * x.re) : cmul(x, w);
+    }
+    const T sc = T(c < 0.0 ? -1.0 : 1.0);
+    if (c == s || c == -s) {
+        const T hi = T(0.75), lo = T(s - 0.75);
+        const T re = sc * x.re - S * x.im, im = sc * x.im + S * x.re;
+        return ADD ? mk(e.re + hi * re + lo * re, e.im + hi * im + lo * im) : mk(hi * re + lo * re, hi * im + lo * im);
+    }
+    if (c > s || -c > s) {
+        const T cr = T(c - (c < 0.0 ? -1.0 : 1.0)), si = T(S * s);
+        const cx<T> u = ADD ? mk(e.re + sc * x.re, e.im + sc * x.im) : mk(sc * x.re, sc * x.im);
+        return mk(u.re + cr * x.re - si * x.im, u.im + cr * x.im + si * x.re);
+    }
+    const T cr = T(c), si = T(S * (s - 1.0));
+    const cx<T> u = ADD ? e + mul_is<S>(x) : mul_is<S>(x);
+    return mk(u.re - si * x.im + cr * x.re, u.im + si * x.re + cr * x.im);
+}
+
+// 2H-point DFT of x[0..H) followed by H zeros: X[2k] = DFT_H(x)[k], X[2k+1] = DFT_H(x w_2H^j)[k].  For odd H
+// the odd frequencies are 2m + H modulo 2H, where w_2H^(j (2m + H)) = w_H^(jm) (-1)^j: no twiddles.
 template <int H, typename T>
 __device__ __forceinline__ void dft_zero_padded(const cx<T>* x, cx<T>* even, cx<T>* odd) {
+    if constexpr (H % 2 == 1) {
+        cx<T> a[H];
 #pragma unroll
-    for (int j = 0; j < H; ++j) {
-        even[j] = x[j];
-        odd[j] = j == 0 ? x[0] : cmulc(x[j], mk(T(WConst<2 * H>::c(j)), T(WConst<2 * H>::s(j))));
+        for (int j = 0; j < H; ++j) {
+            even[j] = x[j];
+            a[j] = j % 2 == 0 ? x[j] : mk(-x[j].re, -x[j].im);
+        }
+        dft_h<H, -1>(a);
+#pragma unroll
+        for (int m = 0; m < H; ++m) odd[(m + (H - 1) / 2) % H] = a[m];
+    } else {
+#pragma unroll
+        for (int j = 0; j < H; ++j) {
+            even[j] = x[j];
+            odd[j] = j == 0 ? x[0] : turn<-1, false>(x[j], x[j], WConst<2 * H>::c(j), WConst<2 * H>::s(j));
+        }
+        dft_h<H, -1>(odd);
     }
     dft_h<H, -1>(even);
-    dft_h<H, -1>(odd);
 }
 
 // Outputs 0..H-1 of the 2H-point inverse DFT of the interleaved (even, odd) inputs, into even.
 template <int H, typename T>
 __device__ __forceinline__ void idft_first_half(cx<T>* even, cx<T>* odd) {
     dft_h<H, +1>(even);
-    dft_h<H, +1>(odd);
-    even[0] = even[0] + odd[0];
+    if constexpr (H % 2 == 1) {
+        cx<T> a[H];
 #pragma unroll
-    for (int n = 1; n < H; ++n) {
-        const T c = T(WConst<2 * H>::c(n)), s = T(WConst<2 * H>::s(n));
-        const cx<T> o = odd[n];
-        even[n] = mk(even[n].re + c * o.re - s * o.im, even[n].im + c * o.im + s * o.re);
+        for (int m = 0; m < H; ++m) a[m] = odd[(m + (H - 1) / 2) % H];
+        dft_h<H, +1>(a);
+#pragma unroll
+        for (int n = 0; n < H; ++n) even[n] = n % 2 == 0 ? even[n] + a[n] : even[n] - a[n];
+    } else {
+        dft_h<H, +1>(odd);
+        even[0] = even[0] + odd[0];
+#pragma unroll
+        for (int n = 1; n < H; ++n) even[n] = turn<+1, true>(even[n], odd[n], WConst<2 * H>::c(n), WConst<2 * H>::s(n));
     }
 }
 
@@ -582,7 +562,7 @@ __global__ void __launch_bounds__(ZwLayout<T, SET, H, R2>::kThreads, 1)
                     const cx<T> v = e[t * LL + s * L];
                     x[s][t] = t == 0 ? v : cmul(v, w[t]);
                 }
-                dft<R2, -1>(x[s]);
+                dft<R2, -1, true>(x[s]);
             }
             if constexpr (SET == kZwZb) {
 #pragma unroll
@@ -612,7 +592,7 @@ __global__ void __launch_bounds__(ZwLayout<T, SET, H, R2>::kThreads, 1)
             }
 #pragma unroll
             for (int s = 0; s < S; ++s) {
-                dft<R2, +1>(x[s]);
+                dft<R2, +1, true>(x[s]);
 #pragma unroll
                 for (int t = 0; t < R2; ++t) e[t * LL + s * L] = t == 0 ? x[s][0] : cmulc(x[s][t], w[t]);
             }
