@@ -1341,19 +1341,24 @@ enum class GramKind {
     kFused,  // TF32x3, operands split inside the kernel (k_gram_tc_ws)
     kSplit,  // TF32x3 after the split pass (k_tf32_split, k_gram_tc)
 };
+// One tile of at most 40 right densities holds the whole request: the fused Gram may sum k-tiles in pairs (see
+// k_gram_tc_ws).
+bool paired_gram(const GramPlan& g) { return g.nl <= clk::tc::BM / 2 && g.nr <= clk::tc::WS_MAX_NB8 / 2; }
 // FP32 potentials and densities can take either TF32x3 Gram: the fused one splits the operands of its
 // tile (at most 64 x 48 densities) itself, once per tile, the other reads split operands that a pass of
-// their own writes.  Per k-tile of 32 atoms an SM takes 1.06 us for a fused tile and 1.10 us for a
-// 64 x 64 tile after the split, whose pass costs 0.019 us a density (36 densities a side over 2.1M
-// atoms: 0.47 ms in one fused tile; 820: 5.56 ms in 91 tiles, and 1.64 ms the split).  CL_TC_SPLIT=1
-// keeps the split pass everywhere; CL_TC_FUSED=1 takes the fused Gram at any tile count.
+// their own writes.  Per k-tile of 32 atoms an SM takes 1.06 us for a fused tile that sums k-tiles in pairs, 1.25 us
+// for one that does not and 1.10 us for a 64 x 64 tile after the split, whose pass costs 0.0167 us a density
+// (110,592 atoms, all pairs of 16 states: 0.213 ms fused, 0.180 + 0.126 split; of 20: 0.464, 0.294 + 0.187; of 24:
+// 0.785, 0.433 + 0.261).  CL_TC_SPLIT=1 keeps the split pass everywhere; CL_TC_FUSED=1 takes the fused Gram at
+// any tile count.
 GramKind gram_kind(const cl_ctx* c, const GramPlan& g, bool v_f32, bool rho_f32, long long n_atoms) {
     if (!use_tc_gram(c) || small_gram(c, n_atoms)) return GramKind::kFp64;
     if (!v_f32 || !rho_f32 || std::getenv("CL_TC_SPLIT")) return GramKind::kSplit;
     if (std::getenv("CL_TC_FUSED")) return GramKind::kFused;
-    const double fused = 1.06 * clk::gram_tile_count(tc_tiles(g, clk::tc::BM / 2, clk::tc::WS_MAX_NB / 2));
+    const double fused = (paired_gram(g) ? 1.06 : 1.25) *
+                         clk::gram_tile_count(tc_tiles(g, clk::tc::BM / 2, clk::tc::WS_MAX_NB / 2));
     const double split = 1.10 * clk::gram_tile_count(tc_tiles(g, clk::tc::BM / 2, clk::tc::BN / 2)) +
-                         0.019 * (g.nl + g.nr);
+                         0.0167 * (g.nl + g.nr);
     return fused <= split ? GramKind::kFused : GramKind::kSplit;
 }
 
@@ -1549,15 +1554,21 @@ void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, const cx<f
     if (smem2 > 227 * 1024) cl::fail(CL_ERR_UNSUPPORTED, "fused Gram needs %zu bytes of shared memory", smem2);
     cudaEvent_t e = prof_begin(c);
     const dim3 grid(tiles, splits);
+    // k-tiles leave the tensor cores in pairs summed in FP32 only for requests in one tile of up to 40 right
+    // densities (36 a side over 2.1M atoms: 0.47 ms); every k-tile of the others goes to FP64 by itself
+    const bool pairs = paired_gram(plan);
     const auto launch_ws = [&](auto ahead, size_t smem) {
         constexpr int AHEAD = decltype(ahead)::value;
-        if (wide) {
-            ensure_smem(k_gram_tc_ws<AHEAD, 12>, 227 * 1024);
-            k_gram_tc_ws<AHEAD, 12><<<grid, ws_threads(12), smem, c->stream>>>(g);
-        } else {
-            ensure_smem(k_gram_tc_ws<AHEAD, 8>, 227 * 1024);
-            k_gram_tc_ws<AHEAD, 8><<<grid, ws_threads(8), smem, c->stream>>>(g);
-        }
+        const auto go = [&](auto kern, int threads) {
+            ensure_smem(kern, 227 * 1024);
+            kern<<<grid, threads, smem, c->stream>>>(g);
+        };
+        if (wide)
+            go(k_gram_tc_ws<AHEAD, 12, false>, ws_threads(12));
+        else if (pairs)
+            go(k_gram_tc_ws<AHEAD, 8, true>, ws_threads(8));
+        else
+            go(k_gram_tc_ws<AHEAD, 8, false>, ws_threads(8));
     };
     if (ws && smem5 <= 227 * 1024)
         launch_ws(std::integral_constant<int, 5>{}, smem5);

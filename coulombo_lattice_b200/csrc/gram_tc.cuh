@@ -724,10 +724,11 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_gram_tc_fused(const FusedG
 //                fourth), and commits them to the stage's empty and the buffer's full barrier;
 //   warps 8-     drain: 8 of them up to N = 80, 12 above (36 densities a side: 0.472 ms with 8, 0.483 with
 //                12); warp w reads lane quarter w % 4 and its share (a half, a third) of the column groups
-//                of 8, two k-tiles at a time: the two FP32 values of a
-//                column summed once (round to nearest, unbiased, at most 2^-24 of the pair
-//                against the TF32 parts' 2^-22 of each product) and added to FP64 registers;
-//                the correction accumulator once after the last k-tile.
+//                of 8, two k-tiles at a time, into FP64 registers.  PAIRS: the two FP32 values of a
+//                column are summed once first (round to nearest, unbiased, at most 2^-24 of the pair
+//                against the TF32 parts' 2^-22 of each product); only where one tile of at most 40
+//                right densities holds the request.  The correction accumulator comes once, after the
+//                last k-tile.
 // TF32 rounding to nearest (ties away from zero, as cvt.rna.tf32.f32 for finite values) is done
 // on the integer pipe: add half the weight of the 13 dropped mantissa bits, clear them.
 // ---------------------------------------------------------------------------------------
@@ -761,7 +762,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-template <int AHEAD, int DRAINS>
+template <int AHEAD, int DRAINS, bool PAIRS>
 __global__ void __launch_bounds__(ws_threads(DRAINS), 1) k_gram_tc_ws(const FusedGram g) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -984,9 +985,9 @@ __global__ void __launch_bounds__(ws_threads(DRAINS), 1) k_gram_tc_ws(const Fuse
                 }
             }
         };
-        // two k-tiles' main products (buffers at columns c0 and c1): their FP32 sum, rounded to
-        // nearest once (unbiased, 2^-24 of the pair against the TF32x3 parts' 2^-22 of each
-        // product), goes into the FP64 sums -- half the conversions and waits of one by one
+        // two k-tiles' main products (buffers at columns c0 and c1), loaded under one wait.  PAIRS: their FP32
+        // sum, rounded to nearest once (unbiased, 2^-24 of the pair against the TF32x3 parts' 2^-22 of each
+        // product), goes into the FP64 sums -- half the conversions of one by one
         const auto add_pair = [&](uint32_t c0, uint32_t c1) {
 #pragma unroll
             for (int j = 0; j < WS_MAX_DC / 8; ++j) {
@@ -997,7 +998,12 @@ __global__ void __launch_bounds__(ws_threads(DRAINS), 1) k_gram_tc_ws(const Fuse
                     tmem_wait_ld16(r);
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
-                        acc[8 * j + i] += (double)(__uint_as_float(r[i]) + __uint_as_float(r[8 + i]));
+                        if (PAIRS) {
+                            acc[8 * j + i] += (double)(__uint_as_float(r[i]) + __uint_as_float(r[8 + i]));
+                        } else {
+                            acc[8 * j + i] += (double)__uint_as_float(r[i]);
+                            acc[8 * j + i] += (double)__uint_as_float(r[8 + i]);
+                        }
                 }
             }
         };
