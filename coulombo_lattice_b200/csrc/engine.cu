@@ -1471,7 +1471,7 @@ void gram_dmma(cl_ctx* c, const cx<SV>* V, long long v_stride, const cx<SR>* rho
     cudaEvent_t e = prof_begin(c);
     const dim3 grid(tiles, splits);
     const auto launch = [&](auto kern) {
-        ensure_smem(kern, 226 * 1024);  // beside 256 bytes of static shared memory
+        ensure_smem(kern, 226 * 1024);  // beside 512 bytes of static shared memory
         kern<<<grid, THREADS, smem, c->stream>>>(rho, g);
     };
     const auto square = [&](auto k) {
@@ -1498,28 +1498,17 @@ void gram_dmma(cl_ctx* c, const cx<SV>* V, long long v_stride, const cx<SR>* rho
              (double)n_atoms * (plan.nl * (double)sizeof(cx<SV>) + plan.nr * (double)sizeof(cx<SR>)));
 }
 
-// The fused Gram on FP32 operands over the whole atom range (see k_gram_tc_fused).
+// The fused Gram on FP32 operands over the whole atom range (see k_gram_tc_ws).
 void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, const cx<float>* rho, long long r_stride,
                    const int* rows_dev, const GramPlan& plan, long long n_atoms, double* out4_dev) {
     using namespace clk::tc;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        CL_CUDA(cudaFuncSetAttribute(k_gram_tc_fused<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        CL_CUDA(cudaFuncSetAttribute(k_gram_tc_fused<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        CL_CUDA(cudaFuncSetAttribute(k_gram_tc_fused<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    });
-    // the warp-specialised kernel takes up to 48 right densities a tile, with 8 drain warps up to 40 (96^3,
-    // blocks of 42 and 36 densities: 0.087 ms in three tiles, 0.070 in two wider ones); CL_TC_NO_WS=1 keeps
-    // the kernel whose warps take every role in turn, up to 64
-    const bool ws = !std::getenv("CL_TC_NO_WS");
+    // up to 48 right densities a tile, with 8 drain warps up to 40 (96^3, blocks of 42 and 36 densities: two tiles of
+    // 48 0.077 ms; with k-tiles summed in pairs they took 0.070, three tiles of 40 0.087)
     FusedGram g{};
-    g.tiles = tc_tiles(plan, BM / 2, ws ? WS_MAX_NB8 / 2 : BN / 2);
-    bool wide = false;
-    if (ws) {
-        const clk::GramTiles wider = tc_tiles(plan, BM / 2, WS_MAX_NB / 2);
-        wide = clk::gram_tile_count(wider) < clk::gram_tile_count(g.tiles);
-        if (wide) g.tiles = wider;
-    }
+    g.tiles = tc_tiles(plan, BM / 2, WS_MAX_NB8 / 2);
+    const clk::GramTiles wider = tc_tiles(plan, BM / 2, WS_MAX_NB / 2);
+    const bool wide = clk::gram_tile_count(wider) < clk::gram_tile_count(g.tiles);
+    if (wide) g.tiles = wider;
     int nA = 1, nB = 1;
     for (int b = 0; b < g.tiles.n; ++b) {
         nA = std::max(nA, std::min(g.tiles.wl[b], g.tiles.b[b].nl));
@@ -1548,15 +1537,16 @@ void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, const cx<f
     g.kt_per = (g.kt_total + splits0 - 1) / splits0;
     const int splits = (g.kt_total + g.kt_per - 1) / g.kt_per;
     // the deepest copy ring that fits: 5 k-tiles ahead (6 slots) at the 2.1M-atom box's 72 densities
-    const size_t smem5 = ws ? ws_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 5) : fused_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 5);
-    const size_t smem3 = ws ? ws_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 3) : fused_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 3);
-    const size_t smem2 = ws ? ws_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 2) : fused_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 2);
+    const size_t smem5 = ws_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 5);
+    const size_t smem3 = ws_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 3);
+    const size_t smem2 = ws_smem_bytes(g.stage_bytes, g.raw_slot_bytes, 2);
     if (smem2 > 227 * 1024) cl::fail(CL_ERR_UNSUPPORTED, "fused Gram needs %zu bytes of shared memory", smem2);
     cudaEvent_t e = prof_begin(c);
     const dim3 grid(tiles, splits);
     // k-tiles leave the tensor cores in pairs summed in FP32 only for requests in one tile of up to 40 right
-    // densities (36 a side over 2.1M atoms: 0.47 ms); every k-tile of the others goes to FP64 by itself
-    const bool pairs = paired_gram(plan);
+    // densities (36 a side over 2.1M atoms: 0.47 ms); every k-tile of the others, with CL_TC_NO_WS=1 of all, goes
+    // to FP64 by itself
+    const bool pairs = paired_gram(plan) && !std::getenv("CL_TC_NO_WS");
     const auto launch_ws = [&](auto ahead, size_t smem) {
         constexpr int AHEAD = decltype(ahead)::value;
         const auto go = [&](auto kern, int threads) {
@@ -1570,18 +1560,12 @@ void gram_tc_fused(cl_ctx* c, const cx<float>* V, long long v_stride, const cx<f
         else
             go(k_gram_tc_ws<AHEAD, 8, false>, ws_threads(8));
     };
-    if (ws && smem5 <= 227 * 1024)
+    if (smem5 <= 227 * 1024)
         launch_ws(std::integral_constant<int, 5>{}, smem5);
-    else if (ws && smem3 <= 227 * 1024)
-        launch_ws(std::integral_constant<int, 3>{}, smem3);
-    else if (ws)
-        launch_ws(std::integral_constant<int, 2>{}, smem2);
-    else if (smem5 <= 227 * 1024)
-        k_gram_tc_fused<5><<<grid, FUSED_THREADS, smem5, c->stream>>>(g);
     else if (smem3 <= 227 * 1024)
-        k_gram_tc_fused<3><<<grid, FUSED_THREADS, smem3, c->stream>>>(g);
+        launch_ws(std::integral_constant<int, 3>{}, smem3);
     else
-        k_gram_tc_fused<2><<<grid, FUSED_THREADS, smem2, c->stream>>>(g);
+        launch_ws(std::integral_constant<int, 2>{}, smem2);
     CL_LAUNCHED();
     prof_end(c, e, CL_KCLASS_GRAM, (double)n_atoms * (plan.nl + plan.nr) * (double)sizeof(cx<float>));
 }

@@ -50,7 +50,6 @@ struct GramArgs {
     const int* lidx;
     long long v_stride;
     const int* ridx;      // right densities: rho[(ridx ? ridx[r] : r) * r_stride + atom]
-    int nl, nr;
     long long r_stride;
     long long na;               // atoms
     long long atoms_per_split;  // a multiple of the chunk
