@@ -1663,10 +1663,10 @@ void gram(cl_ctx* c, const void* V_any, bool v_f32, long long v_stride, const vo
 struct PairSetup {
     DevBuf<clk::PairSeg> segs;  // products grouped by left state, indices into `states` (FP64 kernel)
     // FP64 tensor cores (at most 40 used states, see k_pair_mma)
-    bool mma_ok = false;
+    bool mma_ok = false, mma_sliced = false;
     clk::pm::PairMmaArgs mma{};
     DevBuf<int> mma_prod;
-    int mma_blocks = 0, mma_grid = 1;  // blocks of 8 states; thread blocks
+    int mma_grid = 1;  // thread blocks
     size_t mma_smem = 0;
     // tiles of 4 x 4 states (see k_pair_density_tile)
     bool tile_ok = false;
@@ -1738,55 +1738,83 @@ void pair_tile_setup(cl_ctx* c, const std::vector<int2>& fl, const std::vector<i
     ps.tile_prod.upload(prod.data(), prod.size(), c->stream);
 }
 
-// f(NB, FOLD) as integral constants for nb blocks of 8 states: FOLD from 16 orbitals on, where the products
+// f(NB, PACKED, FOLD, SLICED) as integral constants for n states: FOLD from 16 orbitals on, where the products
 // it leaves out outweigh its shuffles (20 states, 10 orbitals: 0.31 ms without, 0.33 with; 20 orbitals:
-// 0.57 and 0.56; 12 states: 0.139 and 0.126).
+// 0.57 and 0.56; 12 states: 0.139 and 0.126); orbitals in slices come in at more than that.
 template <typename F>
-void with_pair_mma(int nb, int n_orb, F&& f) {
-    const auto blocks = [&](auto fold) {
-        switch (nb) {
-            case 1: f(std::integral_constant<int, 1>{}, fold); break;
-            case 2: f(std::integral_constant<int, 2>{}, fold); break;
-            case 3: f(std::integral_constant<int, 3>{}, fold); break;
-            case 4: f(std::integral_constant<int, 4>{}, fold); break;
-            default: f(std::integral_constant<int, 5>{}, fold); break;
+void with_pair_mma(int n, int n_orb, bool sliced, F&& f) {
+    const auto blocks = [&](auto fold, auto cut) {
+        const std::false_type whole{};
+        switch ((n + 7) / 8) {
+            case 1:
+                if (n <= 4)
+                    f(std::integral_constant<int, 1>{}, std::true_type{}, fold, cut);
+                else
+                    f(std::integral_constant<int, 1>{}, whole, fold, cut);
+                break;
+            case 2: f(std::integral_constant<int, 2>{}, whole, fold, cut); break;
+            case 3: f(std::integral_constant<int, 3>{}, whole, fold, cut); break;
+            case 4: f(std::integral_constant<int, 4>{}, whole, fold, cut); break;
+            default: f(std::integral_constant<int, 5>{}, whole, fold, cut); break;
         }
     };
-    if (n_orb >= 16)
-        blocks(std::true_type{});
+    if (sliced)
+        blocks(std::true_type{}, std::true_type{});
+    else if (n_orb >= 16)
+        blocks(std::true_type{}, std::false_type{});
     else
-        blocks(std::false_type{});
+        blocks(std::false_type{}, std::false_type{});
 }
 
 // Tables and launch shape of the tensor-core kernel: used states ascending, the density row of each
 // product (i, j), i >= j in that order (rows are conj(c_x) c_y, x >= y).  Batches hold about 160 values a
-// state, in powers of two from one atom a warp group up -- more where one block an SM runs anyway (30
-// states: 8 atoms 0.53 ms, 4 atoms 0.60) -- two of them in shared memory; when even the smallest does not
-// fit beside the products (40 states in FP64, many orbitals) the tile kernel runs.
+// state of 8 states, more of fewer (1,280 in all), in powers of two from one tile a warp group up, while enough blocks
+// share an SM and the atoms make a batch for each (12 states, 1 orbital, FP64: 64 atoms, one block an SM, 0.066 ms,
+// 32 atoms 0.051, 16 atoms 0.050; 2 states, 5 orbitals: 32 atoms 0.016, 128 0.014) -- more where one block an SM runs
+// anyway (30 states: 8 atoms 0.53 ms, 4 atoms 0.60) -- two of them in shared memory; when even the smallest does not
+// fit beside the products (many orbitals), it comes in slices of orbitals, as many as let those blocks fit.
 void pair_mma_setup(cl_ctx* c, const std::vector<int2>& fl, const std::vector<int>& used,
                     const std::vector<int>& where, PairSetup& ps) {
     using namespace clk::pm;
     const int n = (int)used.size(), nb = (n + 7) / 8;
     if (n == 0 || nb > MAX_BLOCKS || ps.np > 32767) return;
+    // a step takes 4 orbitals, so one or two waste most of it: of 1 orbital from 9 states on, of 2 from 25 on, the
+    // tile kernel is faster (32,768 atoms, FP32: 1 orbital, 9 states 0.020 ms here, 0.017 there; 20 states 0.033,
+    // 0.028; 40 states 0.088, 0.064, with 2 orbitals 0.088, 0.079; 24 states and 2 orbitals 0.036, 0.043)
+    if ((c->n_orb == 1 ? n > 8 : c->n_orb == 2 && n > 24) && !std::getenv("CL_NO_PAIR_TILE")) return;
     PairMmaArgs& g = ps.mma;
     g = PairMmaArgs{};
     g.n_orb = c->n_orb;
     g.n = c->n_sorted;
     g.np = ps.np;
     g.n_used = n;
-    g.stages = 2;
-    const auto bytes = [&](int at) {
-        const int pitch = state_pitch(at, c->n_orb);
-        return fp64_form(c) ? pair_mma_smem<double>(nb, n, pitch, ps.np, at, g.stages)
-                            : pair_mma_smem<float>(nb, n, pitch, ps.np, at, g.stages);
+    // rows of a tile an atom takes: of up to 4 states, several atoms share a tile
+    g.rows_log2 = n == 1 ? 0 : n == 2 ? 1 : n <= 4 ? 2 : 3;
+    const auto bytes = [&](int at, int orbitals) {
+        const int pitch = state_pitch(at, orbitals);
+        return fp64_form(c) ? pair_mma_smem<double>(nb, n, pitch, ps.np, at)
+                            : pair_mma_smem<float>(nb, n, pitch, ps.np, at);
     };
-    const size_t most = 227 * 1024;
-    int at = warps(nb) / warps_per_atom(nb);
-    if (bytes(at) > most) return;
-    while (at < 64 && (2 * at * c->n_orb <= 160 || (min_blocks(nb) == 1 && at < 16)) && bytes(2 * at) <= most) at *= 2;
+    const size_t most = 227 * 1024, share = 228 * 1024 / min_blocks(nb) - 1024;  // a block's, of those an SM is to hold
+    // batches may grow until one block fewer than that fits, but not below two
+    const size_t room = min_blocks(nb) == 1 ? most : 228 * 1024 / std::max(2, min_blocks(nb) - 1) - 1024;
+    int at = warps(nb) / warps_per_atom(nb) * (8 >> g.rows_log2), staged = c->n_orb;
+    const bool sliced = bytes(at, staged) > most;
+    if (sliced) {
+        g.slice_log2 = 5;
+        while (g.slice_log2 > 3 && bytes(at, 1 << g.slice_log2) > share) --g.slice_log2;
+        staged = 1 << g.slice_log2;
+        if (bytes(at, staged) > most) return;
+    } else {
+        const auto larger = [&] {
+            const bool few = std::min(n, 8) * 2 * at * staged <= 1280 && c->n_sorted >= 2LL * at * 148 * min_blocks(nb);
+            return at < 256 && (few || (min_blocks(nb) == 1 && at < 16)) && bytes(2 * at, staged) <= room;
+        };
+        while (larger()) at *= 2;
+    }
     g.at = at;
     while ((1 << g.at_log2) < at) ++g.at_log2;
-    g.state_pitch = state_pitch(at, c->n_orb);
+    g.state_pitch = state_pitch(at, staged);
     std::vector<int> order(n), pos(n);
     std::iota(order.begin(), order.end(), 0);
     std::sort(order.begin(), order.end(), [&](int x, int y) { return used[x] < used[y]; });
@@ -1804,21 +1832,21 @@ void pair_mma_setup(cl_ctx* c, const std::vector<int2>& fl, const std::vector<in
     }
     ps.mma_prod.upload(prod.data(), prod.size(), c->stream);
     ps.mma_ok = true;
-    ps.mma_blocks = nb;
-    ps.mma_smem = bytes(at);
+    ps.mma_sliced = sliced;
+    ps.mma_smem = bytes(at, staged);
     const long long batches = (g.n + at - 1) / at;
     int resident = 1;
-    with_pair_mma(nb, c->n_orb, [&](auto k, auto fold) {
+    with_pair_mma(n, c->n_orb, sliced, [&](auto k, auto pack, auto fold, auto cut) {
         constexpr int NB = decltype(k)::value;
-        constexpr bool FOLD = decltype(fold)::value;
+        constexpr bool PACKED = decltype(pack)::value, FOLD = decltype(fold)::value, SLICED = decltype(cut)::value;
         const auto count = [&](auto kern) {
             ensure_smem(kern, most);
             CL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, 32 * warps(NB), ps.mma_smem));
         };
         if (fp64_form(c))
-            count(k_pair_mma<NB, FOLD, double>);
+            count(k_pair_mma<NB, PACKED, FOLD, SLICED, double>);
         else
-            count(k_pair_mma<NB, FOLD, float>);
+            count(k_pair_mma<NB, PACKED, FOLD, SLICED, float>);
     });
     ps.mma_grid = (int)std::max<long long>(1, std::min<long long>(batches, 148LL * std::max(1, resident)));
 }
@@ -1885,15 +1913,15 @@ void pair_launch(cl_ctx* c, const PairSetup& ps, void* rho) {
         clk::pm::PairMmaArgs g = ps.mma;
         g.coeff = c->coeff.p;
         g.prod = ps.mma_prod.p;
-        with_pair_mma(ps.mma_blocks, g.n_orb, [&](auto k, auto fold) {
+        with_pair_mma(g.n_used, g.n_orb, ps.mma_sliced, [&](auto k, auto pack, auto fold, auto cut) {
             constexpr int NB = decltype(k)::value;
-            constexpr bool FOLD = decltype(fold)::value;
+            constexpr bool PACKED = decltype(pack)::value, FOLD = decltype(fold)::value, SLICED = decltype(cut)::value;
             const int threads = 32 * clk::pm::warps(NB);
             if (fp64_form(c))
-                clk::pm::k_pair_mma<NB, FOLD, double><<<ps.mma_grid, threads, ps.mma_smem, c->stream>>>(
+                clk::pm::k_pair_mma<NB, PACKED, FOLD, SLICED, double><<<ps.mma_grid, threads, ps.mma_smem, c->stream>>>(
                     g, static_cast<cx<double>*>(rho));
             else
-                clk::pm::k_pair_mma<NB, FOLD, float><<<ps.mma_grid, threads, ps.mma_smem, c->stream>>>(
+                clk::pm::k_pair_mma<NB, PACKED, FOLD, SLICED, float><<<ps.mma_grid, threads, ps.mma_smem, c->stream>>>(
                     g, static_cast<cx<float>*>(rho));
         });
     } else if (fp64_form(c) && !ps.tile_ok) {
