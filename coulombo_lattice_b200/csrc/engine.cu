@@ -297,6 +297,7 @@ struct cl_ctx {
     long long n_atoms = 0, n_sorted = 0;
     DevBuf<cx<double>> coeff;
     DevBuf<int> cell_sorted, orig_sorted, row_ptr;
+    DevBuf<unsigned long long> row_mask;  // sub-lattice forms: the atoms of every row (k_row_masks)
     DevBuf<cx<double>> coeff_stage;  // two states of caller coefficients, input atom order
     long long live_rows = 0;           // rows (y, z) holding at least one atom
     std::vector<int> atom_slot;        // input atom -> sorted (deduplicated) slot
@@ -318,7 +319,7 @@ struct cl_ctx {
 
     // Changes whenever a buffer that a request's launches name gets other storage.
     unsigned long long buffer_moves() const {
-        unsigned long long m = khat64.moves + khat32.moves + coeff.moves + cell_sorted.moves + row_ptr.moves;
+        unsigned long long m = khat64.moves + khat32.moves + coeff.moves + cell_sorted.moves + row_ptr.moves + row_mask.moves;
         m += (unsigned long long)work.moves + rounds.moves + tc_buf.moves;
         m += (unsigned long long)sl.H64.moves + sl.phxy64.moves + sl.phz64.moves + sl.H32.moves + sl.phxy32.moves +
              sl.phz32.moves + sl.zw_tab.moves + sl.zw_col.moves + sl.zw_zph.moves;
@@ -1146,9 +1147,9 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
         cudaEvent_t e = prof_begin(c);
         if (qplane) {
             if (nx == ny)
-                clp::pfwd<T>(c->stream, rho_c, rho_stride, row_ptr, cell, buf, vM, twx, nx, nz, cnt);
+                clp::pfwd<T>(c->stream, rho_c, rho_stride, row_ptr, c->row_mask.p, buf, vM, twx, nx, nz, cnt);
             else
-                clp::pfwd_xy<T>(c->stream, rho_c, rho_stride, row_ptr, cell, buf, vM, twx, twy, nx, ny, nz, cnt);
+                clp::pfwd_xy<T>(c->stream, rho_c, rho_stride, row_ptr, c->row_mask.p, buf, vM, twx, twy, nx, ny, nz, cnt);
         } else if (xy_fwd) {
             clp::xyfwd<T>(c->stream, rho_c, rho_stride, row_ptr, cell, buf, vM, twx, rp0, nx, ny, nz, cnt);
         } else if (!(reg_x && clp::xfwd<T>(c->stream, v_xf, rho_c, rho_stride, row_ptr, cell, buf, vM, twx, rp0, nx,
@@ -1195,9 +1196,9 @@ void run_sublattice(cl_ctx* c, const cx<T>* rho, long long rho_stride, int np, v
         e = prof_begin(c);
         if (qplane) {
             if (nx == ny)
-                clp::pinv<T>(c->stream, buf, vM, twx, row_ptr, cell, out_c, out_stride, nx, nz, cnt);
+                clp::pinv<T>(c->stream, buf, vM, twx, row_ptr, c->row_mask.p, out_c, out_stride, nx, nz, cnt);
             else
-                clp::pinv_xy<T>(c->stream, buf, vM, twx, twy, row_ptr, cell, out_c, out_stride, nx, ny, nz, cnt);
+                clp::pinv_xy<T>(c->stream, buf, vM, twx, twy, row_ptr, c->row_mask.p, out_c, out_stride, nx, ny, nz, cnt);
         } else if (xy_inv) {
             clp::xyinv<T>(c->stream, buf, vM, twx, row_ptr, cell, out_c, out_stride, nx, ny, nz, cnt);
         } else if (!(reg_x && clp::xinv<T>(c->stream, v_xi, buf, vM, twx, row_ptr, cell, out_c, out_stride, nx, nrows,
@@ -1740,7 +1741,8 @@ void pair_tile_setup(cl_ctx* c, const std::vector<int2>& fl, const std::vector<i
 
 // f(NB, PACKED, FOLD, SLICED) as integral constants for n states: FOLD from 16 orbitals on, where the products
 // it leaves out outweigh its shuffles (20 states, 10 orbitals: 0.31 ms without, 0.33 with; 20 orbitals:
-// 0.57 and 0.56; 12 states: 0.139 and 0.126); orbitals in slices come in at more than that.
+// 0.57 and 0.56; 12 states: 0.139 and 0.126), of 5 to 8 states from 10 on (5 states, 8 orbitals: 0.031 and 0.032; 10
+// orbitals: 0.039 and 0.038); orbitals in slices come in at more than that.
 template <typename F>
 void with_pair_mma(int n, int n_orb, bool sliced, F&& f) {
     const auto blocks = [&](auto fold, auto cut) {
@@ -1760,7 +1762,7 @@ void with_pair_mma(int n, int n_orb, bool sliced, F&& f) {
     };
     if (sliced)
         blocks(std::true_type{}, std::true_type{});
-    else if (n_orb >= 16)
+    else if (n_orb >= (n > 4 && n <= 8 ? 10 : 16))
         blocks(std::true_type{}, std::false_type{});
     else
         blocks(std::false_type{}, std::false_type{});
@@ -2299,6 +2301,13 @@ void load_cells(cl_ctx* c, int64_t n_atoms, const int64_t* cells) {
     c->orig_sorted.upload(orig_s.data(), orig_s.size(), c->stream);
     c->row_ptr.upload(rp.data(), rp.size(), c->stream);
     c->slot_of_atom.upload(c->atom_slot.data(), c->atom_slot.size(), c->stream);
+    if (c->sl.active && c->sl.sub[0] <= 64) {
+        c->row_mask.alloc((size_t)nrows);
+        CL_CUDA(cudaMemsetAsync(c->row_mask.p, 0, sizeof(unsigned long long) * nrows, c->stream));
+        clk::k_row_masks<<<grid_for(c->n_sorted), 256, 0, c->stream>>>(c->cell_sorted.p, (int)c->n_sorted, nx,
+                                                                       c->row_mask.p);
+        CL_LAUNCHED();
+    }
     CL_CUDA(cudaStreamSynchronize(c->stream));
     c->cells_seen.assign(cells, cells + n_atoms);
 }

@@ -86,20 +86,20 @@ bool xinv(cudaStream_t s, Variant v, cx<T>* buf, long long M, const cx<T>* tw, c
 bool plane_supported(bool fp32, int nx, int ny);
 // Quadrant plane passes of the sub-lattice forms (plane_w.cuh): planes with atoms in their
 // [0, nx/2) x [0, ny/2) quadrant, x and y transforms both in one launch; pfwd and pinv on n x n planes,
-// pfwd_xy and pinv_xy on planes of two lengths (plane_xy.cuh).
+// pfwd_xy and pinv_xy on planes of two lengths (plane_xy.cuh).  row_mask: the atoms of every row (k_row_masks).
 bool quadrant_supported(bool fp32, int nx, int ny);
 template <typename T>
-bool pfwd(cudaStream_t s, const cx<T>* rho, long long rho_stride, const int* row_ptr, const int* cell, cx<T>* buf,
+bool pfwd(cudaStream_t s, const cx<T>* rho, long long rho_stride, const int* row_ptr, const unsigned long long* row_mask, cx<T>* buf,
           long long M, const cx<T>* tw, int n, int nz, int cnt);
 template <typename T>
-bool pinv(cudaStream_t s, const cx<T>* buf, long long M, const cx<T>* tw, const int* row_ptr, const int* cell,
+bool pinv(cudaStream_t s, const cx<T>* buf, long long M, const cx<T>* tw, const int* row_ptr, const unsigned long long* row_mask,
           cx<T>* out, long long o_stride, int n, int nz, int cnt);
 template <typename T>
-bool pfwd_xy(cudaStream_t s, const cx<T>* rho, long long rho_stride, const int* row_ptr, const int* cell, cx<T>* buf,
+bool pfwd_xy(cudaStream_t s, const cx<T>* rho, long long rho_stride, const int* row_ptr, const unsigned long long* row_mask, cx<T>* buf,
              long long M, const cx<T>* twx, const cx<T>* twy, int nx, int ny, int nz, int cnt);
 template <typename T>
 bool pinv_xy(cudaStream_t s, const cx<T>* buf, long long M, const cx<T>* twx, const cx<T>* twy, const int* row_ptr,
-             const int* cell, cx<T>* out, long long o_stride, int nx, int ny, int nz, int cnt);
+             const unsigned long long* row_mask, cx<T>* out, long long o_stride, int nx, int ny, int nz, int cnt);
 template <typename T>
 bool xyfwd(cudaStream_t s, const cx<T>* rho, long long rho_stride, const int* row_ptr, const int* cell, cx<T>* buf,
            long long M, const cx<T>* tw, const clk::RoundPhase& rp, int nx, int ny, int nz, int cnt);

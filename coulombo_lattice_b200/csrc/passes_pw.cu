@@ -22,7 +22,7 @@ bool quadrant_supported(bool fp32, int nx, int ny) {
 }
 
 template <>
-bool pfwd<float>(cudaStream_t s, const cx<float>* rho, long long rho_stride, const int* row_ptr, const int* cell,
+bool pfwd<float>(cudaStream_t s, const cx<float>* rho, long long rho_stride, const int* row_ptr, const unsigned long long* row_mask,
                  cx<float>* buf, long long M, const cx<float>* tw, int n, int nz, int cnt) {
     return clk::pw::with_plane_w(n, [&](auto tag) {
         using L = clk::pw::PlaneW<float, decltype(tag)::r1, decltype(tag)::r2, true>;
@@ -30,21 +30,21 @@ bool pfwd<float>(cudaStream_t s, const cx<float>* rho, long long rho_stride, con
             auto kern = clk::pw::k_pfwd<float, decltype(tag)::r1, decltype(tag)::r2>;
             set_smem(kern, L::smem);
             kern<<<dim3((unsigned)nz, plane_groups(nz, cnt, L::MIN)), L::THREADS, L::smem, s>>>(
-                rho, rho_stride, row_ptr, cell, buf, M, tw, cnt);
+                rho, rho_stride, row_ptr, row_mask, buf, M, tw, cnt);
         }
     });
 }
 
 template <>
 bool pinv<float>(cudaStream_t s, const cx<float>* buf, long long M, const cx<float>* tw, const int* row_ptr,
-                 const int* cell, cx<float>* out, long long o_stride, int n, int nz, int cnt) {
+                 const unsigned long long* row_mask, cx<float>* out, long long o_stride, int n, int nz, int cnt) {
     return clk::pw::with_plane_w(n, [&](auto tag) {
         using L = clk::pw::PlaneW<float, decltype(tag)::r1, decltype(tag)::r2, false>;
         if constexpr (L::smem <= 227 * 1024) {
             auto kern = clk::pw::k_pinv<float, decltype(tag)::r1, decltype(tag)::r2>;
             set_smem(kern, L::smem);
             kern<<<dim3((unsigned)nz, plane_groups(nz, cnt, L::MIN)), L::THREADS, L::smem, s>>>(
-                buf, M, tw, row_ptr, cell, out, o_stride, cnt);
+                buf, M, tw, row_ptr, row_mask, out, o_stride, cnt);
         }
     });
 }

@@ -67,17 +67,19 @@ struct Occupancy {
     unsigned* base;  // [Q], from the plane's first atom
     bool full;       // every quadrant point, in order
 };
-// (qx, qy): the quadrant; (nx, ny): the plane.
-__device__ __forceinline__ Occupancy plane_occupancy(unsigned* mem, const int* row_ptr, const int* cell, int z, int a0,
-                                                     int a1, int qx, int qy, int nx, int ny) {
+// (qx, qy): the quadrant; ny: rows of the plane; row_mask: the atoms of every row (k_row_masks).  Blocks that built
+// the masks from their atoms' cells spent 5 us on it before the first copy: 96 x 96 planes with 92 x 92 atoms,
+// one density 0.035 -> 0.026 ms forward and 0.038 -> 0.025 inverse, six 0.106 -> 0.080 and 0.112 -> 0.080.
+__device__ __forceinline__ Occupancy plane_occupancy(unsigned* mem, const int* row_ptr,
+                                                     const unsigned long long* row_mask, int z, int a0, int a1, int qx,
+                                                     int qy, int ny) {
     Occupancy o{mem, mem + 2 * qy, a1 - a0 == qx * qy};
-    for (int i = threadIdx.x; i < 2 * qy; i += blockDim.x) o.mask[i] = 0;
-    for (int y = threadIdx.x; y < qy; y += blockDim.x) o.base[y] = row_ptr[z * ny + y] - a0;
-    __syncthreads();
     if (!o.full)
-        for (int i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
-            const int x = cell[i] % nx, y = cell[i] / nx % ny;
-            atomicOr(&o.mask[2 * y + (x >> 5)], 1u << (x & 31));
+        for (int y = threadIdx.x; y < qy; y += blockDim.x) {
+            const unsigned long long m = row_mask[z * ny + y];
+            o.base[y] = row_ptr[z * ny + y] - a0;
+            o.mask[2 * y] = (unsigned)m;
+            o.mask[2 * y + 1] = (unsigned)(m >> 32);
         }
     __syncthreads();
     return o;
@@ -93,7 +95,7 @@ __device__ __forceinline__ int atom_at(const Occupancy& o, int x, int y, int Q) 
 template <typename T, int H, int R2>
 __global__ void __launch_bounds__(PlaneW<T, H, R2, true>::THREADS, PlaneW<T, H, R2, true>::MIN)
     k_pfwd(const cx<T>* __restrict__ rho, long long rho_stride, const int* __restrict__ row_ptr,
-           const int* __restrict__ cell, cx<T>* __restrict__ out, long long out_stride,
+           const unsigned long long* __restrict__ row_mask, cx<T>* __restrict__ out, long long out_stride,
            const cx<T>* __restrict__ tw_g, int np) {
     using L = PlaneW<T, H, R2, true>;
     constexpr int R1 = L::R1, N = L::N, Q = L::Q, PQ = L::PQ, TP = L::TP, SP = L::SP, RB = L::RB, THREADS = L::THREADS;
@@ -104,7 +106,7 @@ __global__ void __launch_bounds__(PlaneW<T, H, R2, true>::THREADS, PlaneW<T, H, 
     const int tid = threadIdx.x, z = blockIdx.x;
     for (int i = tid; i < N; i += THREADS) tw[i] = tw_g[(i / R1) * (i % R1)];  // [t][q]: W^(t q)
     const int a0 = row_ptr[z * N], a1 = row_ptr[z * N + N];
-    const Occupancy occ = plane_occupancy(reinterpret_cast<unsigned*>(tw + N), row_ptr, cell, z, a0, a1, Q, Q, N, N);
+    const Occupancy occ = plane_occupancy(reinterpret_cast<unsigned*>(tw + N), row_ptr, row_mask, z, a0, a1, Q, Q, N);
     const int per = (np + gridDim.y - 1) / gridDim.y;
     const int p_begin = blockIdx.y * per, p_end = min(np, p_begin + per);
     constexpr int PER = 16 / (int)sizeof(cx<T>);  // values a 16-byte copy
@@ -208,7 +210,7 @@ __global__ void __launch_bounds__(PlaneW<T, H, R2, true>::THREADS, PlaneW<T, H, 
 template <typename T, int H, int R2>
 __global__ void __launch_bounds__(PlaneW<T, H, R2, false>::THREADS, PlaneW<T, H, R2, false>::MIN)
     k_pinv(const cx<T>* __restrict__ buf, long long stride, const cx<T>* __restrict__ tw_g,
-           const int* __restrict__ row_ptr, const int* __restrict__ cell, cx<T>* __restrict__ out,
+           const int* __restrict__ row_ptr, const unsigned long long* __restrict__ row_mask, cx<T>* __restrict__ out,
            long long o_stride, int np) {
     using L = PlaneW<T, H, R2, false>;
     constexpr int R1 = L::R1, N = L::N, Q = L::Q, PQ = L::PQ, TP = L::TP, SP = L::SP, RB = L::RB, THREADS = L::THREADS;
@@ -220,7 +222,7 @@ __global__ void __launch_bounds__(PlaneW<T, H, R2, false>::THREADS, PlaneW<T, H,
     const int tid = threadIdx.x, z = blockIdx.x;
     for (int i = tid; i < N; i += THREADS) tw[i] = tw_g[(i / R1) * (i % R1)];  // [t][q]: W^(t q)
     const int a0 = row_ptr[z * N], a1 = row_ptr[z * N + N];
-    const Occupancy occ = plane_occupancy(reinterpret_cast<unsigned*>(tw + N), row_ptr, cell, z, a0, a1, Q, Q, N, N);
+    const Occupancy occ = plane_occupancy(reinterpret_cast<unsigned*>(tw + N), row_ptr, row_mask, z, a0, a1, Q, Q, N);
     const int per = (np + gridDim.y - 1) / gridDim.y;
     const int p_begin = blockIdx.y * per, p_end = min(np, p_begin + per);
     cx<T> v[IX][R2];
@@ -298,11 +300,12 @@ __global__ void __launch_bounds__(PlaneW<T, H, R2, false>::THREADS, PlaneW<T, H,
                 od[k] = c[(2 * k + 1) * PQ];
             }
             idft_first_half<H>(ev, od);
+            int i[H];
 #pragma unroll
-            for (int n = 0; n < H; ++n) {
-                const int i = atom_at(occ, x, t + R2 * n, Q);
-                if (i >= 0) op[i] = ev[n];
-            }
+            for (int n = 0; n < H; ++n) i[n] = atom_at(occ, x, t + R2 * n, Q);
+#pragma unroll
+            for (int n = 0; n < H; ++n)
+                if (i[n] >= 0) op[i[n]] = ev[n];
         }
         // I is rewritten only after the barrier that follows the next plane's first stage
     }

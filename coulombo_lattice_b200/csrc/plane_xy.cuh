@@ -92,11 +92,12 @@ __device__ __noinline__ void y_inverse(cx<T>* I, int pitch, int Q, const cx<T>* 
             od[k] = c[(2 * k + 1) * pitch];
         }
         idft_first_half<H>(ev, od);
+        int a[H];
 #pragma unroll
-        for (int n = 0; n < H; ++n) {
-            const int a = atom_at(occ, i.x, i.k + R2 * n, Q);
-            if (a >= 0) op[a] = ev[n];
-        }
+        for (int n = 0; n < H; ++n) a[n] = atom_at(occ, i.x, i.k + R2 * n, Q);
+#pragma unroll
+        for (int n = 0; n < H; ++n)
+            if (a[n] >= 0) op[a[n]] = ev[n];
     }
 }
 
@@ -125,7 +126,7 @@ struct PlaneXY {
 template <typename T, int H, int R2>
 __global__ void __launch_bounds__(PlaneXY<T, H, R2, true>::THREADS, PlaneXY<T, H, R2, true>::MIN)
     k_pfwd_xy(const cx<T>* __restrict__ rho, long long rho_stride, const int* __restrict__ row_ptr,
-              const int* __restrict__ cell, cx<T>* __restrict__ out, long long out_stride,
+              const unsigned long long* __restrict__ row_mask, cx<T>* __restrict__ out, long long out_stride,
               const cx<T>* __restrict__ twx_g, const cx<T>* __restrict__ twy_g, int ny, int np) {
     using L = PlaneW<T, H, R2, true>;
     constexpr int R1 = L::R1, N = L::N, Q = L::Q, PQ = L::PQ, TP = L::TP, SP = L::SP, RB = L::RB, THREADS = L::THREADS;
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(PlaneXY<T, H, R2, true>::THREADS, PlaneXY<T, H
     for (int i = tid; i < N; i += THREADS) tw[i] = twx_g[(i / R1) * (i % R1)];
     for (int i = tid; i < ny; i += THREADS) twy[i] = twy_g[(i / ry1) * (i % ry1)];
     const int a0 = row_ptr[z * ny], a1 = row_ptr[z * ny + ny];
-    const Occupancy occ = plane_occupancy(reinterpret_cast<unsigned*>(twy + ny), row_ptr, cell, z, a0, a1, Q, qy, N, ny);
+    const Occupancy occ = plane_occupancy(reinterpret_cast<unsigned*>(twy + ny), row_ptr, row_mask, z, a0, a1, Q, qy, ny);
     const int per = (np + gridDim.y - 1) / gridDim.y;
     const int p_begin = blockIdx.y * per, p_end = min(np, p_begin + per);
     constexpr int PER = 16 / (int)sizeof(cx<T>);  // values a 16-byte copy
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(PlaneXY<T, H, R2, true>::THREADS, PlaneXY<T, H
 template <typename T, int H, int R2>
 __global__ void __launch_bounds__(PlaneXY<T, H, R2, false>::THREADS, PlaneXY<T, H, R2, false>::MIN)
     k_pinv_xy(const cx<T>* __restrict__ buf, long long stride, const cx<T>* __restrict__ twx_g,
-              const cx<T>* __restrict__ twy_g, const int* __restrict__ row_ptr, const int* __restrict__ cell,
+              const cx<T>* __restrict__ twy_g, const int* __restrict__ row_ptr, const unsigned long long* __restrict__ row_mask,
               cx<T>* __restrict__ out, long long o_stride, int ny, int np) {
     using L = PlaneW<T, H, R2, false>;
     constexpr int R1 = L::R1, N = L::N, Q = L::Q, PQ = L::PQ, TP = L::TP, SP = L::SP, RB = L::RB, THREADS = L::THREADS;
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(PlaneXY<T, H, R2, false>::THREADS, PlaneXY<T, 
     for (int i = tid; i < N; i += THREADS) tw[i] = twx_g[(i / R1) * (i % R1)];
     for (int i = tid; i < ny; i += THREADS) twy[i] = twy_g[(i / ry1) * (i % ry1)];
     const int a0 = row_ptr[z * ny], a1 = row_ptr[z * ny + ny];
-    const Occupancy occ = plane_occupancy(reinterpret_cast<unsigned*>(twy + ny), row_ptr, cell, z, a0, a1, Q, qy, N, ny);
+    const Occupancy occ = plane_occupancy(reinterpret_cast<unsigned*>(twy + ny), row_ptr, row_mask, z, a0, a1, Q, qy, ny);
     const int per = (np + gridDim.y - 1) / gridDim.y;
     const int p_begin = blockIdx.y * per, p_end = min(np, p_begin + per);
     cx<T> v[IX][R2];

@@ -194,6 +194,14 @@ __global__ void k_sl_widen(const cx<T>* __restrict__ src, long long s_stride, cx
         d[i] = widen(s[i]);
 }
 
+// The atoms of every row of the virtual grid, for the quadrant plane passes (plane_w.cuh): bit x of row_mask[row]
+// for an atom at (x, row), x < 64; row_mask is zero before.
+template <typename M>
+__global__ void k_row_masks(const int* __restrict__ cell, int n, int nx, M* __restrict__ row_mask) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        atomicOr(&row_mask[cell[i] / nx], M(1) << (cell[i] % nx));
+}
+
 // out[s][a] = Re V[s][slot[a]] for the states s = blockIdx.y and the atoms a in the caller's order.
 template <typename T>
 __global__ void k_potential_of_atoms(const cx<T>* __restrict__ V, long long v_stride, const int* __restrict__ slot,
