@@ -1768,6 +1768,26 @@ void with_pair_mma(int n, int n_orb, bool sliced, F&& f) {
         blocks(std::false_type{}, std::false_type{});
 }
 
+// Whether np products of n states with t4 of their 4 x 4 tiles named go to the tile kernel, which forms those tiles
+// alone and takes orbitals one by one; the tensor-core kernel forms every 8 x 8 tile over steps of 4 orbitals.  Of 1
+// orbital from 9 states on it does (32,768 atoms, FP32: 9 states 0.020 ms on the tensor cores, 0.017 in tiles; 20 states
+// 0.033 and 0.028), beyond 10 orbitals or up to 16 states it does not (12 orbitals, 40 potentials: 0.137 and 0.163; 16
+// states of 5 orbitals, all products: 0.030 and 0.042).  Between them the two costs decide, us at 32,768 atoms fitted to
+// 17 to 40 states, 2 to 10 orbitals, and products from potentials to all (the choice costs 0.4 % on average, at most 15 %):
+// the tile kernel's coefficients, tiles and products; the tensor-core kernel's steps, by its blocks, and products.
+// Measured, 5 orbitals: FP32 potentials of 24 states 0.043 ms on the tensor cores and 0.039, of 40 0.092 and 0.059; all
+// products of 24, 0.052 and 0.067, of 40, 0.134 and 0.138; FP64 of 40, 0.183 and 0.153.
+bool pair_tiles_faster(int n, int n_orb, int np, int t4, bool fp64) {
+    const int nb = (n + 7) / 8;
+    if (n_orb == 1) return n > 8;
+    if (nb <= 2 || n_orb > (nb == 3 ? 8 : 10)) return false;
+    const int pad = (n + 3) / 4 * 4;
+    const double tiles = 4 + 0.25 * pad + n_orb * (0.185 * pad + 0.2 * t4) + np * (fp64 ? 0.05 : 0.035);
+    static const double steps[3][3] = {{32, 43, 56}, {58, 76, 108}, {69, 93, 138}};
+    const double product = nb == 3 ? (fp64 ? 0.02 : 0.01) : (fp64 ? 0.08 : 0.04);
+    return tiles < 0.97 * (steps[nb - 3][(n_orb + 3) / 4 - 1] + np * product);
+}
+
 // Tables and launch shape of the tensor-core kernel: used states ascending, the density row of each
 // product (i, j), i >= j in that order (rows are conj(c_x) c_y, x >= y).  Batches hold about 160 values a
 // state of 8 states, more of fewer (1,280 in all), in powers of two from one tile a warp group up, while enough blocks
@@ -1780,10 +1800,23 @@ void pair_mma_setup(cl_ctx* c, const std::vector<int2>& fl, const std::vector<in
     using namespace clk::pm;
     const int n = (int)used.size(), nb = (n + 7) / 8;
     if (n == 0 || nb > MAX_BLOCKS || ps.np > 32767) return;
-    // a step takes 4 orbitals, so one or two waste most of it: of 1 orbital from 9 states on, of 2 from 25 on, the
-    // tile kernel is faster (32,768 atoms, FP32: 1 orbital, 9 states 0.020 ms here, 0.017 there; 20 states 0.033,
-    // 0.028; 40 states 0.088, 0.064, with 2 orbitals 0.088, 0.079; 24 states and 2 orbitals 0.036, 0.043)
-    if ((c->n_orb == 1 ? n > 8 : c->n_orb == 2 && n > 24) && !std::getenv("CL_NO_PAIR_TILE")) return;
+    std::vector<int> order(n), pos(n);
+    std::iota(order.begin(), order.end(), 0);
+    std::sort(order.begin(), order.end(), [&](int x, int y) { return used[x] < used[y]; });
+    for (int k = 0; k < n; ++k) pos[order[k]] = k;
+    std::vector<int> prod((size_t)64 * nb * nb, -1);
+    std::array<std::array<bool, 2 * MAX_BLOCKS>, 2 * MAX_BLOCKS> named{};  // tiles of 4 x 4 states
+    int t4 = 0;
+    for (int p = 0; p < ps.np; ++p) {
+        const int i = pos[where[fl[p].x]], j = pos[where[fl[p].y]];
+        if (i < j) cl::fail(CL_ERR_STATE, "pair density with its lower state first");
+        int& row = prod[(size_t)i * 8 * nb + j];
+        if (row >= 0) return;  // the same product twice: the kernels with a row per product
+        row = p;
+        t4 += !named[i / 4][j / 4];
+        named[i / 4][j / 4] = true;
+    }
+    if (pair_tiles_faster(n, c->n_orb, ps.np, t4, fp64_form(c)) && !std::getenv("CL_NO_PAIR_TILE")) return;
     PairMmaArgs& g = ps.mma;
     g = PairMmaArgs{};
     g.n_orb = c->n_orb;
@@ -1817,21 +1850,7 @@ void pair_mma_setup(cl_ctx* c, const std::vector<int2>& fl, const std::vector<in
     g.at = at;
     while ((1 << g.at_log2) < at) ++g.at_log2;
     g.state_pitch = state_pitch(at, staged);
-    std::vector<int> order(n), pos(n);
-    std::iota(order.begin(), order.end(), 0);
-    std::sort(order.begin(), order.end(), [&](int x, int y) { return used[x] < used[y]; });
-    for (int k = 0; k < n; ++k) {
-        pos[order[k]] = k;
-        g.state[k] = used[order[k]];
-    }
-    std::vector<int> prod((size_t)64 * nb * nb, -1);
-    for (int p = 0; p < ps.np; ++p) {
-        const int i = pos[where[fl[p].x]], j = pos[where[fl[p].y]];
-        if (i < j) cl::fail(CL_ERR_STATE, "pair density with its lower state first");
-        int& row = prod[(size_t)i * 8 * nb + j];
-        if (row >= 0) return;  // the same product twice: the kernels with a row per product
-        row = p;
-    }
+    for (int k = 0; k < n; ++k) g.state[k] = used[order[k]];
     ps.mma_prod.upload(prod.data(), prod.size(), c->stream);
     ps.mma_ok = true;
     ps.mma_sliced = sliced;
