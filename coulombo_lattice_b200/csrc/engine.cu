@@ -231,10 +231,13 @@ size_t l2_chunk_bytes() {
     return (size_t)(std::max(0.0, mb) * 1024 * 1024);
 }
 
+// Allows launches of `kernel` with `bytes` of dynamic shared memory.  The limit is one per kernel, whatever the
+// thread or context: all set the same, the most that fits beside the kernel's static shared memory, so that none lowers
+// it between another's call and launch.
 template <typename K>
-void ensure_smem(K kernel, size_t bytes) {
-    if (bytes > 227 * 1024) cl::fail(CL_ERR_UNSUPPORTED, "tile needs %zu bytes of shared memory", bytes);
-    CL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+void ensure_smem(K kernel, size_t bytes, size_t most = 227 * 1024) {
+    if (bytes > most) cl::fail(CL_ERR_UNSUPPORTED, "tile needs %zu bytes of shared memory", bytes);
+    CL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
 }
 
 }  // namespace
@@ -1472,7 +1475,7 @@ void gram_dmma(cl_ctx* c, const cx<SV>* V, long long v_stride, const cx<SR>* rho
     cudaEvent_t e = prof_begin(c);
     const dim3 grid(tiles, splits);
     const auto launch = [&](auto kern) {
-        ensure_smem(kern, 226 * 1024);  // beside 512 bytes of static shared memory
+        ensure_smem(kern, 226 * 1024, 226 * 1024);  // beside 512 bytes of static shared memory
         kern<<<grid, THREADS, smem, c->stream>>>(rho, g);
     };
     const auto square = [&](auto k) {
@@ -1927,8 +1930,6 @@ void pair_setup(cl_ctx* c, const std::vector<int2>& fl, PairSetup& ps) {
 }
 
 void pair_launch(cl_ctx* c, const PairSetup& ps, void* rho) {
-    // the shared-memory attribute is per kernel, so another setup (of another group or
-    // request) may have lowered it since this one was prepared
     cudaEvent_t e = prof_begin(c);
     if (ps.mma_ok) {
         clk::pm::PairMmaArgs g = ps.mma;

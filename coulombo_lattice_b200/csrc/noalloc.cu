@@ -83,7 +83,8 @@ clk::FftPlan plan_for(int n) {
 template <typename K>
 void allow_smem(K kernel, size_t bytes) {
     if (bytes > 227 * 1024) cl::fail(CL_ERR_UNSUPPORTED, "tile needs %zu bytes of shared memory", bytes);
-    NA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    // one limit per kernel, whatever the thread: all set the same
+    NA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
 }
 
 template <int S>

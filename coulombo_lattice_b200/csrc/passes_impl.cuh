@@ -19,9 +19,10 @@ constexpr int default_lines() {
 }
 
 template <typename K>
-void set_smem(K kernel, size_t bytes) {
-    // an oversized request makes the launch itself fail, which the caller reports
-    if (bytes <= 227 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+void set_smem(K kernel, size_t bytes, size_t most = 227 * 1024) {
+    // one limit per kernel, whatever the thread or context: all set the same, the most beside its static shared
+    // memory; an oversized request makes the launch itself fail, which the caller reports
+    if (bytes <= most) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
 }
 
 // Calls f(std::integral_constant<int, L>) with the variant's lines per block (the half-width

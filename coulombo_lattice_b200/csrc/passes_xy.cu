@@ -39,7 +39,7 @@ bool xyfwd(cudaStream_t s, const cx<T>* rho, long long rho_stride, const int* ro
         constexpr int TH = decltype(threads)::value, MB = decltype(minb)::value;
         auto kern = clk::k_xyfwd_plane<T, Tag::r1, Tag::r2, TH, MB>;
         const size_t smem = clk::PlaneSmem<T, Tag::r1, Tag::r2, TH, true, MB>::bytes;
-        set_smem(kern, smem);
+        set_smem(kern, smem, smem);  // constant of the kernel, beside static shared memory
         const int nr = std::max(1, rp.n_rounds);
         kern<<<dim3((unsigned)nz, plane_groups(nz * nr, cnt, MB), nr), TH, smem, s>>>(rho, rho_stride, row_ptr, cell,
                                                                                      buf, M, tw, rp, cnt);
@@ -54,7 +54,7 @@ bool xyinv(cudaStream_t s, cx<T>* buf, long long M, const cx<T>* tw, const int* 
         constexpr int TH = decltype(threads)::value, MB = decltype(minb)::value;
         auto kern = clk::k_xyinv_plane<T, Tag::r1, Tag::r2, TH, MB>;
         const size_t smem = clk::PlaneSmem<T, Tag::r1, Tag::r2, TH, false>::bytes;
-        set_smem(kern, smem);
+        set_smem(kern, smem, smem);  // constant of the kernel, beside static shared memory
         kern<<<dim3((unsigned)nz, plane_groups(nz, cnt, MB)), TH, smem, s>>>(buf, M, tw, row_ptr, cell, out,
                                                                              o_stride, cnt);
     });
